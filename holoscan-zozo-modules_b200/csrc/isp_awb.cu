@@ -110,9 +110,8 @@ __global__ void __launch_bounds__(kThreads, 3) isp_awb_kernel(const __grid_const
   Span<unsigned int> hist = carve_span<unsigned int>(smem, kHistAt, kGridAt - kHistAt, rec);
   Span<float> grid_s = carve_span<float>(smem, kGridAt, kGridSmemGains * 4, rec);
   __shared__ uint64_t bars[2];
-  __shared__ u64 red[kWarps];
+  __shared__ u64 red[4 * kWarps];
   __shared__ int minmax[2];
-  __shared__ int first;
   __shared__ bool last;
   Span<Scratch> s = p.scratch;
   const int tid = threadIdx.x;
@@ -146,47 +145,49 @@ __global__ void __launch_bounds__(kThreads, 3) isp_awb_kernel(const __grid_const
   const int ty1 = min(ty0 + band_tiles, tiles_y);
   const int x0 = strip * 64;
   const auto issue = [&](int ty, int b) {
-    tma_load_2d(&map, boxes + b * 64 * 128, &bars[b], awb_box_x(p.raw_format, x0), ty * 64,
-                static_cast<unsigned int>(kBoxRows * box_bytes));
+    if (!use_tma) {
+      fill_box(p, boxes + b * 64 * 128, box_bytes, kBoxRows,
+               awb_box_x(p.raw_format, x0) * (p.raw_format == kRawU16 ? 2 : 1), ty * 64);
+    } else if (tid == 0) {
+      fence_async_shared();
+      tma_load_2d(&map, boxes + b * 64 * 128, &bars[b], awb_box_x(p.raw_format, x0), ty * 64,
+                  static_cast<unsigned int>(kBoxRows * box_bytes));
+    }
   };
   cp_async_wait_all();
   __syncthreads();  // barriers initialised, the gains in shared memory
-  if (use_tma && tid == 0 && ty0 < ty1) issue(ty0, 0);
+  if (ty0 < ty1) issue(ty0, 0);
   // The band's maps and table (block-synchronised inside), while the first
   // box is in flight.
   const LscTile lt = build_band_lsc(p, grid, kPat, x0, ty0 * 64, (ty1 - ty0) * 64, col_mx, col_ix, col_tx, row_my,
                                     row_k, row_ty, table, minmax);
   u64 acc[4] = {0, 0, 0, 0};
   uint32_t phases = 0;  // bit b: parity of buffer b's next completion
+  AwbCell cell;
   for (int ty = ty0; ty < ty1; ++ty) {
     const int buf = (ty - ty0) & 1;
+    if (!use_tma) {
+      box_filled();
+      __syncthreads();
+    }
     // The other buffer was read by the previous tile (the block synchronised
     // since): load the next tile into it while this one is summed.
-    if (use_tma && tid == 0 && ty + 1 < ty1) {
-      fence_async_shared();
-      issue(ty + 1, buf ^ 1);
-    }
+    if (ty + 1 < ty1) issue(ty + 1, buf ^ 1);
     if (use_tma && !mbar_wait(&bars[buf], (phases >> buf) & 1U)) {
       if (tid == 0) report_wait_timeout(s);
     }
     phases ^= 1U << buf;
-    Span<const uint8_t> box = boxes + buf * 64 * 128;
     const int rows = (ty - ty0) * 64;  // the tile's first row within the band
     unsigned int sum[3] = {0U, 0U, 0U};
     unsigned int quads = 0;
-    if (use_tma) {
-      awb_tile_fmt<0, kWhitePatch, kPat>(p, box, box_bytes, x0, ty * 64, lt, row_k + rows, row_ty + rows, table, black,
-                                          inv, hist, sum, quads);
-    } else {
-      awb_tile_fmt<1, kWhitePatch, kPat>(p, box, box_bytes, x0, ty * 64, lt, row_k + rows, row_ty + rows, table, black,
-                                          inv, hist, sum, quads);
-    }
+    awb_tile<kWhitePatch, kPat>(p, grid, boxes + buf * 64 * 128, box_bytes, x0, ty * 64, lt, row_k + rows, row_ty + rows,
+                                table, black, inv, hist, cell, sum, quads);
 #pragma unroll
     for (int k = 0; k < 3; ++k) acc[k] += sum[k];
     acc[3] += quads;
     __syncthreads();
   }
-  awb_flush<true>(p, acc, hist, kWhitePatch, red, &first, &last, static_cast<unsigned int>(ty1 > ty0 ? ty1 - ty0 : 0),
+  awb_flush<true>(p, acc, hist, kWhitePatch, red, &last, static_cast<unsigned int>(ty1 > ty0 ? ty1 - ty0 : 0),
             static_cast<unsigned int>(strips * tiles_y));
 }
 

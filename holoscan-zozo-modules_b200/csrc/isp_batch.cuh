@@ -40,6 +40,57 @@ __device__ __forceinline__ int frame_of_item(Span<const BatchFrame> frames, int 
   return f;
 }
 
+// One tile of a frame of any settings (BatchFrame::variant). Only what differs
+// between the variants is compiled per variant: the demosaics. With one copy
+// of the whole tile per variant (eight, each with the finish of four output
+// formats) the CTAs of an SM, at work on different variants, waited for
+// instructions more than for anything else (1.3 of 7.4 cycles per
+// instruction).
+template <bool kLutSmem, int kTileH, class AfterA>
+__device__ __forceinline__ void run_tile_any(const FrameDesc& p, const FrameSetup& f, const TileSmem& m, int* minmax,
+                                             int variant, int x0, int y0, bool use_tma, uint64_t* bar, uint32_t& phase,
+                                             u64 (&acc)[4], AfterA after_a) {
+  const bool sharpen = (variant & 2) != 0;
+  const auto no_wait = [] {};
+  acc[3] += sharpen ? tile_samples<Geom<true, kTileH>::kHalo, kTileH>(p, f, m, minmax, x0, y0, use_tma, bar, phase, no_wait)
+                    : tile_samples<Geom<false, kTileH>::kHalo, kTileH>(p, f, m, minmax, x0, y0, use_tma, bar, phase, no_wait);
+  __syncthreads();
+  after_a();
+  if (sharpen) {
+    const Span<float2> red = f.swap_rb ? m.B : m.R, blue = f.swap_rb ? m.R : m.B;
+    switch (variant) {
+      case 2: phase_b2<false, 0, kTileH>(m.P, red, m.G, blue); break;
+      case 3: phase_b2<true, 0, kTileH>(m.P, red, m.G, blue); break;
+      case 6: phase_b2<false, 2, kTileH>(m.P, red, m.G, blue); break;
+      default: phase_b2<true, 2, kTileH>(m.P, red, m.G, blue); break;
+    }
+    __syncthreads();
+  }
+  unsigned int sums[3] = {0U, 0U, 0U};
+  unsigned int npix = 0;
+#pragma unroll 1
+  for (int k = 0; k < kTileH / 32; ++k) {
+    int r, uc;
+    unit_rc(threadIdx.x + k * kThreads, r, uc);
+    float2 rgb[4][3];
+    if (sharpen) {
+      sharpened_row(m, r, uc, p.sharpen, rgb);
+    } else {
+      switch (variant) {
+        case 0: demosaiced_row<false, 0>(m, r, uc, rgb); break;
+        case 1: demosaiced_row<true, 0>(m, r, uc, rgb); break;
+        case 4: demosaiced_row<false, 2>(m, r, uc, rgb); break;
+        default: demosaiced_row<true, 2>(m, r, uc, rgb); break;
+      }
+      if (f.swap_rb) swap_red_blue(rgb);
+    }
+    finish_row<-1, kLutSmem>(p, f, m.hist, rgb, x0 + 4 * uc, y0 + r, sums, npix);
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) acc[k] += sums[k] - npix * kTwo23Bits;  // mod 2^32: the true sum
+  __syncthreads();  // the next tile overwrites the tables, P and the planes
+}
+
 template <bool kLutSmem, int kTileH>
 __global__ void __launch_bounds__(kThreads, kTileH == kTH ? 2 : 3)
     isp_batch_kernel(const BatchFrame* frames_in, int nframes, const int2* ranges_in) {
@@ -90,7 +141,7 @@ __global__ void __launch_bounds__(kThreads, kTileH == kTH ? 2 : 3)
   unsigned int done = 0;
   for (int item = r.x; item < r.y; ++item) {
     if (item >= frames[f].tile_begin + frames[f].tiles) {
-      flush_frame(fd, fs, acc, m.hist, red, &last, done, static_cast<unsigned int>(frames[f].tiles));
+      flush_frame(fd, fs, acc, m, red, &last, done, static_cast<unsigned int>(frames[f].tiles));
       __syncthreads();
       f = frame_of_item(frames, nframes, f, item, false);
       load_desc(&fd, &frames[f].desc);
@@ -115,30 +166,21 @@ __global__ void __launch_bounds__(kThreads, kTileH == kTH ? 2 : 3)
         }
       }
     };
-    switch (bf.variant) {
-      case 0: run_tile<false, false, 0, kLutSmem, decltype(prefetch), -1, kTileH>(fd, fs, m, minmax, x0, ty * kTileH, use_tma, &bar, phase, acc, prefetch); break;
-      case 1: run_tile<true, false, 0, kLutSmem, decltype(prefetch), -1, kTileH>(fd, fs, m, minmax, x0, ty * kTileH, use_tma, &bar, phase, acc, prefetch); break;
-      case 2: run_tile<false, true, 0, kLutSmem, decltype(prefetch), -1, kTileH>(fd, fs, m, minmax, x0, ty * kTileH, use_tma, &bar, phase, acc, prefetch); break;
-      case 3: run_tile<true, true, 0, kLutSmem, decltype(prefetch), -1, kTileH>(fd, fs, m, minmax, x0, ty * kTileH, use_tma, &bar, phase, acc, prefetch); break;
-      case 4: run_tile<false, false, 1, kLutSmem, decltype(prefetch), -1, kTileH>(fd, fs, m, minmax, x0, ty * kTileH, use_tma, &bar, phase, acc, prefetch); break;
-      case 5: run_tile<true, false, 1, kLutSmem, decltype(prefetch), -1, kTileH>(fd, fs, m, minmax, x0, ty * kTileH, use_tma, &bar, phase, acc, prefetch); break;
-      case 6: run_tile<false, true, 1, kLutSmem, decltype(prefetch), -1, kTileH>(fd, fs, m, minmax, x0, ty * kTileH, use_tma, &bar, phase, acc, prefetch); break;
-      default: run_tile<true, true, 1, kLutSmem, decltype(prefetch), -1, kTileH>(fd, fs, m, minmax, x0, ty * kTileH, use_tma, &bar, phase, acc, prefetch); break;
-    }
+    run_tile_any<kLutSmem, kTileH>(fd, fs, m, minmax, bf.variant, x0, ty * kTileH, use_tma, &bar, phase, acc, prefetch);
     ++done;
   }
-  flush_frame(fd, fs, acc, m.hist, red, &last, done, static_cast<unsigned int>(frames[f].tiles));
+  flush_frame(fd, fs, acc, m, red, &last, done, static_cast<unsigned int>(frames[f].tiles));
 }
 
 // The statistics tile of a frame for its Bayer pattern and mode.
-template <int kSrc>
 __device__ __forceinline__ void awb_tile_any(const FrameDesc& p, int pattern, bool white_patch, Span<const uint8_t> box,
                                              int box_bytes, int x0, int y0, const LscTile& lt, Span<const int> row_k,
                                              Span<const float> row_ty, Span<const float> table, const float (&black)[4],
                                              const float (&inv)[4], Span<unsigned int> hist, unsigned int (&sum)[3],
                                              unsigned int& quads) {
+  AwbCell cell;  // the table is the tile's own
 #define ISP_AWB_CASE(P, W) \
-  awb_tile_fmt<kSrc, W, P>(p, box, box_bytes, x0, y0, lt, row_k, row_ty, table, black, inv, hist, sum, quads)
+  awb_tile<W, P>(p, p.lsc, box, box_bytes, x0, y0, lt, row_k, row_ty, table, black, inv, hist, cell, sum, quads)
   switch (pattern * 2 + (white_patch ? 1 : 0)) {
     case 0: ISP_AWB_CASE(0, false); break;
     case 1: ISP_AWB_CASE(0, true); break;
@@ -179,7 +221,6 @@ __global__ void __launch_bounds__(kThreads, 3) isp_awb_batch_kernel(const BatchF
   __shared__ uint64_t bars[2];
   __shared__ u64 red[4 * kWarps];
   __shared__ int minmax[2];
-  __shared__ int first;
   __shared__ bool last;
   __shared__ __align__(16) FrameDesc fd;
   griddep_launch_dependents();  // the tile batch may become resident as this one finishes
@@ -212,7 +253,7 @@ __global__ void __launch_bounds__(kThreads, 3) isp_awb_batch_kernel(const BatchF
   unsigned int done = 0;
   for (int item = r.x; item < r.y; ++item) {
     if (item >= frames[f].awb_begin + frames[f].awb_tiles) {
-      awb_flush(fd, acc, hist, fd.awb_mode == kWbWhitePatch, red, &first, &last, done,
+      awb_flush(fd, acc, hist, fd.awb_mode == kWbWhitePatch, red, &last, done,
                 static_cast<unsigned int>(frames[f].awb_tiles));
       f = frame_of_item(frames, nframes, f, item, true);
       load_desc(&fd, &frames[f].desc);
@@ -237,12 +278,19 @@ __global__ void __launch_bounds__(kThreads, 3) isp_awb_batch_kernel(const BatchF
     const int ty = local / bf.awb_tiles_x;
     const int x0 = (local - ty * bf.awb_tiles_x) * 64;
     const int y0 = ty * 64;
+    const bool use_tma = bf.use_tma != 0;
+    const int box_bytes = awb_box_bytes(fd.raw_format);
+    if (!use_tma) {
+      fill_box(fd, boxes + buf * 64 * 128, box_bytes, 64, awb_box_x(fd.raw_format, x0) * (fd.raw_format == kRawU16 ? 2 : 1), y0);
+    }
     const LscTile lt = build_lsc(fd, fd.lsc, fd.pattern, x0, 64, y0, 64, false, 0, 0, col_mx, col_ix, col_tx, row_my, row_k,
                                  row_ty, table, minmax);
-    const bool use_tma = bf.use_tma != 0;
     if (use_tma) {
       if (!mbar_wait(&bars[buf], (phases >> buf) & 1U) && tid == 0) report_wait_timeout(fd.scratch);
       phases ^= 1U << buf;
+    } else {
+      box_filled();
+      __syncthreads();
     }
     float black[4], inv[4];
 #pragma unroll
@@ -252,22 +300,15 @@ __global__ void __launch_bounds__(kThreads, 3) isp_awb_batch_kernel(const BatchF
     }
     unsigned int sum[3] = {0U, 0U, 0U};
     unsigned int quads = 0;
-    const int box_bytes = awb_box_bytes(fd.raw_format);
-    const bool wp = fd.awb_mode == kWbWhitePatch;
-    if (use_tma) {
-      awb_tile_any<0>(fd, fd.pattern, wp, boxes + buf * 64 * 128, box_bytes, x0, y0, lt, row_k, row_ty, table, black,
-                      inv, hist, sum, quads);
-    } else {
-      awb_tile_any<1>(fd, fd.pattern, wp, boxes + buf * 64 * 128, box_bytes, x0, y0, lt, row_k, row_ty, table, black,
-                      inv, hist, sum, quads);
-    }
+    awb_tile_any(fd, fd.pattern, fd.awb_mode == kWbWhitePatch, boxes + buf * 64 * 128, box_bytes, x0, y0, lt, row_k, row_ty,
+                 table, black, inv, hist, sum, quads);
 #pragma unroll
     for (int k = 0; k < 3; ++k) acc[k] += sum[k];
     acc[3] += quads;
     __syncthreads();
     ++done;
   }
-  awb_flush(fd, acc, hist, fd.awb_mode == kWbWhitePatch, red, &first, &last, done,
+  awb_flush(fd, acc, hist, fd.awb_mode == kWbWhitePatch, red, &last, done,
             static_cast<unsigned int>(frames[f].awb_tiles));
 }
 

@@ -189,7 +189,6 @@ FrameDesc make_desc(const isp_params_c& p, const DeviceState& s, const isp_raw_v
   d.out = make_span(static_cast<uint8_t*>(out.data), out_bytes, rec);
   d.out_pitch = static_cast<int64_t>(out.pitch);
   d.out_format = out.format;
-  d.out_vector = (reinterpret_cast<uintptr_t>(out.data) % 16U == 0U) && (out.pitch % 16U == 0U);
   d.hist_out = make_span(stats != nullptr ? stats->histogram : nullptr,
                          static_cast<size_t>(ISP_HISTOGRAM_CHANNELS) * ISP_HISTOGRAM_BINS, rec);
   d.stats_out = make_span(stats != nullptr ? stats->stats : nullptr, static_cast<size_t>(ISP_STATS_SIZE), rec);

@@ -54,6 +54,9 @@ static_assert(cfa_of(0, 0) == kChR && cfa_of(1, 3) == kChR && cfa_of(2, 1) == kC
 // for the frame (a 17 x 13 x 4 grid is 884).
 constexpr int kGridSmemGains = 1024;
 
+// A frame's constants per quad position (3 x 4) and its gains.
+constexpr int kQuadFloats = 15;
+
 // Paired pixels. The tile pass computes two pixels in the two lanes of every
 // f32x2 operation: columns c and c + kHalf of the same row, which have the
 // same Bayer colour and so the same arithmetic. Samples and RGB values live
@@ -80,15 +83,19 @@ struct Geom {
 
 // ---- Shared memory layout -------------------------------------------------
 
+// The regions whose size a kernel instance knows come first, so that their
+// offsets from the one base register are constants; the TMA box (its size
+// depends on the raw format) and the tone table follow.
 struct Layout {
-  int raw;      // TMA box: box rows x box bytes
   int samples;  // float2 [kSH][kPW]
   int r, g, b;  // float2 [kCH][kCW2] each (sharpening)
   int lsc;      // float2 [kLscTableRows][2][kPW]
   int cols;     // int col_mx[kSW]; int col_ix[kSW]; float col_tx[kSW]
   int rows;     // int row_my[kSH]; int row_k[kSH]; float row_ty[kSH]
+  int quad;     // float [kQuadFloats]: the frame's constants per quad position
   int hist;     // u32 [4][256]
   int grid;     // float [kGridSmemGains]: the frame's lens shading grid, when it fits
+  int raw;      // TMA box: box rows x box bytes
   int lut;      // float2 [tone_size] when in shared memory
   int total;
 };
@@ -101,8 +108,6 @@ __host__ __device__ constexpr Layout layout_of(bool sharpen, int box_bytes_row, 
   const int plane = align128((tile_h + 2) * kCW2 * 8);
   Layout l{};
   int o = 0;
-  l.raw = o;
-  o = align128(o + sh * box_bytes_row);
   l.samples = o;
   o = align128(o + sh * kPW * 8);
   l.r = o;
@@ -115,10 +120,14 @@ __host__ __device__ constexpr Layout layout_of(bool sharpen, int box_bytes_row, 
   o = align128(o + 3 * kSW * 4);
   l.rows = o;
   o = align128(o + 3 * sh * 4);
+  l.quad = o;
+  o = align128(o + kQuadFloats * 4);
   l.hist = o;
   o = align128(o + kHistChannels * kHistBins * 4);
   l.grid = o;
   o = align128(o + kGridSmemGains * 4);
+  l.raw = o;
+  o = align128(o + sh * box_bytes_row);
   l.lut = o;
   o = align128(o + lut_entries * 8);
   l.total = o;
@@ -226,41 +235,53 @@ __device__ __forceinline__ int box_x(int fmt, int x0) {
 
 // ---- Raw unpacking from a box row ----------------------------------------
 
-// Samples x0 - 4 + 4u .. + 3 of a box row (box starting at box_x(fmt, x0)).
-__device__ __forceinline__ void unpack4(int fmt, Span<const uint8_t> row, int u, unsigned int s[4]) {
+// Samples x0 - 4 + 4u .. + 3 of a box row (box starting at box_x(fmt, x0)) as
+// 16-bit halves: w[0] holds the first two, w[1] the last two. Packed halves
+// cost 2.5 (RAW10) or 3 (RAW12) integer operations a sample where extracting
+// each sample on its own took 4, and the saturation tests take a maximum of
+// two samples per instruction.
+__device__ __forceinline__ void unpack4(int fmt, Span<const uint8_t> row, int u, unsigned int (&w)[2]) {
   if (fmt == kRawU8) {
-    const unsigned int w = *span_cast<const unsigned int>(row + 12 + 4 * u);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) s[k] = (w >> (8 * k)) & 0xFFU;
+    const unsigned int v = *span_cast<const unsigned int>(row + 12 + 4 * u);
+    w[0] = __byte_perm(v, 0U, 0x4140);
+    w[1] = __byte_perm(v, 0U, 0x4342);
   } else if (fmt == kRawU16) {
-    const uint2 w = *span_cast<const uint2>(row + 8 + 8 * u);
-    s[0] = w.x & 0xFFFFU;
-    s[1] = w.x >> 16;
-    s[2] = w.y & 0xFFFFU;
-    s[3] = w.y >> 16;
+    const uint2 v = *span_cast<const uint2>(row + 8 + 8 * u);
+    w[0] = v.x;
+    w[1] = v.y;
   } else if (fmt == kRawRaw10) {
     // Group g0 - 1 + u at byte 11 + 5u: four high bytes, then the low bits.
     const int b = 11 + 5 * u;
-    Span<const unsigned int> w = span_cast<const unsigned int>(row + (b & ~3));
-    const unsigned int sh = 8U * static_cast<unsigned int>(b & 3);
-    const unsigned int hi4 = __funnelshift_r(w[0], w[1], sh);
-    const unsigned int lo = (w[1] >> sh) & 0xFFU;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) s[k] = (((hi4 >> (8 * k)) & 0xFFU) << 2) | ((lo >> (2 * k)) & 3U);
+    Span<const unsigned int> v = span_cast<const unsigned int>(row + (b & ~3));
+    const unsigned int at = static_cast<unsigned int>(b & 3);
+    const unsigned int next = v[1];
+    const unsigned int hi4 = __funnelshift_r(v[0], next, 8U * at);
+    // The four 2-bit fields: t holds the low byte at bits 0 and 14, so that
+    // fields 0 and 1 (2 and 3 after >> 4) lie at bits 0 and 16.
+    const unsigned int t = __byte_perm(next, 0U, 0x4440U + at) * 0x4001U;
+    w[0] = __byte_perm(hi4, 0U, 0x4140) * 4U + (t & 0x00030003U);
+    w[1] = __byte_perm(hi4, 0U, 0x4342) * 4U + ((t >> 4) & 0x00030003U);
   } else {
-    // Two groups of three bytes at byte 10 + 6u.
+    // Two groups of three bytes at byte 10 + 6u: two high bytes, then the low
+    // nibbles, copied to bits 0 and 12 so that they lie at bits 0 and 16.
     const int b = 10 + 6 * u;
-    Span<const unsigned int> w = span_cast<const unsigned int>(row + (b & ~3));
+    Span<const unsigned int> v = span_cast<const unsigned int>(row + (b & ~3));
     const unsigned int sh = 8U * static_cast<unsigned int>(b & 3);
-    const unsigned int v0 = __funnelshift_r(w[0], w[1], sh);  // a0 a1 a2 b0
-    const unsigned int v1 = w[1] >> sh;                        // b1 b2 ..
-    const unsigned int a2 = (v0 >> 16) & 0xFFU;
-    const unsigned int b2 = (v1 >> 8) & 0xFFU;
-    s[0] = ((v0 & 0xFFU) << 4) | (a2 & 15U);
-    s[1] = (((v0 >> 8) & 0xFFU) << 4) | (a2 >> 4);
-    s[2] = ((v0 >> 24) << 4) | (b2 & 15U);
-    s[3] = ((v1 & 0xFFU) << 4) | (b2 >> 4);
+    const unsigned int next = v[1];
+    const unsigned int v0 = __funnelshift_r(v[0], next, sh);  // a0 a1 a2 b0
+    const unsigned int v1 = next >> sh;                        // b1 b2 ..
+    w[0] = __byte_perm(v0, 0U, 0x4140) * 16U + ((__byte_perm(v0, 0U, 0x4442) * 0x1001U) & 0x000F000FU);
+    w[1] = (__byte_perm(v0, v1, 0x0403) & 0x00FF00FFU) * 16U +
+           ((__byte_perm(v1, 0U, 0x4441) * 0x1001U) & 0x000F000FU);
   }
+}
+
+// 2^23 + a 16-bit half of w, as the bits of a float.
+__device__ __forceinline__ unsigned int magic_low(unsigned int w) { return __byte_perm(w, kTwo23Bits, 0x7610); }
+__device__ __forceinline__ unsigned int magic_high(unsigned int w) { return __byte_perm(w, kTwo23Bits, 0x7632); }
+// Whether a 16-bit half of w is at least `white`.
+__device__ __forceinline__ bool any_half_at_least(unsigned int w, unsigned int white) {
+  return max(w & 0xFFFFU, w >> 16) >= white;
 }
 
 // One sample at image column mx of a box row (box starting at box_x(fmt, x0)).
@@ -275,6 +296,72 @@ __device__ __forceinline__ unsigned int unpack1(int fmt, Span<const uint8_t> row
   Span<const uint8_t> g = row + 3 * ((mx >> 1) - (x0 >> 1)) + 16;
   const int k = mx & 1;
   return (static_cast<unsigned int>(g[k]) << 4) | ((g[2] >> (4 * k)) & 15U);
+}
+
+// The four samples whose mirrored columns col_mx holds, from a box row, as
+// unpack4's halves. For the few units of an edge tile that reach past the
+// image; out of line, so that they cost the others no registers or code.
+__device__ __noinline__ uint2 unpack_edge4(int fmt, Span<const uint8_t> row, Span<const int> col_mx, int x0) {
+  unsigned int s[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) s[k] = unpack1(fmt, row, col_mx[k], x0);
+  return make_uint2(s[0] | (s[1] << 16), s[2] | (s[3] << 16));
+}
+
+// ---- Boxes without TMA -----------------------------------------------------
+
+// The bytes of a raw row (raw_row_bytes, isp_params.cpp:184-197).
+__device__ __forceinline__ int raw_bytes_of(int fmt, int width) {
+  return fmt == kRawU8 ? width : fmt == kRawU16 ? 2 * width : fmt == kRawRaw10 ? 5 * ((width + 3) >> 2) : 3 * ((width + 1) >> 1);
+}
+
+// Fills a box as TMA would, for a frame whose rows are not 16-byte aligned:
+// `rows` rows of `box_bytes` bytes from byte bx (a multiple of 16) of image
+// rows y0 .., zero outside the image. Warps take rows, lanes 4-byte words:
+// asynchronous copies where rows are 4-byte aligned, else two aligned words
+// shifted together; the words at a row's ends byte by byte, so that nothing
+// outside the frame's rows is read. The caller waits (box_filled) and
+// synchronises the block. The copies are in flight while the tile's lens
+// shading table is built. A 1366x768 16-bit frame with packed rows (white
+// patch, RGB32F) takes 31.6 us this way; with a load from global memory per
+// sample in both passes it took 42.9.
+__device__ void fill_box(const FrameDesc& p, Span<uint8_t> box, int box_bytes, int rows, int bx, int y0) {
+  const int row_bytes = raw_bytes_of(p.raw_format, p.width);
+  const int words = box_bytes >> 2;
+  const bool aligned = ((reinterpret_cast<uintptr_t>(span_ptr(p.raw)) | static_cast<uintptr_t>(p.raw_pitch)) & 3U) == 0U;
+  for (int j = threadIdx.x >> 5; j < rows; j += kWarps) {
+    const int y = y0 + j;
+    const bool inside = y >= 0 && y < p.height;
+    Span<const uint8_t> row = p.raw + static_cast<int64_t>(inside ? y : 0) * p.raw_pitch;
+    for (int c = threadIdx.x & 31; c < words; c += 32) {
+      const int o = bx + 4 * c;
+      Span<uint8_t> dst = box + j * box_bytes + 4 * c;
+      unsigned int v = 0U;
+      if (inside && o > -4 && o < row_bytes) {
+        if (aligned && o >= 0 && o + 4 <= row_bytes) {
+          cp_async4(span_range(dst, 4), span_range(row + o, 4));
+          continue;
+        }
+        if (o >= 4 && o + 8 <= row_bytes) {
+          const unsigned int back = static_cast<unsigned int>(reinterpret_cast<uintptr_t>(span_ptr(row + o)) & 3U);
+          Span<const unsigned int> w = span_cast<const unsigned int>(row + (o - static_cast<int>(back)));
+          v = __funnelshift_r(__ldg(&w[0]), __ldg(&w[1]), 8U * back);
+        } else {
+          for (int b = 0; b < 4; ++b) {
+            if (o + b >= 0 && o + b < row_bytes) v |= static_cast<unsigned int>(__ldg(&row[o + b])) << (8 * b);
+          }
+        }
+      }
+      *span_cast<unsigned int>(dst) = v;
+    }
+  }
+}
+
+// Waits for this thread's part of fill_box and orders it before a later TMA
+// copy into the same box (a batch mixes both); the block barrier is the caller's.
+__device__ __forceinline__ void box_filled() {
+  cp_async_wait_all();
+  fence_async_shared();
 }
 
 // ---- Lens shading tables --------------------------------------------------
@@ -450,18 +537,6 @@ __device__ __forceinline__ u64 warp_sum(u64 v) {
   return v;
 }
 
-// Sum of one u64 per thread over the block; the result in every thread.
-__device__ u64 block_sum(u64 v, u64* red) {
-  v = warp_sum(v);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  u64 total = 0;
-#pragma unroll
-  for (int w = 0; w < kWarps; ++w) total += red[w];
-  return total;
-}
-
 // Sums of four u64 per thread over the block, in `out` of thread 0; `red`
 // holds 4 x kWarps values.
 __device__ __forceinline__ void block_sum4(const u64 (&v)[4], u64* red, u64 (&out)[4]) {
@@ -482,85 +557,73 @@ __device__ __forceinline__ void block_sum4(const u64 (&v)[4], u64* red, u64 (&ou
   }
 }
 
-// Exclusive prefix sum of one u64 per thread over the block.
-__device__ u64 block_exclusive_scan(u64 v, u64* red) {
+// histogram_percentile (isp_math.hpp:336-352) by one warp: lane l owns bins
+// 32l .. 32l + 31; the prefix counts are exact integers, so every comparison is
+// the reference's. The result in every lane. (Three warps take the three
+// colours side by side, without block barriers: one colour after the other by
+// the whole block took two dozen of them at the end of every frame.)
+__device__ float warp_percentile(Span<const unsigned int> hist, float percentile) {
+  constexpr int kPerLane = kAwbBins / 32;
   const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  u64 inc = v;
+  uint4 h[kPerLane / 4];
+  u64 mine = 0;
+#pragma unroll
+  for (int k = 0; k < kPerLane / 4; ++k) {
+    h[k] = __ldcg(&span_cast<const uint4>(hist)[lane * (kPerLane / 4) + k]);
+    mine += static_cast<u64>(h[k].x) + h[k].y + h[k].z + h[k].w;
+  }
+  u64 inc = mine;
 #pragma unroll
   for (int offset = 1; offset < 32; offset <<= 1) {
     const u64 up = __shfl_up_sync(0xFFFFFFFFU, inc, offset);
     if (lane >= offset) inc += up;
   }
-  __syncthreads();
-  if (lane == 31) red[warp] = inc;
-  __syncthreads();
-  u64 before = 0;
-  for (int w = 0; w < warp; ++w) before += red[w];
-  return before + inc - v;
-}
-
-// histogram_percentile (isp_math.hpp:336-352) by the whole block: thread t
-// owns bins 4t..4t+3; the prefix counts are exact integers, so every
-// comparison is the reference's.
-__device__ float block_percentile(Span<const unsigned int> hist, float percentile, u64* red, int* first) {
-  const int t = threadIdx.x;
-  unsigned int h[4];
-  u64 mine = 0;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    h[k] = __ldcg(&hist[4 * t + k]);
-    mine += h[k];
-  }
-  const u64 total = block_sum(mine, red);
+  const u64 total = __shfl_sync(0xFFFFFFFFU, inc, 31);
   if (total == 0) return 0.0F;
-  const u64 below0 = block_exclusive_scan(mine, red);
   const double target = static_cast<double>(percentile) * static_cast<double>(total);
-  if (t == 0) *first = kAwbBins;
-  __syncthreads();
-  u64 below = below0;
-  int mine_first = kAwbBins;
-  u64 mine_below = 0;
-  unsigned int mine_count = 0;
+  // This lane's first counted bin that reaches the target; the lowest such
+  // lane holds the answer.
+  u64 below = inc - mine;
+  int bin = -1;
+  u64 bin_below = 0;
+  unsigned int bin_count = 0;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    if (mine_first == kAwbBins && h[k] != 0U && static_cast<double>(below + h[k]) >= target) {
-      mine_first = 4 * t + k;
-      mine_below = below;
-      mine_count = h[k];
+  for (int k = 0; k < kPerLane; ++k) {
+    const uint4 w = h[k >> 2];
+    const unsigned int n = (k & 3) == 0 ? w.x : (k & 3) == 1 ? w.y : (k & 3) == 2 ? w.z : w.w;
+    if (bin < 0 && n != 0U && static_cast<double>(below + n) >= target) {
+      bin = lane * kPerLane + k;
+      bin_below = below;
+      bin_count = n;
     }
-    below += h[k];
+    below += n;
   }
-  if (mine_first < kAwbBins) atomicMin(first, mine_first);
-  __syncthreads();
-  const int b = *first;
-  __shared__ float result;
-  if (b == kAwbBins) {
-    if (t == 0) result = 1.0F;
-  } else if (mine_first == b) {
-    const double within = (target - static_cast<double>(mine_below)) / static_cast<double>(mine_count);
-    result = static_cast<float>((static_cast<double>(b) + within) / kAwbBins);
+  const unsigned int found = __ballot_sync(0xFFFFFFFFU, bin >= 0);
+  if (found == 0U) return 1.0F;
+  float result = 1.0F;
+  if (bin >= 0) {
+    const double within = (target - static_cast<double>(bin_below)) / static_cast<double>(bin_count);
+    result = static_cast<float>((static_cast<double>(bin) + within) / kAwbBins);
   }
-  __syncthreads();
-  const float r = result;
-  __syncthreads();
-  return r;
+  return __shfl_sync(0xFFFFFFFFU, result, __ffs(static_cast<int>(found)) - 1);
 }
 
 // finish_white_balance (isp_math.hpp:357-384) in the statistics pass's last
 // CTA; then the sums are cleared for the next frame.
-__device__ void awb_finish(const FrameDesc& p, Span<Scratch> s, u64* red, int* first) {
+__device__ void awb_finish(const FrameDesc& p, Span<Scratch> s) {
+  __shared__ float level[3];
+  const int warp = threadIdx.x >> 5;
   const u64 nquads = __ldcg(&s->awb_quads);
-  float level[3] = {0.0F, 0.0F, 0.0F};
-  if (nquads != 0) {
+  if (nquads != 0 && warp < 3) {
+    float v;
     if (p.awb_mode == kWbGrayWorld) {
       const double q = static_cast<double>(nquads);
-      level[0] = static_cast<float>(static_cast<double>(__ldcg(&s->awb_sum[0])) / q);
-      level[1] = static_cast<float>(static_cast<double>(__ldcg(&s->awb_sum[1])) / (2.0 * q));
-      level[2] = static_cast<float>(static_cast<double>(__ldcg(&s->awb_sum[2])) / q);
+      const double sum = static_cast<double>(__ldcg(&s->awb_sum[warp]));
+      v = static_cast<float>(warp == 1 ? sum / (2.0 * q) : sum / q);
     } else {
-      for (int k = 0; k < 3; ++k) level[k] = block_percentile(sub_span(s, &s->awb_hist[k][0], kAwbBins), p.awb_percentile, red, first);
+      v = warp_percentile(sub_span(s, &s->awb_hist[warp][0], kAwbBins), p.awb_percentile);
     }
+    if ((threadIdx.x & 31) == 0) level[warp] = v;
   }
   __syncthreads();
   if (threadIdx.x == 0 && nquads != 0 && level[0] > 0.0F && level[1] > 0.0F && level[2] > 0.0F) {
@@ -574,8 +637,11 @@ __device__ void awb_finish(const FrameDesc& p, Span<Scratch> s, u64* red, int* f
     }
     s->awb_valid = 1;
   }
-  const Span<unsigned int> bins = sub_span(s, &s->awb_hist[0][0], 3 * kAwbBins);
-  for (int i = threadIdx.x; i < 3 * kAwbBins; i += kThreads) bins[i] = 0U;
+  if (p.awb_mode == kWbWhitePatch) {
+    static_assert(offsetof(Scratch, awb_hist) % 16 == 0, "bins are cleared 16 bytes at a time");
+    const Span<uint4> bins = span_cast<uint4>(sub_span(s, &s->awb_hist[0][0], 3 * kAwbBins));
+    for (int i = threadIdx.x; i < 3 * kAwbBins / 4; i += kThreads) bins[i] = make_uint4(0U, 0U, 0U, 0U);
+  }
   if (threadIdx.x < 3) s->awb_sum[threadIdx.x] = 0;
   if (threadIdx.x == 3) s->awb_quads = 0;
   if (threadIdx.x == 4) s->awb_done = 0;

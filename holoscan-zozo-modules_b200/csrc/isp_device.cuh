@@ -30,53 +30,31 @@ __device__ __forceinline__ int color_of(int channel) {
 
 __device__ __forceinline__ float clamp01(float v) { return v < 0.0F ? 0.0F : v > 1.0F ? 1.0F : v; }
 
-// One sample's raw counts (isp_math.hpp:101-119), read through the read-only path.
-__device__ __forceinline__ int load_raw(const FrameDesc& p, int x, int y) {
-  Span<const uint8_t> row = p.raw + static_cast<int64_t>(y) * p.raw_pitch;
-  switch (p.raw_format) {
-    case kRawU8:
-      return __ldg(&row[x]);
-    case kRawU16:
-      return __ldg(&span_cast<const uint16_t>(row)[x]);
-    case kRawRaw10: {
-      Span<const uint8_t> g = row + 5 * (x >> 2);
-      const int k = x & 3;
-      return (static_cast<int>(__ldg(&g[k])) << 2) | ((__ldg(&g[4]) >> (2 * k)) & 3);
-    }
-    default: {
-      Span<const uint8_t> g = row + 3 * (x >> 1);
-      const int k = x & 1;
-      return (static_cast<int>(__ldg(&g[k])) << 4) | ((__ldg(&g[2]) >> (4 * k)) & 15);
-    }
-  }
-}
+// A frame's lens shading grid.
+struct LscGrid {
+  Span<const float> gains;
+  int width, height, channels;
+  float sx, sy;
+};
 
 // Lens shading gain at (x, y) (isp_math.hpp:121-140): bilinear in the grid,
-// first across (top and bottom rows of the cell), then down.
-__device__ __forceinline__ float lens_shading_gain(const FrameDesc& p, Span<const float> grid, int x, int y,
-                                                   int channel) {
-  const float fx = static_cast<float>(x) * p.lsc_sx;
-  const float fy = static_cast<float>(y) * p.lsc_sy;
+// first across (top and bottom rows of the cell), then down. Out of line: only
+// grids too dense for a tile's table come here.
+static __device__ __noinline__ float lens_shading_gain_outline(LscGrid p, int x, int y, int channel) {
+  const float fx = static_cast<float>(x) * p.sx;
+  const float fy = static_cast<float>(y) * p.sy;
   int ix = static_cast<int>(fx);
   int iy = static_cast<int>(fy);
-  ix = ix > p.lsc_width - 2 ? p.lsc_width - 2 : ix;
-  iy = iy > p.lsc_height - 2 ? p.lsc_height - 2 : iy;
+  ix = ix > p.width - 2 ? p.width - 2 : ix;
+  iy = iy > p.height - 2 ? p.height - 2 : iy;
   const float tx = fx - static_cast<float>(ix);
   const float ty = fy - static_cast<float>(iy);
-  const int step = p.lsc_channels;
-  const int row = p.lsc_width * step;
-  Span<const float> g = grid + (iy * p.lsc_width + ix) * step + (step == 4 ? channel : 0);
+  const int step = p.channels;
+  const int row = p.width * step;
+  Span<const float> g = p.gains + (iy * p.width + ix) * step + (step == 4 ? channel : 0);
   const float top = g[0] + (g[step] - g[0]) * tx;
   const float bottom = g[row] + (g[row + step] - g[row]) * tx;
   return top + (bottom - top) * ty;
-}
-
-// Black level and lens shading (isp_math.hpp:144-148): 0 at black, 1 at white.
-__device__ __forceinline__ float linearize(const FrameDesc& p, Span<const float> grid, int raw, int x, int y,
-                                           int channel) {
-  float v = (static_cast<float>(raw) - p.black[channel]) * p.inv_range[channel];
-  v = v > 0.0F ? v : 0.0F;
-  return grid != nullptr ? v * lens_shading_gain(p, grid, x, y, channel) : v * 1.0F;
 }
 
 // The Malvar-He-Cutler or bilinear estimates at the centre of a 5x5
@@ -163,8 +141,8 @@ __device__ __forceinline__ float sharpen_one(float c, float m01, float m21, floa
 // estimate_rb_site, estimate_g_site and sharpen_one with the operations
 // two-lane ones: each lane sees exactly the scalar function's operations, in
 // the same order (sums left to right as written above). A sum that consumes
-// a product runs per lane (isp_ops.cuh: the assembler may fuse two-lane
-// products into two-lane sums).
+// a product is a psum2 or pdiff2 (isp_ops.cuh: the assembler may fuse two-lane
+// products into plain two-lane sums).
 
 template <bool kMalvar>
 __device__ __forceinline__ void estimate_rb_site2(const float2 (&n)[5][5], float2& at_green, float2& diagonal) {
@@ -177,8 +155,7 @@ __device__ __forceinline__ void estimate_rb_site2(const float2 (&n)[5][5], float
     const float2 axial2 = add2(add2(add2(n[0][2], n[4][2]), n[2][0]), n[2][4]);
     const float2 diagonal1 = add2(add2(add2(n[1][1], n[1][3]), n[3][1]), n[3][3]);
     at_green = mul_sat2(sub2(exact_scale_add2(axial1, bc2(2.0F), mul2(bc2(4.0F), c)), axial2), bc2(0.125F));
-    // 1.5 axial2 is a rounded product: subtracted per lane (isp_ops.cuh).
-    diagonal = mul_sat2(sub_lanes(exact_scale_add2(diagonal1, bc2(2.0F), mul2(bc2(6.0F), c)), mul2(bc2(1.5F), axial2)),
+    diagonal = mul_sat2(pdiff2(exact_scale_add2(diagonal1, bc2(2.0F), mul2(bc2(6.0F), c)), mul2(bc2(1.5F), axial2)),
                         bc2(0.125F));
   }
 }
@@ -193,12 +170,12 @@ __device__ __forceinline__ void estimate_g_site2(const float2 (&n)[5][5], float2
     const float2 diagonal1 = add2(add2(add2(n[1][1], n[1][3]), n[3][1]), n[3][3]);
     const float2 horizontal2 = add2(n[2][0], n[2][4]);
     const float2 vertical2 = add2(n[0][2], n[4][2]);
-    // 0.5 v2 is exact except below the normal range: added per lane all the same.
-    across = mul_sat2(add_lanes(sub2(sub2(exact_scale_add2(add2(n[2][1], n[2][3]), bc2(4.0F), c5), horizontal2), diagonal1),
-                                mul2(bc2(0.5F), vertical2)),
+    // 0.5 v2 is exact except below the normal range: a product of its own all the same.
+    across = mul_sat2(psum2(mul2(bc2(0.5F), vertical2),
+                            sub2(sub2(exact_scale_add2(add2(n[2][1], n[2][3]), bc2(4.0F), c5), horizontal2), diagonal1)),
                       bc2(0.125F));
-    down = mul_sat2(add_lanes(sub2(sub2(exact_scale_add2(add2(n[1][2], n[3][2]), bc2(4.0F), c5), vertical2), diagonal1),
-                              mul2(bc2(0.5F), horizontal2)),
+    down = mul_sat2(psum2(mul2(bc2(0.5F), horizontal2),
+                          sub2(sub2(exact_scale_add2(add2(n[1][2], n[3][2]), bc2(4.0F), c5), vertical2), diagonal1)),
                     bc2(0.125F));
   }
 }
@@ -227,7 +204,7 @@ __device__ __forceinline__ float2 sharpen_one2(float2 c, float2 m01, float2 m21,
   const float2 axial = add2(add2(add2(m01, m21), m10), m12);
   const float2 corners = add2(add2(add2(m00, m02), m20), m22);
   const float2 blur = mul2(add2(exact_scale_add2(axial, bc2(2.0F), mul2(bc2(4.0F), c)), corners), bc2(0.0625F));
-  return add_sat2(c, mul2(amount, sub_lanes(c, blur)));  // blur is a product: per lane
+  return add_sat2(c, mul2(amount, pdiff2(c, blur)));
 }
 
 // Colour correction (isp_math.hpp:229-233).

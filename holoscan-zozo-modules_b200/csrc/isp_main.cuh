@@ -1,7 +1,7 @@
 // isp_main.cuh - the fused tile pass of the B200 ISP as device templates: a
 // frame's per-CTA setup, one 64x64 tile (phases A, B, C), and the per-frame
 // flush with the last-tile finish. The single-frame kernel here and the
-// batch kernel (isp_batch.cu) are both built from them, so every frame gets
+// batch kernel (isp_batch.cuh) are both built from them, so every frame gets
 // the same arithmetic however it is launched. Each isp_main_*.cu
 // translation unit instantiates one demosaic method and sharpening setting,
 // so the instances compile in parallel.
@@ -26,6 +26,10 @@ struct TileSmem {
   Span<int> row_my;
   Span<int> row_k;
   Span<float> row_ty;
+  // The frame's black levels, inverse ranges and white balance gains per quad
+  // position [3][4], then the gains of red, green and blue: read once per tile
+  // and thread, so they need no registers in between.
+  Span<float> quad;
   Span<unsigned int> hist;
   Span<float> grid;
   Span<float2> lut_s;
@@ -35,7 +39,7 @@ struct TileSmem {
 // accesses to them; `rec` is where it counts violations).
 __device__ __forceinline__ TileSmem carve(unsigned char* smem, const Layout& L, int sample_rows, CheckRecord* rec) {
   TileSmem m;
-  m.box = carve_span<uint8_t>(smem, L.raw, L.samples - L.raw, rec);
+  m.box = carve_span<uint8_t>(smem, L.raw, L.lut - L.raw, rec);
   m.P = carve_span<float2>(smem, L.samples, L.r - L.samples, rec);
   m.R = carve_span<float2>(smem, L.r, L.g - L.r, rec);
   m.G = carve_span<float2>(smem, L.g, L.b - L.g, rec);
@@ -47,18 +51,15 @@ __device__ __forceinline__ TileSmem carve(unsigned char* smem, const Layout& L, 
   m.row_my = carve_span<int>(smem, L.rows, sample_rows * 4, rec);
   m.row_k = carve_span<int>(smem, L.rows + sample_rows * 4, sample_rows * 4, rec);
   m.row_ty = carve_span<float>(smem, L.rows + 2 * sample_rows * 4, sample_rows * 4, rec);
+  m.quad = carve_span<float>(smem, L.quad, kQuadFloats * 4, rec);
   m.hist = carve_span<unsigned int>(smem, L.hist, L.grid - L.hist, rec);
-  m.grid = carve_span<float>(smem, L.grid, L.lut - L.grid, rec);
+  m.grid = carve_span<float>(smem, L.grid, L.raw - L.grid, rec);
   m.lut_s = carve_span<float2>(smem, L.lut, L.total - L.lut, rec);
   return m;
 }
 
 // What every tile of a frame reads, set up once per frame by a CTA.
 struct FrameSetup {
-  float gains[3];  // the white balance the frame is processed with
-  float qblack[4];  // per quad position
-  float qinv[4];
-  float qgain[4];
   Span<const float2> lut;
   Span<const float> grid;  // lens shading gains: shared memory when they fit
   float lut_scale;
@@ -93,7 +94,7 @@ __device__ __forceinline__ Span<const float> frame_grid(const FrameDesc& p, cons
   return p.lsc != nullptr && gains <= kGridSmemGains ? Span<const float>(m.grid) : p.lsc;
 }
 
-// Reads the frame's gains (its estimate, for auto white balance) and, with
+// Reads the frame's gains (its estimate, for auto white balance) into m.quad and, with
 // kFill, fills the frame's shared memory (fill_frame_smem, its copies waited
 // for; without kFill the caller filled it before and waits for the copies).
 // The caller synchronises the block before the first tile.
@@ -101,14 +102,11 @@ template <bool kLutSmem, bool kFill = true>
 __device__ __forceinline__ FrameSetup setup_frame(const FrameDesc& p, const TileSmem& m) {
   if constexpr (kFill) fill_frame_smem<kLutSmem>(p, m);
   FrameSetup f;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) f.gains[k] = p.auto_wb ? __ldcg(&p.scratch->awb_gains[k]) : p.wb[k];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int ch = p.cfa[k];
-    f.qblack[k] = p.black[ch];
-    f.qinv[k] = p.inv_range[ch];
-    f.qgain[k] = f.gains[color_of(ch)];
+  if (threadIdx.x < kQuadFloats) {
+    const int t = threadIdx.x;
+    const int ch = t < 12 ? cfa_of(p.pattern, t & 3) : 0;
+    const int color = t < 12 ? color_of(ch) : t - 12;
+    m.quad[t] = t < 4 ? p.black[ch] : t < 8 ? p.inv_range[ch] : p.auto_wb ? __ldcg(&p.scratch->awb_gains[color]) : p.wb[color];
   }
   f.grid = frame_grid(p, m);
   f.lut = kLutSmem ? m.lut_s : p.tone;
@@ -142,18 +140,17 @@ __device__ __forceinline__ void unit_rows2(int t, int& r, int& uc) {
   r = 8 * w + 2 * (((l >> 2) & 1) + ((l >> 4) << 1));
 }
 
-__device__ __forceinline__ void unit_rc(int u, bool same_parity, int& r, int& uc) {
+__device__ __forceinline__ void unit_rc(int u, int& r, int& uc) {
   const int w = u >> 5;
   const int l = u & 31;
   const int ro = ((l >> 2) & 1) + ((l >> 4) << 1);  // 0..3
   uc = (l & 3) | (((l >> 3) & 1) << 2);
-  r = same_parity ? ((w >> 1) << 3) + 2 * ro + (w & 1) : 4 * w + ro;
+  r = ((w >> 1) << 3) + 2 * ro + (w & 1);
 }
 
 // The per-pixel tail of four pairs of one output row (pixels x .. x + 3 and
 // x + 32 .. x + 35 of row y): colour matrix, statistics, tone, store and
-// histograms, with the per-pixel guards only where the row leaves the image
-// or the output rows are not 16-byte aligned. kOutSel: the output format
+// histograms, with the per-pixel guards only where the row leaves the image. kOutSel: the output format
 // fixed at compile time (the single-frame kernels), or -1 to choose it per
 // unit (the batch kernel).
 template <int kOutSel, bool kLutSmem>
@@ -163,48 +160,33 @@ __device__ __forceinline__ void finish_row(const FrameDesc& p, const FrameSetup&
   if (y >= p.height) return;
   const int nl = min(max(p.width - x, 0), 4);
   const int nr = min(max(p.width - x - kHalf, 0), 4);
-  if (nl == 4 && nr == 4 && p.out_vector) {
+  if (nl == 4 && nr == 4) {
     if constexpr (kOutSel < 0) {
-      finish_pairs_any<kLutSmem, true>(p, rgb, x, y, nl, nr, f.lut, f.lut_scale, f.want_stats, f.want_hist, hist, sums,
-                                       npix);
+      finish_pairs_any<kLutSmem, true>(p, rgb, x, y, nl, nr, f.lut, f.lut_scale, f.want_hist, hist, sums, npix);
     } else {
-      finish_pairs<kOutSel, kLutSmem, true>(p, rgb, x, y, nl, nr, f.lut, f.lut_scale, f.want_stats, f.want_hist, hist,
-                                            sums, npix);
+      finish_pairs<kOutSel, kLutSmem, true>(p, rgb, x, y, nl, nr, f.lut, f.lut_scale, f.want_hist, hist, sums, npix);
     }
   } else {
     if constexpr (kOutSel < 0) {
-      finish_pairs_any<kLutSmem, false>(p, rgb, x, y, nl, nr, f.lut, f.lut_scale, f.want_stats, f.want_hist, hist,
-                                        sums, npix);
+      finish_pairs_any<kLutSmem, false>(p, rgb, x, y, nl, nr, f.lut, f.lut_scale, f.want_hist, hist, sums, npix);
     } else {
-      finish_pairs<kOutSel, kLutSmem, false>(p, rgb, x, y, nl, nr, f.lut, f.lut_scale, f.want_stats, f.want_hist,
-                                             hist, sums, npix);
+      finish_pairs<kOutSel, kLutSmem, false>(p, rgb, x, y, nl, nr, f.lut, f.lut_scale, f.want_hist, hist, sums, npix);
     }
   }
 }
 
-// A hook that does nothing (run_tile's default hooks).
-struct NoHook {
-  __device__ __forceinline__ void operator()() const {}
-};
-
-// One 64x64 tile at (x0, y0) (kTileH rows). Its box is waited for on `bar`.
-// Hooks, all run by every thread: `after_lsc()` once the tile's lens shading
-// maps and table are built, before the box wait and phase A (the frame's
-// gains may be read there); `after_a()` after phase A, when the box is free
-// again (to claim or prefetch the next tile); `before_c()` before phase C.
-// Adds the tile's statistics sums and saturated count to `acc` (per thread).
-
-template <bool kMalvar, bool kSharpen, int kLayout, bool kLutSmem, class AfterA, int kOutSel = -1, int kTileH = kTH,
-          class BeforeC = NoHook, class AfterLsc = NoHook>
-__device__ __forceinline__ void run_tile(const FrameDesc& p, const FrameSetup& f, const TileSmem& m, int* minmax,
-                                         int x0, int y0, bool use_tma, uint64_t* bar, uint32_t& phase,
-                                         u64 (&acc)[4], AfterA after_a, BeforeC before_c = BeforeC{},
-                                         AfterLsc after_lsc = AfterLsc{}) {
-  using G = Geom<kSharpen, kTileH>;
-  constexpr int kPat = kLayout * 2;
-  const int tid = threadIdx.x;
+// A tile's set-up and phase A: its lens shading maps and table, its box (waited
+// for on `bar`, or filled without TMA), its samples; returns the thread's
+// saturated count. The caller synchronises the block. `after_lsc()`, run by
+// every thread, comes once the maps and table are built and before anything
+// reads the frame's gains (without TMA, before the box is filled).
+template <int kHalo, int kTileH, class AfterLsc>
+__device__ __forceinline__ unsigned int tile_samples(const FrameDesc& p, const FrameSetup& f, const TileSmem& m,
+                                                     int* minmax, int x0, int y0, bool use_tma, uint64_t* bar,
+                                                     uint32_t& phase, AfterLsc after_lsc) {
+  constexpr int kSH = kTileH + 2 * kHalo;
   const int box_bytes = box_row_bytes(p.raw_format);
-  const bool interior = x0 >= 4 && y0 >= G::kHalo && x0 + kSW - 4 <= p.width && y0 + kTileH + G::kHalo <= p.height;
+  const bool interior = x0 >= 4 && y0 >= kHalo && x0 + kSW - 4 <= p.width && y0 + kTileH + kHalo <= p.height;
   TileCtx t;
   t.x0 = x0;
   t.y0 = y0;
@@ -215,27 +197,73 @@ __device__ __forceinline__ void run_tile(const FrameDesc& p, const FrameSetup& f
   t.row_ty = m.row_ty;
   t.table = m.table;
   t.grid = f.grid;
-  t.lt = interior ? build_lsc_inner(p, f.grid, p.pattern, x0 - 4, y0 - G::kHalo, G::kSH, m.col_mx, m.col_ix,
-                                    m.col_tx, m.row_my, m.row_k, m.row_ty, span_cast<float>(m.table), minmax)
-                  : build_lsc<true>(p, f.grid, p.pattern, x0 - 4, kSW, y0 - G::kHalo, G::kSH, true, p.width + 3,
-                                    p.height + G::kHalo - 1, m.col_mx, m.col_ix, m.col_tx, m.row_my, m.row_k, m.row_ty,
-                                    span_cast<float>(m.table), minmax);
-  after_lsc();
-  if (use_tma) {
-    if (!mbar_wait(bar, phase) && tid == 0) report_wait_timeout(p.scratch);
-    phase ^= 1U;
-  }
-
-  // A. Samples of the tile and its halo, preprocessed once, as pairs.
-  unsigned int saturated;
   if (!use_tma) {
-    saturated = phase_a2_fmt<2, G::kHalo, kTileH>(p, t, m.P, box_bytes, f.qblack, f.qinv, f.qgain, f.want_stats);
-  } else if (interior) {
-    saturated = phase_a2_fmt<0, G::kHalo, kTileH>(p, t, m.P, box_bytes, f.qblack, f.qinv, f.qgain, f.want_stats);
-  } else {
-    saturated = phase_a2_fmt<1, G::kHalo, kTileH>(p, t, m.P, box_bytes, f.qblack, f.qinv, f.qgain, f.want_stats);
+    after_lsc();  // raw samples are read from here on
+    fill_box(p, m.box, box_bytes, kSH, box_x(p.raw_format, x0) * (p.raw_format == kRawU16 ? 2 : 1), y0 - kHalo);
   }
-  acc[3] += saturated;
+  t.lt = interior ? build_lsc_inner(p, f.grid, p.pattern, x0 - 4, y0 - kHalo, kSH, m.col_mx, m.col_ix, m.col_tx, m.row_my,
+                                    m.row_k, m.row_ty, span_cast<float>(m.table), minmax)
+                  : build_lsc<true>(p, f.grid, p.pattern, x0 - 4, kSW, y0 - kHalo, kSH, true, p.width + 3,
+                                    p.height + kHalo - 1, m.col_mx, m.col_ix, m.col_tx, m.row_my, m.row_k, m.row_ty,
+                                    span_cast<float>(m.table), minmax);
+  if (use_tma) {
+    after_lsc();
+    if (!mbar_wait(bar, phase) && threadIdx.x == 0) report_wait_timeout(p.scratch);
+    phase ^= 1U;
+  } else {
+    box_filled();
+    __syncthreads();
+  }
+  return phase_a2<kHalo, kTileH>(p, t, m.P, box_bytes, span_cast<const float2>(m.quad), f.want_stats, interior);
+}
+
+// RGB of four pairs of output row r, sharpened from the planes.
+__device__ __forceinline__ void sharpened_row(const TileSmem& m, int r, int uc, float amount, float2 (&rgb)[4][3]) {
+  float2 o[4];
+  sharpen_row1(m.R, r, uc, bc2(amount), o);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) rgb[i][0] = o[i];
+  sharpen_row1(m.G, r, uc, bc2(amount), o);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) rgb[i][1] = o[i];
+  sharpen_row1(m.B, r, uc, bc2(amount), o);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) rgb[i][2] = o[i];
+}
+
+// RGB of four pairs of output row r straight from the samples.
+template <bool kMalvar, int kPat>
+__device__ __forceinline__ void demosaiced_row(const TileSmem& m, int r, int uc, float2 (&rgb)[4][3]) {
+  if (r & 1) {
+    demosaic_row4<kMalvar, kPat, 1>(m.P, r, uc, rgb);
+  } else {
+    demosaic_row4<kMalvar, kPat, 0>(m.P, r, uc, rgb);
+  }
+}
+
+__device__ __forceinline__ void swap_red_blue(float2 (&rgb)[4][3]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 red = rgb[i][0];
+    rgb[i][0] = rgb[i][2];
+    rgb[i][2] = red;
+  }
+}
+
+// One 64x64 tile at (x0, y0) (kTileH rows) of the single-frame kernel.
+// Hooks, all run by every thread: `after_lsc()` as in tile_samples;
+// `after_a()` after phase A, when the box is free again (to claim the next
+// tile); `before_c()` before phase C. Adds the tile's statistics sums and
+// saturated count to `acc` (per thread).
+template <bool kMalvar, bool kSharpen, int kLayout, bool kLutSmem, int kOutSel, int kTileH, class AfterA, class BeforeC,
+          class AfterLsc>
+__device__ __forceinline__ void run_tile(const FrameDesc& p, const FrameSetup& f, const TileSmem& m, int* minmax,
+                                         int x0, int y0, bool use_tma, uint64_t* bar, uint32_t& phase,
+                                         u64 (&acc)[4], AfterA after_a, BeforeC before_c, AfterLsc after_lsc) {
+  constexpr int kPat = kLayout * 2;
+  const int tid = threadIdx.x;
+  // A. Samples of the tile and its halo, preprocessed once, as pairs.
+  acc[3] += tile_samples<Geom<kSharpen, kTileH>::kHalo, kTileH>(p, f, m, minmax, x0, y0, use_tma, bar, phase, after_lsc);
   __syncthreads();
   after_a();
 
@@ -251,7 +279,7 @@ __device__ __forceinline__ void run_tile(const FrameDesc& p, const FrameSetup& f
   //    of at most 2^20).
   unsigned int sums[3] = {0U, 0U, 0U};
   unsigned int npix = 0;
-  if constexpr (kSharpen && kOutSel >= 0 && kTileH == kTH) {
+  if constexpr (kSharpen && kTileH == kTH) {
     // One unit per thread: output rows r and r + 1 of group uc, whose RGB
     // rows r .. r + 3 each plane loads once.
     int r, uc;
@@ -280,41 +308,18 @@ __device__ __forceinline__ void run_tile(const FrameDesc& p, const FrameSetup& f
     finish_row<kOutSel, kLutSmem>(p, f, m.hist, rgb0, x0 + 4 * uc, y0 + r, sums, npix);
     finish_row<kOutSel, kLutSmem>(p, f, m.hist, rgb1, x0 + 4 * uc, y0 + r + 1, sums, npix);
   } else {
-    // Units of four pairs of one row, kTileH / 32 per thread: sharpened (the
-    // batch kernel, whose output format is chosen per unit, keeps one call
-    // site of the finish; and short tiles), or demosaiced straight from the
-    // samples.
+    // Units of four pairs of one row, kTileH / 32 per thread: sharpened (short
+    // tiles), or demosaiced straight from the samples.
 #pragma unroll 1
     for (int k = 0; k < kTileH / 32; ++k) {
       int r, uc;
-      unit_rc(tid + k * kThreads, true, r, uc);
+      unit_rc(tid + k * kThreads, r, uc);
       float2 rgb[4][3];
       if constexpr (kSharpen) {
-        const float2 amount = bc2(p.sharpen);
-        float2 o[4];
-        sharpen_row1(m.R, r, uc, amount, o);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) rgb[i][0] = o[i];
-        sharpen_row1(m.G, r, uc, amount, o);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) rgb[i][1] = o[i];
-        sharpen_row1(m.B, r, uc, amount, o);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) rgb[i][2] = o[i];
+        sharpened_row(m, r, uc, p.sharpen, rgb);
       } else {
-        if (r & 1) {
-          demosaic_row4<kMalvar, kPat, 1>(m.P, r, uc, rgb);
-        } else {
-          demosaic_row4<kMalvar, kPat, 0>(m.P, r, uc, rgb);
-        }
-        if (f.swap_rb) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float2 red = rgb[i][0];
-            rgb[i][0] = rgb[i][2];
-            rgb[i][2] = red;
-          }
-        }
+        demosaiced_row<kMalvar, kPat>(m, r, uc, rgb);
+        if (f.swap_rb) swap_red_blue(rgb);
       }
       finish_row<kOutSel, kLutSmem>(p, f, m.hist, rgb, x0 + 4 * uc, y0 + r, sums, npix);
     }
@@ -329,7 +334,7 @@ __device__ __forceinline__ void run_tile(const FrameDesc& p, const FrameSetup& f
 // into the frame's scratch; the CTA that completes the frame's tile count
 // writes the user's histogram and statistics and clears the scratch (and
 // the tile claims of the single-frame pass). `red` holds 4 x kWarps values.
-__device__ void flush_frame(const FrameDesc& p, const FrameSetup& f, const u64 (&acc)[4], Span<unsigned int> hist,
+__device__ void flush_frame(const FrameDesc& p, const FrameSetup& f, const u64 (&acc)[4], const TileSmem& m,
                             u64* red, bool* last, unsigned int tiles_done, unsigned int tiles_total) {
   Span<Scratch> sc = p.scratch;
   const int tid = threadIdx.x;
@@ -355,32 +360,52 @@ __device__ void flush_frame(const FrameDesc& p, const FrameSetup& f, const u64 (
     const Span<unsigned long long> pairs =
         span_cast<unsigned long long>(sub_span(sc, &sc->hist[0], kHistChannels * kHistBins));
     for (int i = tid; i < kHistChannels * kHistBins / 2; i += kThreads) {
-      const uint2 h = span_cast<const uint2>(hist)[i];
+      const uint2 h = span_cast<const uint2>(m.hist)[i];
       if ((h.x | h.y) != 0U) atomicAdd(&pairs[i], (static_cast<unsigned long long>(h.y) << 32) | h.x);
     }
   }
-  __threadfence();
   __syncthreads();
-  if (tid == 0) *last = atomicAdd(&sc->main_done, tiles_done) + tiles_done == tiles_total;
+  if (tid == 0) {
+    // The block's atomics come before the count that hands the frame over
+    // (the barrier above orders them before this thread's fence).
+    __threadfence();
+    *last = atomicAdd(&sc->main_done, tiles_done) + tiles_done == tiles_total;
+  }
   __syncthreads();
   if (!*last) return;
   __threadfence();
-  if (f.want_hist) {
-    const Span<unsigned int> bins = sub_span(sc, &sc->hist[0], kHistChannels * kHistBins);
-    for (int i = tid; i < kHistChannels * kHistBins; i += kThreads) {
-      p.hist_out[i] = __ldcg(&bins[i]);
-      bins[i] = 0U;
-    }
-  }
-  if (f.want_stats && tid == 0) {
-    const u64 sum[3] = {__ldcg(&sc->sum[0]), __ldcg(&sc->sum[1]), __ldcg(&sc->sum[2])};
-    finish_stats(p, sum, __ldcg(&sc->saturated), f.gains);
-    sc->sum[0] = sc->sum[1] = sc->sum[2] = 0;
-    sc->saturated = 0;
-  }
+  // The frame's end is one chain of round trips to L2 that nothing hides, so
+  // warp 0 forms the statistics while the others move the histogram, all of a
+  // thread's bins loaded before the first is stored.
   if (tid == 0) {
+    if (f.want_stats) {
+      const u64 sum[3] = {__ldcg(&sc->sum[0]), __ldcg(&sc->sum[1]), __ldcg(&sc->sum[2])};
+      const float gains[3] = {m.quad[12], m.quad[13], m.quad[14]};
+      finish_stats(p, sum, __ldcg(&sc->saturated), gains);
+      sc->sum[0] = sc->sum[1] = sc->sum[2] = 0;
+      sc->saturated = 0;
+    }
     sc->main_done = 0;
     sc->tile_next = 0;
+  }
+  if (f.want_hist && tid >= 32) {
+    constexpr int kMovers = kThreads - 32;
+    constexpr int kBins = kHistChannels * kHistBins;
+    const Span<unsigned int> bins = sub_span(sc, &sc->hist[0], kBins);
+    unsigned int n[(kBins + kMovers - 1) / kMovers];
+#pragma unroll
+    for (int k = 0; k < (kBins + kMovers - 1) / kMovers; ++k) {
+      const int i = tid - 32 + k * kMovers;
+      n[k] = i < kBins ? __ldcg(&bins[i]) : 0U;
+    }
+#pragma unroll
+    for (int k = 0; k < (kBins + kMovers - 1) / kMovers; ++k) {
+      const int i = tid - 32 + k * kMovers;
+      if (i < kBins) {
+        p.hist_out[i] = n[k];
+        bins[i] = 0U;
+      }
+    }
   }
 }
 
@@ -407,13 +432,15 @@ __global__ void __launch_bounds__(kThreads, kTileH == kTH ? 2 : 3)
     const int x0 = (t - ty * tiles_x) * kTW;
     tma_load_2d(&map, m.box, &bar, box_x(fmt, x0), ty * kTileH - G::kHalo, static_cast<unsigned int>(G::kSH * box_bytes));
   };
-  // The first tile's box reads only the input frame: it is requested before
-  // the wait below (the barrier initialised and made visible to the copy
-  // engine first; the other threads meet it after the block barrier).
+  // Behind a statistics pass, the first tile's box (which reads only the input
+  // frame, as that pass did) is requested before the wait below, the barrier
+  // initialised and made visible to the copy engine first; the other threads
+  // meet it after the block barrier. Without one the kernel queued before may
+  // be anything, and raw samples are read after the wait.
   if (use_tma && threadIdx.x == 0) {
     mbar_init(&bar);
     fence_async_shared();
-    if (static_cast<int>(blockIdx.x) < tiles) issue(blockIdx.x);
+    if (p.auto_wb && static_cast<int>(blockIdx.x) < tiles) issue(blockIdx.x);
   }
   fill_frame_smem<kLutSmem>(p, m);
   // The frame's set-up waits for the statistics pass (its gains); the first
@@ -426,18 +453,21 @@ __global__ void __launch_bounds__(kThreads, kTileH == kTH ? 2 : 3)
   bool waited = false;
   const auto wait_frame = [&] {
     if (waited) return;
-    // Launched as a programmatic dependent of the statistics pass, this
-    // kernel becomes resident on the SMs that pass leaves while it finishes;
-    // the wait returns once the pass has completed and its writes (the gains
-    // that setup_frame reads) are visible. Without a programmatic launch it
-    // returns at once.
+    // Launched as a programmatic dependent of the statistics pass (or, with
+    // manual white balance, of the previous frame's tile pass), this kernel
+    // becomes resident on the SMs that pass leaves while it finishes; the wait
+    // returns once the pass has completed and its writes (the gains that
+    // setup_frame reads, the cleared sums) are visible. Without a programmatic
+    // launch it returns at once.
     griddep_wait();
+    if (use_tma && !p.auto_wb && threadIdx.x == 0 && static_cast<int>(blockIdx.x) < tiles) issue(blockIdx.x);
     // The next frame's statistics pass may launch now (when queued right
     // behind this kernel): it sums its own raw frame on the SMs this pass
     // leaves as it finishes, and waits for this pass's completion before its
     // estimate touches the white balance state read here.
     griddep_launch_dependents();
     f = setup_frame<kLutSmem, false>(p, m);
+    __syncthreads();  // the constants in m.quad, for every thread's phase A
     waited = true;
   };
 
@@ -478,14 +508,13 @@ __global__ void __launch_bounds__(kThreads, kTileH == kTH ? 2 : 3)
     const auto before_c = [&] {
       if constexpr (kSharpen) request();
     };
-    run_tile<kMalvar, kSharpen, kLayout, kLutSmem, decltype(after_a), kOut, kTileH, decltype(before_c),
-             decltype(wait_frame)>(p, f, m, minmax, x0, ty * kTileH, use_tma != 0, &bar, phase, acc, after_a, before_c,
-                                   wait_frame);
+    run_tile<kMalvar, kSharpen, kLayout, kLutSmem, kOut, kTileH>(p, f, m, minmax, x0, ty * kTileH, use_tma != 0, &bar,
+                                                                 phase, acc, after_a, before_c, wait_frame);
     ++done;
     tile = next_tile;  // written before run_tile's closing barrier
   }
   wait_frame();  // a CTA without a tile still takes part in the flush
-  flush_frame(p, f, acc, m.hist, red, &last, done, static_cast<unsigned int>(tiles));
+  flush_frame(p, f, acc, m, red, &last, done, static_cast<unsigned int>(tiles));
 }
 
 template <bool kMalvar, bool kSharpen, int kOut, int kTileH>

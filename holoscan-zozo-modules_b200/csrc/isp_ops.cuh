@@ -66,10 +66,15 @@ __device__ __forceinline__ float exact_scale_add(float a, float k, float b) { re
 // that consumes it (one rounding instead of two), whatever rounding mode the
 // instructions name; measured on this toolchain, about half of such sums
 // then differ from the reference in the last bit. Scalar operations with an
-// explicit rounding mode are never fused. So in this code a two-lane product
-// feeds only a multiply, an operand of a fused multiply-add, a per-lane
-// (scalar) add, or a two-lane add when the product is exact (a scale by a
-// power of two), where one rounding and two give the same result.
+// explicit rounding mode are never fused, and neither is a product that is
+// an operand of a fused multiply-add. So a sum that consumes a two-lane
+// product p runs as p * 1 + q with the 1 read from constant memory, whose
+// value the assembler does not know (psum2 and the forms beside it): one
+// instruction whose only rounding is the sum's, where two scalar adds took
+// two. Apart from these, a two-lane product feeds only a multiply, an
+// operand of a fused multiply-add, a per-lane (scalar) add, or a two-lane add
+// when the product is exact (a scale by a power of two), where one rounding
+// and two give the same result.
 #define ISP_F32X2_BINARY(NAME, OP)                                                                      \
   __device__ __forceinline__ float2 NAME(float2 a, float2 b) {                                          \
     float2 r;                                                                                           \
@@ -97,10 +102,21 @@ __device__ __forceinline__ float2 exact_scale_add2(float2 a, float2 k, float2 b)
 }
 // magic_trunc per lane: 2^23 + trunc(x) for 0 <= x < 2^23 (x not a product).
 __device__ __forceinline__ float2 magic_trunc2(float2 x) { return add2_rz(x, bc2(kTwo23)); }
-// Per-lane scalar forms, for sums that consume a two-lane product.
-__device__ __forceinline__ float2 add_lanes(float2 a, float2 b) { return make_float2(fadd(a.x, b.x), fadd(a.y, b.y)); }
-__device__ __forceinline__ float2 sub_lanes(float2 a, float2 b) { return make_float2(fsub(a.x, b.x), fsub(a.y, b.y)); }
-__device__ __forceinline__ float2 magic_trunc_lanes(float2 x) { return make_float2(magic_trunc(x.x), magic_trunc(x.y)); }
+// 1 and -1 that the assembler cannot fold (the host may write constant memory).
+static __constant__ float g_one = 1.0F;
+static __constant__ float g_minus_one = -1.0F;
+// p + q, q - p and 2^23 + trunc(p) per lane, where p (and q) may be two-lane products.
+__device__ __forceinline__ float2 psum2(float2 p, float2 q) { return exact_scale_add2(p, bc2(g_one), q); }
+__device__ __forceinline__ float2 pdiff2(float2 q, float2 p) { return exact_scale_add2(p, bc2(g_minus_one), q); }
+__device__ __forceinline__ float2 magic_trunc_product2(float2 p) {
+  const float one = g_one;
+  float2 r;
+  asm("{ .reg .b64 a, k, b, d; mov.b64 a, {%2, %3}; mov.b64 k, {%4, %4}; mov.b64 b, {%5, %5}; "
+      "fma.rz.f32x2 d, a, k, b; mov.b64 {%0, %1}, d; }"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(p.x), "f"(p.y), "f"(one), "f"(kTwo23));
+  return r;
+}
 // (float)n per lane from n OR-ed with kTwo23Bits.
 __device__ __forceinline__ float2 magic_to_float2(unsigned int a_bits, unsigned int b_bits) {
   return sub2(make_float2(__uint_as_float(a_bits), __uint_as_float(b_bits)), bc2(kTwo23));

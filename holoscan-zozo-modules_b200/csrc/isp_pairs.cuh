@@ -18,6 +18,16 @@
 //   C. per unit of four pairs of one row: demosaic (or sharpen,
 //      isp_math.hpp:219-227), colour matrix, statistics sums, tone, store and
 //      histogram codes (isp_math.hpp:229-305).
+//
+// What bounds the pass is the shared-memory pipe: ncu counts 57 wavefronts per
+// 32 pixels of a sharpened 3840x2160 RAW10 frame, 75 % of the pipe while the
+// SMs work (issue slots 59 %, FMA pipe 44 %): tone table lookups 20 and
+// histogram atomics 13, most of them bank conflicts that the data decides,
+// the rest the planes and tables of the phases. So the phases are shaped to
+// touch shared memory less (A keeps its table rows in registers, B's units are
+// six rows high), and sums of products run two lanes at a time (isp_ops.cuh).
+// The frame's pass went from 101.0 to 91.9 us with these, a 1920x1080 16-bit
+// one with the same stages from 43.3 to 38.8 us.
 #pragma once
 
 #include "isp_common.cuh"
@@ -51,169 +61,204 @@ __device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); 
 
 // A. Samples of the tile and its halo as pairs; returns the saturated count
 //    of the tile's own samples (raw >= white, isp_math.hpp:316), each counted
-//    once. kSrc: 0 interior tile from the TMA box, 1 edge tile from the box
-//    (mirrored columns), 2 no box (global loads, mirrored).
-template <int kFmt, int kSrc, int kHalo, int kTileH>
+//    once.
+//
+//    A thread takes one unit of four pairs across and kRowsEach rows of one
+//    parity, two apart: the row parity's constants, and the two rows of the
+//    lens shading table that these rows lie between, stay in registers (with
+//    one row per unit the table's four loads per eight samples were the
+//    phase's largest share of shared-memory traffic). The two 16-byte halves
+//    of a unit go to shared memory in an order that alternates every four
+//    lanes (`flip`), so that a quarter-warp's stores and table loads, 32
+//    bytes apart, meet every bank once.
+//
+//    One body serves every raw format and every tile: the unpacking branches
+//    on the format, and only the units of an edge tile whose columns reach
+//    past the image are unpacked sample by sample. (One copy per format, tile
+//    kind and shading kept what they share alive across all of them and
+//    spilled, and the batch kernel, whose CTAs mix formats, waited for
+//    instructions.)
+template <int kHalo, int kTileH>
 __device__ __forceinline__ unsigned int phase_a2(const FrameDesc& p, const TileCtx& t, Span<float2> P, int box_bytes,
-                                                 const float (&qblack)[4], const float (&qinv)[4],
-                                                 const float (&qgain)[4], bool want_stats) {
+                                                 Span<const float2> quad, bool want_stats, bool interior) {
   constexpr int kSH = kTileH + 2 * kHalo;
+  constexpr int kGroups = kThreads / kUnitsA / 2;  // groups of rows of each parity
+  constexpr int kRowsEach = (kSH / 2 + kGroups - 1) / kGroups;
+  const int tid = threadIdx.x;
+  const int q = tid / kUnitsA;
+  const int u = tid - q * kUnitsA;
+  const int par = q & 1;  // row parity: y0 - halo is even
+  const int first = 2 * (q >> 1) * kRowsEach + par;
+  const int flip = ((tid >> 2) & 1) * 2;
+  const int fmt = p.raw_format;
   const unsigned int white = static_cast<unsigned int>(p.white);
   unsigned int saturated = 0;
-  for (int unit = threadIdx.x; unit < kUnitsA * kSH; unit += kThreads) {
-    const int j = unit / kUnitsA;
-    const int u = unit - j * kUnitsA;
-    const int par = j & 1;  // row parity: y0 - halo is even
-    unsigned int sl[4], sr[4];  // samples 4u + k and 4u + 32 + k
-    if constexpr (kSrc == 0) {
-      Span<const uint8_t> row = t.box + j * box_bytes;
-      unpack4(kFmt, row, u, sl);
-      unpack4(kFmt, row, u + kHalf / 4, sr);
-    } else if constexpr (kSrc == 1) {
-      Span<const uint8_t> row = t.box + (t.row_my[j] - (t.y0 - kHalo)) * box_bytes;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        sl[k] = unpack1(kFmt, row, t.col_mx[4 * u + k], t.x0);
-        sr[k] = unpack1(kFmt, row, t.col_mx[4 * u + kHalf + k], t.x0);
-      }
+  if (q >= 2 * kGroups) return saturated;
+  // The rows' two quad positions' constants.
+  const float2 black = quad[par], inv = quad[2 + par], gain = quad[4 + par];
+  const int pl = p.lsc_channels == 4 ? par : 0;
+  // The unit's left and right columns: unpacked as they lie in the box when
+  // inside the image, or when the tile has no use for them (further right
+  // than any mirrored neighbour); one by one from their mirrored columns else.
+  const int xl = t.x0 - 4 + 4 * u;
+  const int xr = xl + kHalf;
+  const bool plain_l = interior || (xl >= 0 && xl + 4 <= p.width) || xl > p.width + 3;
+  const bool plain_r = interior || xr + 4 <= p.width || xr > p.width + 3;
+  int cell = -1;           // the table row that top and step were read for
+  float2 top[4], step[4];  // T[k] and T[k + 1] - T[k] of the unit's pairs, in the unit's (flipped) order
+#pragma unroll 1
+  for (int i = 0; i < kRowsEach; ++i) {
+    const int j = first + 2 * i;
+    if (j >= kSH) break;
+    unsigned int wl[2], wr[2];  // samples 4u + k and 4u + 32 + k, as 16-bit halves
+    Span<const uint8_t> row = t.box + (interior ? j : t.row_my[j] - (t.y0 - kHalo)) * box_bytes;
+    if (plain_l) {
+      unpack4(fmt, row, u, wl);
     } else {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        sl[k] = static_cast<unsigned int>(load_raw(p, t.col_mx[4 * u + k], t.row_my[j]));
-        sr[k] = static_cast<unsigned int>(load_raw(p, t.col_mx[4 * u + kHalf + k], t.row_my[j]));
-      }
+      const uint2 e = unpack_edge4(fmt, row, t.col_mx + 4 * u, t.x0);
+      wl[0] = e.x;
+      wl[1] = e.y;
+    }
+    if (plain_r) {
+      unpack4(fmt, row, u + kHalf / 4, wr);
+    } else {
+      const uint2 e = unpack_edge4(fmt, row, t.col_mx + 4 * u + kHalf, t.x0);
+      wr[0] = e.x;
+      wr[1] = e.y;
     }
     // Tile samples are s = 4 .. 67: the left lanes of units 1..8 hold 4..35,
-    // their right lanes 36..67.
-    if (want_stats && j >= kHalo && j < kHalo + kTileH && u >= 1 && u <= kHalf / 4) {
-      const int y = t.y0 + j - kHalo;
-      const int xl = t.x0 + 4 * (u - 1);
-      if (y < p.height) {
+    // their right lanes 36..67. Saturated samples are rare: one maximum over
+    // the unit's eight samples decides whether any is counted.
+    if (want_stats && any_half_at_least(__vmaxu2(__vmaxu2(wl[0], wl[1]), __vmaxu2(wr[0], wr[1])), white)) {
+      if (j >= kHalo && j < kHalo + kTileH && u >= 1 && u <= kHalf / 4 && t.y0 + j - kHalo < p.height) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          saturated += (xl + k < p.width && sl[k] >= white) ? 1U : 0U;
-          saturated += (xl + kHalf + k < p.width && sr[k] >= white) ? 1U : 0U;
+          const unsigned int l = (wl[k >> 1] >> (16 * (k & 1))) & 0xFFFFU, r = (wr[k >> 1] >> (16 * (k & 1))) & 0xFFFFU;
+          saturated += (xl + k < p.width && l >= white) ? 1U : 0U;
+          saturated += (xr + k < p.width && r >= white) ? 1U : 0U;
         }
       }
     }
-    // The row's two quad positions' constants.
-    const float bl0 = par ? qblack[2] : qblack[0];
-    const float bl1 = par ? qblack[3] : qblack[1];
-    const float iv0 = par ? qinv[2] : qinv[0];
-    const float iv1 = par ? qinv[3] : qinv[1];
-    const float gn0 = par ? qgain[2] : qgain[0];
-    const float gn1 = par ? qgain[3] : qgain[1];
-    float2 v[4];
+    // The halves in the order they are stored.
+    const unsigned int al = flip ? wl[1] : wl[0], bl = flip ? wl[0] : wl[1];
+    const unsigned int ar = flip ? wr[1] : wr[0], br = flip ? wr[0] : wr[1];
+    // linearize (isp_math.hpp:144-148): (raw - black) * inv_range, without its
+    // maximum with 0: all gains are positive, so a negative value stays
+    // negative up to the saturating multiply below, which makes it the 0 that
+    // the maximum would have made it.
+    float2 v[4] = {magic_to_float2(magic_low(al), magic_low(ar)), magic_to_float2(magic_high(al), magic_high(ar)),
+                   magic_to_float2(magic_low(bl), magic_low(br)), magic_to_float2(magic_high(bl), magic_high(br))};
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      // linearize (isp_math.hpp:144-148): max((raw - black) * inv_range, 0).
-      const float2 raw = magic_to_float2(sl[k] | kTwo23Bits, sr[k] | kTwo23Bits);
-      const float2 x = mul2(sub2(raw, bc2((k & 1) ? bl1 : bl0)), bc2((k & 1) ? iv1 : iv0));
-      v[k] = make_float2(fmaxf(x.x, 0.0F), fmaxf(x.y, 0.0F));
-    }
+    for (int k = 0; k < 4; ++k) v[k] = mul2(sub2(v[k], bc2((k & 1) ? black.y : black.x)), bc2((k & 1) ? inv.y : inv.x));
     if (t.lt.rows > 0) {
       if (t.lt.rows <= kLscTableRows) {
         const int kk = t.row_k[j];
-        const int pl = p.lsc_channels == 4 ? par : 0;
-        Span<const float2> r0 = t.table + (kk * 2 + pl) * kPW + 4 * u;
-        Span<const float2> r1 = t.table + ((kk + 1) * 2 + pl) * kPW + 4 * u;
-        const float4 a0 = lds4(r0), b0 = lds4(r0 + 2), a1 = lds4(r1), b1 = lds4(r1 + 2);
-        const float2 t0[4] = {lo2(a0), hi2(a0), lo2(b0), hi2(b0)};
-        const float2 t1[4] = {lo2(a1), hi2(a1), lo2(b1), hi2(b1)};
+        if (kk != cell) {
+          cell = kk;
+          Span<const float2> r0 = t.table + (kk * 2 + pl) * kPW + 4 * u;
+          Span<const float2> r1 = r0 + 2 * kPW;
+          const float4 a0 = lds4(r0 + flip), b0 = lds4(r0 + (flip ^ 2)), a1 = lds4(r1 + flip), b1 = lds4(r1 + (flip ^ 2));
+          top[0] = lo2(a0);
+          top[1] = hi2(a0);
+          top[2] = lo2(b0);
+          top[3] = hi2(b0);
+          step[0] = sub2(lo2(a1), top[0]);
+          step[1] = sub2(hi2(a1), top[1]);
+          step[2] = sub2(lo2(b1), top[2]);
+          step[3] = sub2(hi2(b1), top[3]);
+        }
         const float2 ty = bc2(t.row_ty[j]);
-        // top + (bottom - top) * ty (isp_math.hpp:121-140); the product is
-        // rounded, so the sum runs per lane (isp_ops.cuh).
+        // top + (bottom - top) * ty (isp_math.hpp:121-140).
 #pragma unroll
-        for (int k = 0; k < 4; ++k) v[k] = mul2(v[k], add_lanes(t0[k], mul2(sub2(t1[k], t0[k]), ty)));
+        for (int k = 0; k < 4; ++k) v[k] = mul2(v[k], psum2(mul2(step[k], ty), top[k]));
       } else {
+        // A grid too dense for the table: each gain from the grid.
+        const LscGrid g{t.grid, p.lsc_width, p.lsc_height, p.lsc_channels, p.lsc_sx, p.lsc_sy};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const int ch = p.cfa[(par << 1) | (k & 1)];
-          v[k].x = fmul(v[k].x, lens_shading_gain(p, t.grid, t.col_mx[4 * u + k], t.row_my[j], ch));
-          v[k].y = fmul(v[k].y, lens_shading_gain(p, t.grid, t.col_mx[4 * u + kHalf + k], t.row_my[j], ch));
+          const int ch = cfa_of(p.pattern, (par << 1) | (k & 1));
+          const int s = 4 * u + (k ^ flip);
+          v[k].x = fmul(v[k].x, lens_shading_gain_outline(g, t.col_mx[s], t.row_my[j], ch));
+          v[k].y = fmul(v[k].y, lens_shading_gain_outline(g, t.col_mx[s + kHalf], t.row_my[j], ch));
         }
       }
     }
-    // White balance and the clip to 1 (v >= 0): the saturating multiply.
+    // White balance and the clip to [0, 1]: the saturating multiply.
     Span<float2> dst = P + j * kPW;
-    const int sw = psw(j);
-    sts4(dst + ((4 * u) ^ sw), mul_sat2(v[0], bc2(gn0)), mul_sat2(v[1], bc2(gn1)));
-    sts4(dst + ((4 * u + 2) ^ sw), mul_sat2(v[2], bc2(gn0)), mul_sat2(v[3], bc2(gn1)));
+    const int sw = psw(j) ^ flip;
+    sts4(dst + ((4 * u) ^ sw), mul_sat2(v[0], bc2(gain.x)), mul_sat2(v[1], bc2(gain.y)));
+    sts4(dst + ((4 * u + 2) ^ sw), mul_sat2(v[2], bc2(gain.x)), mul_sat2(v[3], bc2(gain.y)));
   }
   return saturated;
 }
 
-template <int kSrc, int kHalo, int kTileH>
-__device__ __forceinline__ unsigned int phase_a2_fmt(const FrameDesc& p, const TileCtx& t, Span<float2> P, int box_bytes,
-                                                     const float (&qblack)[4], const float (&qinv)[4],
-                                                     const float (&qgain)[4], bool want_stats) {
-  // Global loads (no TMA box) read the format at run time in load_raw.
-  if constexpr (kSrc == 2) return phase_a2<kRawU8, kSrc, kHalo, kTileH>(p, t, P, box_bytes, qblack, qinv, qgain, want_stats);
-  switch (p.raw_format) {
-    case kRawU8: return phase_a2<kRawU8, kSrc, kHalo, kTileH>(p, t, P, box_bytes, qblack, qinv, qgain, want_stats);
-    case kRawU16: return phase_a2<kRawU16, kSrc, kHalo, kTileH>(p, t, P, box_bytes, qblack, qinv, qgain, want_stats);
-    case kRawRaw10: return phase_a2<kRawRaw10, kSrc, kHalo, kTileH>(p, t, P, box_bytes, qblack, qinv, qgain, want_stats);
-    default: return phase_a2<kRawRaw12, kSrc, kHalo, kTileH>(p, t, P, box_bytes, qblack, qinv, qgain, want_stats);
-  }
-}
-
 // B. (Sharpening) RGB of the tile and its ring into the paired planes, in
-//    units of 2 rows x 2 pairs: 33 x 17 units cover the 66 x 34 pairs.
+//    units of kRows rows x 2 pairs: 17 units across cover the 34 pairs, and
+//    kRows divides the kTileH + 2 rows.
 //    RGB pair (row cr, column q): pixels (q - 1, q + 31) of image row
 //    y0 - 1 + cr, whose sample pair is P[cr + 3][q + 3] (halo 4).
 //    With swap_rb the demosaic's red and blue go to the other planes: the
 //    demosaic runs as the layout's canonical pattern (RGGB or GRBG), and
 //    BGGR and GBRG trade red and blue.
+//    The kernel's limit is the shared-memory pipe, so a unit is as high as
+//    the block's threads allow: of 66 rows, 11 units of 6 (32 loads for 12
+//    pairs, one round of 187 threads) instead of 33 of 2 (16 for 4 pairs,
+//    three rounds). The unit's rows run one after the other through a window
+//    of five sample rows that the unrolled loop keeps in registers.
 template <bool kMalvar, int kPat, int kTileH>
 __device__ __forceinline__ void phase_b2(Span<const float2> P, Span<float2> R, Span<float2> G, Span<float2> B) {
-  constexpr int kUnitsQ = kCW2 / 2;                   // 17
-  constexpr int kUnits = (kTileH + 2) / 2 * kUnitsQ;  // 33 x 17 for 64 rows
+  constexpr int kUnitsQ = kCW2 / 2;  // 17
+  constexpr int kRows = (kTileH + 2) % 6 == 0 ? 6 : 2;
+  constexpr int kUnits = (kTileH + 2) / kRows * kUnitsQ;
+  static_assert((kTileH + 2) % kRows == 0 && kRows % 2 == 0, "whole units, each starting at an odd image row");
   for (int unit = threadIdx.x; unit < kUnits; unit += kThreads) {
     const int ur = unit / kUnitsQ;
     const int uq = unit - ur * kUnitsQ;
-    // Window w[a][b] = P[2ur + 1 + a][2uq + 1 + b]; rows 0 and 5 need columns
-    // 2..3, rows 1 and 4 columns 1..4, rows 2 and 3 columns 0..5 (Malvar);
-    // bilinear needs rows 1..4, columns 1..4.
-    float2 w[6][6] = {};
+    // Window row a holds P[kRows ur + 1 + a][2uq + 1 + b], b = 0 .. 5. As a
+    // pixel row's own row all six columns are needed, as a neighbour only
+    // columns 1 .. 4 (bilinear needs those alone, and no rows two away).
+    float2 w[kRows + 4][6];
+    const int base = kRows * ur + 1;
 #pragma unroll
-    for (int a = 0; a < 6; ++a) {
-      const int j = 2 * ur + 1 + a;
+    for (int a = 0; a < kRows + 4; ++a) {
+      if (!kMalvar && (a == 0 || a == kRows + 3)) continue;
+      const int j = base + a;
       Span<const float2> row = P + j * kPW;  // pair 2uq is w column -1
       const int sw = psw(j);
-      const bool edge = a == 0 || a == 5;
-      const bool mid = a == 2 || a == 3;
-      if (!kMalvar && edge) continue;
       const float4 m1 = lds4(row + ((2 * uq + 2) ^ sw)), m2 = lds4(row + ((2 * uq + 4) ^ sw));  // w columns 1..4
       w[a][1] = lo2(m1);
       w[a][2] = hi2(m1);
       w[a][3] = lo2(m2);
       w[a][4] = hi2(m2);
-      if (kMalvar && mid) {
+      if (kMalvar && a >= 2 && a < kRows + 2) {
         w[a][0] = hi2(lds4(row + ((2 * uq) ^ sw)));
         w[a][5] = lo2(lds4(row + ((2 * uq + 6) ^ sw)));
       }
-    }
-    float2 rgb[2][2][3];
-#pragma unroll
-    for (int dy = 0; dy < 2; ++dy) {
+      // Pixel row dy needs window rows dy .. dy + 4 (bilinear: dy + 1 .. dy + 3).
+      const int dy = kMalvar ? a - 4 : a - 3;
+      if (dy < 0 || dy >= kRows) continue;
+      float2 rgb[2][3];
 #pragma unroll
       for (int dq = 0; dq < 2; ++dq) {
         float2 n[5][5];
 #pragma unroll
-        for (int a = 0; a < 5; ++a) {
+        for (int c = 0; c < 5; ++c) {
 #pragma unroll
-          for (int b = 0; b < 5; ++b) n[a][b] = w[dy + a][dq + b];  // unused corners are never read
+          for (int b = 0; b < 5; ++b) {
+            // Taps outside the demosaic's support are never read.
+            const bool used = kMalvar ? (c == 2 || (b > 0 && b < 4 && (c != 0 && c != 4)) || b == 2)
+                                      : (c > 0 && c < 4 && b > 0 && b < 4);
+            n[c][b] = used ? w[dy + c][dq + b] : make_float2(0.0F, 0.0F);
+          }
         }
-        // Pixel row y0 - 1 + 2ur + dy, column x0 + 2uq + dq - 1: parities (dy + 1) & 1 and (dq + 1) & 1.
-        demosaic2<kMalvar>(n, cfa_of(kPat, (((dy + 1) & 1) << 1) | ((dq + 1) & 1)), rgb[dy][dq]);
+        // Pixel row y0 - 1 + kRows ur + dy, column x0 + 2uq + dq - 1: parities (dy + 1) & 1 and (dq + 1) & 1.
+        demosaic2<kMalvar>(n, cfa_of(kPat, (((dy + 1) & 1) << 1) | ((dq + 1) & 1)), rgb[dq]);
       }
-    }
-#pragma unroll
-    for (int dy = 0; dy < 2; ++dy) {
-      const int o = (2 * ur + dy) * kCW2 + 2 * cchunk(uq, ur & 1);  // csw(2 ur + dy) == ur & 1
-      sts4(R + o, rgb[dy][0][0], rgb[dy][1][0]);
-      sts4(G + o, rgb[dy][0][1], rgb[dy][1][1]);
-      sts4(B + o, rgb[dy][0][2], rgb[dy][1][2]);
+      const int cr = kRows * ur + dy;
+      const int o = cr * kCW2 + 2 * cchunk(uq, csw(cr));
+      sts4(R + o, rgb[0][0], rgb[1][0]);
+      sts4(G + o, rgb[0][1], rgb[1][1]);
+      sts4(B + o, rgb[0][2], rgb[1][2]);
     }
   }
 }
@@ -344,6 +389,27 @@ __device__ __forceinline__ float tone_lookup(Span<const float2> table, float m, 
   return fadd(e.x, fmul(frac, e.y));
 }
 
+// Adds one to bin `index - bias` of the block's histogram channel `channel`.
+__device__ __forceinline__ void count_code(Span<unsigned int> hist, int channel, unsigned int index, unsigned int bias) {
+#ifdef ISP_CHECKED
+  atomicAdd(&hist[channel * kHistBins + static_cast<int>(index - bias)], 1U);
+#else
+  // The shared address, the bias folded into its base (mod 2^32).
+  const uint32_t addr = smem_u32(hist) + 4U * channel * kHistBins - 4U * bias + 4U * index;
+  asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(addr) : "memory");
+#endif
+}
+
+// The luma code (2126 r + 7152 g + 722 b + 5000) / 10000 (isp_math.hpp:303-305)
+// of codes that carry `bias` each, as the top byte of one 32-bit sum: the
+// weights in units of 2^-24 and an offset a little above one half, which gives
+// the quotient for all 2^24 triples of codes (checked exhaustively) without
+// the division's wide multiply and without taking the bias off the codes.
+__device__ __forceinline__ unsigned int luma_of(unsigned int r, unsigned int g, unsigned int b, unsigned int bias) {
+  constexpr unsigned int kR = 3566836U, kG = 11999065U, kB = 1211315U, kOffset = 8389408U;
+  return (kR * r + kG * g + kB * b + (kOffset - (kR + kG + kB) * bias)) >> 24;
+}
+
 // Stores four pixels of one row, x .. x + 3 (isp_math.hpp:250-276), from
 // their toned values t, their rounded integer codes c (2^23 + code as float
 // bits: 8-bit codes for RGB8/RGBA8, 16-bit values for RGB16) and counts their
@@ -352,14 +418,11 @@ template <int kOut>
 __device__ __forceinline__ void store_seg4(const FrameDesc& p, int x, int y, const float (&t)[4][3],
                                            const unsigned int (&c)[4][3], int n, bool want_hist, Span<unsigned int> hist) {
   Span<uint8_t> row = p.out + static_cast<int64_t>(y) * p.out_pitch;
-  const bool vec = n == 4 && p.out_vector;
-  unsigned int q[4][3];  // histogram codes
+  // Whole words where this row allows them: x is a multiple of four pixels, so
+  // the row's own alignment decides.
+  constexpr unsigned int kAlign = kOut == kOutRgb8 ? 4U : kOut == kOutRgb16 ? 8U : 16U;
+  const bool vec = n == 4 && (static_cast<unsigned int>(reinterpret_cast<uintptr_t>(span_ptr(row))) & (kAlign - 1U)) == 0U;
   if constexpr (kOut == kOutRgb8 || kOut == kOutRgba8) {
-#pragma unroll
-    for (int d = 0; d < 4; ++d) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) q[d][k] = c[d][k] & 0xFFU;  // 2^23 + code, code < 256
-    }
     if constexpr (kOut == kOutRgb8) {
       if (vec) {
         Span<unsigned int> o = span_cast<unsigned int>(row + 3 * x);
@@ -371,7 +434,7 @@ __device__ __forceinline__ void store_seg4(const FrameDesc& p, int x, int y, con
         for (int d = 0; d < 4; ++d) {
           if (d >= n) break;
 #pragma unroll
-          for (int k = 0; k < 3; ++k) row[3 * (x + d) + k] = static_cast<uint8_t>(q[d][k]);
+          for (int k = 0; k < 3; ++k) row[3 * (x + d) + k] = static_cast<uint8_t>(c[d][k]);
         }
       }
     } else {
@@ -392,16 +455,6 @@ __device__ __forceinline__ void store_seg4(const FrameDesc& p, int x, int y, con
       }
     }
   } else if constexpr (kOut == kOutRgb16) {
-#pragma unroll
-    for (int d = 0; d < 4; ++d) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        // (v * 255 + 32767) / 65535 == ((v + 128) * 0xFF01) >> 24 for v < 2^16
-        // (checked for every v); c = 2^23 bits + v, and the product of
-        // (c + 128 - 2^23 bits) stays below 2^32.
-        q[d][k] = ((c[d][k] + (128U - kTwo23Bits)) * 0xFF01U) >> 24;
-      }
-    }
     if (vec) {
       Span<uint2> o = span_cast<uint2>(row + 6 * x);
       o[0] = make_uint2(__byte_perm(c[0][0], c[0][1], 0x5410), __byte_perm(c[0][2], c[1][0], 0x5410));
@@ -417,11 +470,6 @@ __device__ __forceinline__ void store_seg4(const FrameDesc& p, int x, int y, con
       }
     }
   } else {
-#pragma unroll
-    for (int d = 0; d < 4; ++d) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) q[d][k] = c[d][k] & 0xFFU;
-    }
     if (vec) {
       Span<float4> o = span_cast<float4>(row + 12 * x);
       o[0] = make_float4(t[0][0], t[0][1], t[0][2], t[1][0]);
@@ -441,11 +489,20 @@ __device__ __forceinline__ void store_seg4(const FrameDesc& p, int x, int y, con
 #pragma unroll
     for (int d = 0; d < 4; ++d) {
       if (d >= n) break;
-      const unsigned int luma = (2126U * q[d][0] + 7152U * q[d][1] + 722U * q[d][2] + 5000U) / 10000U;
-      atomicAdd(&hist[luma], 1U);
-      atomicAdd(&hist[kHistBins + q[d][0]], 1U);
-      atomicAdd(&hist[2 * kHistBins + q[d][1]], 1U);
-      atomicAdd(&hist[3 * kHistBins + q[d][2]], 1U);
+      // The 8-bit codes, with the 2^23 bits still on them where they are the
+      // stored codes themselves.
+      constexpr unsigned int kBias = kOut == kOutRgb16 ? 0U : kTwo23Bits;
+      unsigned int q[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        // 16-bit values: (v * 255 + 32767) / 65535 == ((v + 128) * 0xFF01) >> 24
+        // for v < 2^16 (checked for every v); c = 2^23 bits + v, and the
+        // product of (c + 128 - 2^23 bits) stays below 2^32.
+        q[k] = kOut == kOutRgb16 ? ((c[d][k] + (128U - kTwo23Bits)) * 0xFF01U) >> 24 : c[d][k];
+      }
+      count_code(hist, 0, luma_of(q[0], q[1], q[2], kBias), 0U);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) count_code(hist, 1 + k, q[k], kBias);
     }
   }
 }
@@ -453,13 +510,16 @@ __device__ __forceinline__ void store_seg4(const FrameDesc& p, int x, int y, con
 // The per-pixel tail of four pairs of one row (pixels x .. x + 3 and
 // x + 32 .. x + 35 of image row y): colour matrix, statistics sums, tone,
 // codes, stores. nl, nr: pixels of the left and right groups inside the
-// image (0..4); kFull: both are 4 and the rows may be stored 16 bytes at a
-// time (the interior units, compiled without the per-pixel guards). sums:
+// image (0..4); kFull: both are 4 (the interior units, compiled without the
+// per-pixel guards). sums:
 // 2^23 bits + to_fixed summed mod 2^32, npix the number of terms, so that the
-// caller subtracts npix x 2^23 bits.
+// caller subtracts npix x 2^23 bits. The sums are formed whether the frame
+// wants them or not: a test per value cut the twelve values of a unit into as
+// many blocks of code, and two versions of the function overran the
+// instruction cache of the batch kernel.
 template <int kOut, bool kLutSmem, bool kFull>
 __device__ __forceinline__ void finish_pairs(const FrameDesc& p, const float2 (&rgb)[4][3], int x, int y, int nl_,
-                                             int nr_, Span<const float2> lut, float lut_scale, bool want_stats,
+                                             int nr_, Span<const float2> lut, float lut_scale,
                                              bool want_hist, Span<unsigned int> hist, unsigned int (&sums)[3],
                                              unsigned int& npix) {
   const int nl = kFull ? 4 : nl_;
@@ -471,60 +531,57 @@ __device__ __forceinline__ void finish_pairs(const FrameDesc& p, const float2 (&
     const float2* c = rgb[i];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      // clamp01((m0 r + m1 g) + m2 b), isp_math.hpp:229-233: rounded
-      // products, so the sums run per lane (isp_ops.cuh).
-      const float2 lin = add_sat2(add_lanes(mul2(bc2(p.ccm[3 * k]), c[0]), mul2(bc2(p.ccm[3 * k + 1]), c[1])),
+      // clamp01((m0 r + m1 g) + m2 b), isp_math.hpp:229-233.
+      const float2 lin = add_sat2(psum2(mul2(bc2(p.ccm[3 * k]), c[0]), mul2(bc2(p.ccm[3 * k + 1]), c[1])),
                                   mul2(bc2(p.ccm[3 * k + 2]), c[2]));
-      if (want_stats) {
-        // to_fixed (isp_math.hpp:245-247): trunc(lin 2^20 + 0.5). lin 2^20 is
-        // exact and so is the sum below 2^20 + 1; above it both roundings
-        // truncate to 2^20.
-        const float2 m = magic_trunc2(exact_scale_add2(lin, bc2(kFixedOne), bc2(0.5F)));
-        sums[k] += (i < nl ? __float_as_uint(m.x) : 0U) + (i < nr ? __float_as_uint(m.y) : 0U);
-      }
-      // f = lin (N - 1) is a rounded product: its truncation and f - i per lane.
+      // to_fixed (isp_math.hpp:245-247): trunc(lin 2^20 + 0.5). lin 2^20 is
+      // exact and so is the sum below 2^20 + 1; above it both roundings
+      // truncate to 2^20.
+      const float2 fixed = magic_trunc2(exact_scale_add2(lin, bc2(kFixedOne), bc2(0.5F)));
+      sums[k] += (i < nl ? __float_as_uint(fixed.x) : 0U) + (i < nr ? __float_as_uint(fixed.y) : 0U);
+      // f = lin (N - 1), a product; i = trunc(f); f - i.
       const float2 f = mul2(lin, bc2(lut_scale));
-      const float2 m = magic_trunc_lanes(f);
-      const float2 frac = sub_lanes(f, sub2(m, bc2(kTwo23)));
+      const float2 m = magic_trunc_product2(f);
+      const float2 frac = psum2(f, sub2(bc2(kTwo23), m));
       const float2 toned = make_float2(tone_lookup<kLutSmem>(lut, m.x, frac.x), tone_lookup<kLutSmem>(lut, m.y, frac.y));
       tl[i][k] = toned.x;
       tr[i][k] = toned.y;
       float2 code;
-      // trunc(t scale + 0.5): the product is rounded, so + 0.5 runs per lane.
+      // trunc(t scale + 0.5). RGB32F stores t itself; its code is of t clamped.
       if constexpr (kOut == kOutRgb16) {
-        code = magic_trunc2(add_lanes(mul2(toned, bc2(65535.0F)), bc2(0.5F)));
+        code = magic_trunc2(psum2(mul2(toned, bc2(65535.0F)), bc2(0.5F)));
       } else if constexpr (kOut == kOutRgb32f) {
-        const float2 clamped = make_float2(clamp01(toned.x), clamp01(toned.y));
-        code = magic_trunc2(add_lanes(mul2(clamped, bc2(255.0F)), bc2(0.5F)));
+        const float2 clamped = mul_sat2(toned, bc2(1.0F));
+        code = magic_trunc2(psum2(mul2(clamped, bc2(255.0F)), bc2(0.5F)));
       } else {
-        code = magic_trunc2(add_lanes(mul2(toned, bc2(255.0F)), bc2(0.5F)));
+        code = magic_trunc2(psum2(mul2(toned, bc2(255.0F)), bc2(0.5F)));
       }
       cl[i][k] = __float_as_uint(code.x);
       cr[i][k] = __float_as_uint(code.y);
     }
   }
-  if (want_stats) npix += static_cast<unsigned int>(nl + nr);
+  npix += static_cast<unsigned int>(nl + nr);
   if (kFull || nl > 0) store_seg4<kOut>(p, x, y, tl, cl, nl, want_hist, hist);
   if (kFull || nr > 0) store_seg4<kOut>(p, x + kHalf, y, tr, cr, nr, want_hist, hist);
 }
 
 template <bool kLutSmem, bool kFull>
 __device__ __forceinline__ void finish_pairs_any(const FrameDesc& p, const float2 (&rgb)[4][3], int x, int y, int nl,
-                                                 int nr, Span<const float2> lut, float lut_scale, bool want_stats,
-                                                 bool want_hist, Span<unsigned int> hist, unsigned int (&sums)[3],
+                                                 int nr, Span<const float2> lut, float lut_scale, bool want_hist,
+                                                 Span<unsigned int> hist, unsigned int (&sums)[3],
                                                  unsigned int& npix) {
   switch (p.out_format) {
     case kOutRgb8:
-      finish_pairs<kOutRgb8, kLutSmem, kFull>(p, rgb, x, y, nl, nr, lut, lut_scale, want_stats, want_hist, hist, sums, npix);
+      finish_pairs<kOutRgb8, kLutSmem, kFull>(p, rgb, x, y, nl, nr, lut, lut_scale, want_hist, hist, sums, npix);
       break;
     case kOutRgba8:
-      finish_pairs<kOutRgba8, kLutSmem, kFull>(p, rgb, x, y, nl, nr, lut, lut_scale, want_stats, want_hist, hist, sums, npix);
+      finish_pairs<kOutRgba8, kLutSmem, kFull>(p, rgb, x, y, nl, nr, lut, lut_scale, want_hist, hist, sums, npix);
       break;
     case kOutRgb16:
-      finish_pairs<kOutRgb16, kLutSmem, kFull>(p, rgb, x, y, nl, nr, lut, lut_scale, want_stats, want_hist, hist, sums, npix);
+      finish_pairs<kOutRgb16, kLutSmem, kFull>(p, rgb, x, y, nl, nr, lut, lut_scale, want_hist, hist, sums, npix);
       break;
     default:
-      finish_pairs<kOutRgb32f, kLutSmem, kFull>(p, rgb, x, y, nl, nr, lut, lut_scale, want_stats, want_hist, hist, sums, npix);
+      finish_pairs<kOutRgb32f, kLutSmem, kFull>(p, rgb, x, y, nl, nr, lut, lut_scale, want_hist, hist, sums, npix);
       break;
   }
 }

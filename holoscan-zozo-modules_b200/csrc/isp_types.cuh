@@ -87,7 +87,6 @@ struct FrameDesc {
   Span<uint8_t> out;
   int64_t out_pitch;
   int out_format;
-  int out_vector;  // out and out_pitch allow the kernels' vector stores
   Span<uint32_t> hist_out;  // user histogram [4][256], or null
   Span<float> stats_out;    // user statistics [12], or null
   Span<Scratch> scratch;
