@@ -40,6 +40,50 @@ constexpr int kCfa[4][4] = {
     {kChGb, kChB, kChR, kChGr},
 };
 
+// The pipeline whose frame was queued last on each stream (by stream id): at
+// most one entry per live pipeline, removed when the pipeline moves to
+// another stream or is destroyed. A frame that follows on its stream waits
+// for that frame's event instead of its own pipeline's last one. Both come
+// earlier in the stream, so either order is right; but when nothing was queued
+// since, the wait is for the stream's last operation, which costs nothing and
+// leaves the frame's kernels free to start under that frame's end
+// (frame_overlap), whichever camera it belongs to. With the cameras of a rig
+// in turn on one stream, each waiting for its own last frame, no two frames
+// overlapped. If the caller queued other work since, the wait keeps the
+// frame behind all of it.
+std::mutex g_tails_mutex;
+std::map<unsigned long long, isp_b200_pipeline*> g_tails;
+
+void drop_stream_tail(isp_b200_pipeline& pl) {
+  std::lock_guard<std::mutex> lock(g_tails_mutex);
+  const auto it = g_tails.find(pl.tail_stream_id);
+  if (it != g_tails.end() && it->second == &pl) g_tails.erase(it);
+}
+
+void set_stream_tail(isp_b200_pipeline& pl) {
+  if (!pl.last_stream_known) return drop_stream_tail(pl);
+  std::lock_guard<std::mutex> lock(g_tails_mutex);
+  if (pl.tail_stream_id != pl.last_stream_id) {
+    const auto it = g_tails.find(pl.tail_stream_id);
+    if (it != g_tails.end() && it->second == &pl) g_tails.erase(it);
+    pl.tail_stream_id = pl.last_stream_id;
+  }
+  g_tails[pl.tail_stream_id] = &pl;
+}
+
+cudaError_t wait_for_stream_tail(cudaStream_t stream, isp_b200_pipeline& pl) {
+  // A capturing stream waits for the pipeline's own event as it always did:
+  // that decides what the capture may depend on.
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+    static_cast<void>(cudaGetLastError());
+    return cudaStreamWaitEvent(stream, pl.done, 0);
+  }
+  std::lock_guard<std::mutex> lock(g_tails_mutex);  // keeps the event's pipeline alive
+  const auto it = g_tails.find(pl.last_stream_id);
+  return cudaStreamWaitEvent(stream, it != g_tails.end() ? it->second->done : pl.done, 0);
+}
+
 std::mutex g_shapes_mutex;
 std::deque<LaunchShapes> g_shapes;  // per device; growing keeps references valid
 
@@ -354,6 +398,9 @@ cudaError_t launch_frame(const FrameDesc& d, const isp_params_c& p, LaunchShapes
   // becomes resident on the SMs the statistics pass leaves and waits in the
   // kernel (griddepcontrol.wait) for its completion before anything else. An
   // event recorded in between (before_main) keeps the two kernels apart.
+  // With manual white balance there is no statistics pass, and the tile pass
+  // follows the previous frame's in the same way (after_previous): only its
+  // tables, none of the caller's buffers, are read before that wait.
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(threads);
@@ -363,7 +410,7 @@ cudaError_t launch_frame(const FrameDesc& d, const isp_params_c& p, LaunchShapes
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = d.auto_wb ? 1 : 0;
+  cfg.numAttrs = d.auto_wb || after_previous ? 1 : 0;
   const cudaError_t e = cudaLaunchKernelExC(&cfg, k, args);
   if (e != cudaSuccess || after_main == nullptr) return e;
   return cudaEventRecord(after_main, stream);
@@ -435,6 +482,7 @@ int isp_b200_create(const isp_params_c* params, isp_b200_pipeline** out) {
 
 void isp_b200_destroy(isp_b200_pipeline* pl) {
   if (pl == nullptr) return;
+  drop_stream_tail(*pl);
   if (pl->queued) cudaEventSynchronize(pl->done);
   if (pl->host_stream != nullptr) cudaStreamSynchronize(pl->host_stream);
   device_state_free(&pl->state);
@@ -498,9 +546,9 @@ int isp_b200_process(isp_b200_pipeline* pl, const isp_raw_view_c* raw, const isp
   // previous frame first (cuda_pipeline.cu:304-310). On the same stream the
   // next frame's statistics pass may still overlap this one's end
   // (frame_overlap): it follows the tile pass as its programmatic dependent.
-  const bool same_stream = pl->queued && stream == pl->last_stream;
+  const bool same_stream = pl->follows_on(stream);
   if (pl->queued) {
-    error = cudaStreamWaitEvent(stream, pl->done, 0);
+    error = same_stream ? wait_for_stream_tail(stream, *pl) : cudaStreamWaitEvent(stream, pl->done, 0);
     if (error != cudaSuccess) return fail_cuda(error, "cudaStreamWaitEvent");
   }
   const char* step = "launch";
@@ -511,7 +559,8 @@ int isp_b200_process(isp_b200_pipeline* pl, const isp_raw_view_c* raw, const isp
   error = cudaEventRecord(pl->done, stream);
   if (error != cudaSuccess) return fail_cuda(error, "cudaEventRecord");
   pl->queued = true;
-  pl->last_stream = stream;
+  pl->set_last_stream(stream);
+  set_stream_tail(*pl);
   clear_error();
   return ISP_OK;
 }
@@ -658,7 +707,7 @@ int isp_b200_check_bounded_wait(isp_b200_pipeline* pl, uint32_t polls, void* str
   if (error == cudaSuccess) error = cudaEventRecord(pl->done, stream);
   if (error != cudaSuccess) return fail_cuda(error, "isp_b200_check_bounded_wait");
   pl->queued = true;
-  pl->last_stream = stream;
+  pl->set_last_stream(stream);
   clear_error();
   return ISP_OK;
 }

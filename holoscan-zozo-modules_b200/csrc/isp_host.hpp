@@ -109,7 +109,20 @@ struct isp_b200_pipeline {
   int device = 0;
   cudaEvent_t done = nullptr;
   bool queued = false;
-  cudaStream_t last_stream = nullptr;  // the stream of the last queued frame
+  // The stream of the last queued frame: its id, which unlike a handle is
+  // never used again, when known.
+  unsigned long long last_stream_id = 0;
+  bool last_stream_known = false;
+  unsigned long long tail_stream_id = 0;  // the stream it may stand as the last frame of (isp_capi.cu)
+  void set_last_stream(cudaStream_t stream) {
+    last_stream_known = cudaStreamGetId(stream, &last_stream_id) == cudaSuccess;
+  }
+  // Whether `stream` is the one of the last queued frame, so that its order is
+  // the frames' order.
+  bool follows_on(cudaStream_t stream) const {
+    unsigned long long id = 0;
+    return queued && last_stream_known && cudaStreamGetId(stream, &id) == cudaSuccess && id == last_stream_id;
+  }
   bool frame_overlap = true;           // isp_b200_set_frame_overlap
   int tile_rows = 0;                   // isp_b200_set_tile_rows: 0 = per shape (isp_b200_autotune), else 64 / 32
   struct ShapePick {
