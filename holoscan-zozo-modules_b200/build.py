@@ -38,7 +38,8 @@ SOURCES = ["isp_batch.cu", "isp_batch_global_lut.cu", "isp_batch_short.cu", "isp
            "isp_main_malvar_sharpen_short.cu",
            "isp_awb.cu", "isp_kernels.cu", "isp_capi.cu", "isp_batch_host.cu", "isp_noalloc.cu", "isp_server.cu", "isp_synth.cu", "isp_view.cu", "isp_params.cpp",
            # the colour converter (the step after the ISP)
-           "cc/cc_direct_yuv.cu", "cc/cc_direct_rgb.cu", "cc/cc_direct_gray.cu", "cc/cc_resample.cu", "cc/cc_capi.cu",
+           "cc/cc_direct_yuv.cu", "cc/cc_direct_rgb.cu", "cc/cc_direct_gray.cu", "cc/cc_resample.cu",
+           "cc/cc_resample_planar.cu", "cc/cc_resample_packed.cu", "cc/cc_resample_rgb.cu", "cc/cc_resample_other.cu", "cc/cc_capi.cu",
            "cc/cc_plan.cpp"]
 
 

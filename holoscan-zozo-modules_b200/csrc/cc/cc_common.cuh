@@ -402,91 +402,6 @@ __device__ __forceinline__ void store_chroma(const Image& img, int cx, int cy, f
 
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
-// sum + s w per sample, product then sum, each rounded (:163-165).
-__device__ __forceinline__ Px accumulate(Px sum, const Px& s, float w) {
-  return {__fadd_rn(sum.c0, __fmul_rn(s.c0, w)), __fadd_rn(sum.c1, __fmul_rn(s.c1, w)),
-          __fadd_rn(sum.c2, __fmul_rn(s.c2, w)), __fadd_rn(sum.a, __fmul_rn(s.a, w))};
-}
-
-// Weight of source pixel [i, i + 1) in the footprint [lo, hi) (:168-172).
-__device__ __forceinline__ float covered(int i, float lo, float hi) {
-  const float fi = static_cast<float>(i);
-  const float fj = static_cast<float>(i + 1);
-  const float a = fi > lo ? fi : lo;
-  const float b = fj < hi ? fj : hi;
-  return b > a ? __fsub_rn(b, a) : 0.0F;
-}
-
-// The source sampled for content pixel (dx, dy) (:175-233), resize mode kMode.
-template <int kSrc, int kMode>
-__device__ __forceinline__ Px sample_px(const Plan& p, int dx, int dy) {
-  const float rx = static_cast<float>(dx - p.cx0);
-  const float ry = static_cast<float>(dy - p.cy0);
-  const float x0 = static_cast<float>(p.sx0);
-  const float y0 = static_cast<float>(p.sy0);
-  if constexpr (kMode == CC_NEAREST) {
-    const int sx = clampi(static_cast<int>(floorf(__fadd_rn(x0, __fmul_rn(__fadd_rn(rx, 0.5F), p.scale_x)))), p.sx0, p.sx1);
-    const int sy = clampi(static_cast<int>(floorf(__fadd_rn(y0, __fmul_rn(__fadd_rn(ry, 0.5F), p.scale_y)))), p.sy0, p.sy1);
-    return load_px<kSrc>(p.src, sx, sy);
-  } else if constexpr (kMode == CC_BILINEAR) {
-    const float fx = __fsub_rn(__fadd_rn(x0, __fmul_rn(__fadd_rn(rx, 0.5F), p.scale_x)), 0.5F);
-    const float fy = __fsub_rn(__fadd_rn(y0, __fmul_rn(__fadd_rn(ry, 0.5F), p.scale_y)), 0.5F);
-    const float bx = floorf(fx);
-    const float by = floorf(fy);
-    const float ax = __fsub_rn(fx, bx);
-    const float ay = __fsub_rn(fy, by);
-    const int ix = static_cast<int>(bx);
-    const int iy = static_cast<int>(by);
-    const int xa = clampi(ix, p.sx0, p.sx1);
-    const int xb = clampi(ix + 1, p.sx0, p.sx1);
-    const int ya = clampi(iy, p.sy0, p.sy1);
-    const int yb = clampi(iy + 1, p.sy0, p.sy1);
-    const float bx1 = __fsub_rn(1.0F, ax);
-    const float by1 = __fsub_rn(1.0F, ay);
-    const float w00 = __fmul_rn(bx1, by1);
-    const float w10 = __fmul_rn(ax, by1);
-    const float w01 = __fmul_rn(bx1, ay);
-    const float w11 = __fmul_rn(ax, ay);
-    // Taps of zero weight are skipped, as the definition does.
-    Px s{0.0F, 0.0F, 0.0F, 0.0F};
-    if (w00 != 0.0F) s = accumulate(s, load_px<kSrc>(p.src, xa, ya), w00);
-    if (w10 != 0.0F) s = accumulate(s, load_px<kSrc>(p.src, xb, ya), w10);
-    if (w01 != 0.0F) s = accumulate(s, load_px<kSrc>(p.src, xa, yb), w01);
-    if (w11 != 0.0F) s = accumulate(s, load_px<kSrc>(p.src, xb, yb), w11);
-    return s;
-  } else {
-    // Area: the footprint [lo, hi) on each axis, inside the source rectangle.
-    const float lx = __fadd_rn(x0, __fmul_rn(rx, p.scale_x));
-    const float ly = __fadd_rn(y0, __fmul_rn(ry, p.scale_y));
-    const float right = static_cast<float>(p.sx1 + 1);
-    const float bottom = static_cast<float>(p.sy1 + 1);
-    const float lxs = __fadd_rn(lx, p.scale_x);
-    const float lys = __fadd_rn(ly, p.scale_y);
-    const float hx = lxs < right ? lxs : right;
-    const float hy = lys < bottom ? lys : bottom;
-    const int ix0 = clampi(static_cast<int>(floorf(lx)), p.sx0, p.sx1);
-    const int iy0 = clampi(static_cast<int>(floorf(ly)), p.sy0, p.sy1);
-    Px s{0.0F, 0.0F, 0.0F, 0.0F};
-    float total = 0.0F;
-    for (int y = iy0; y <= p.sy1 && static_cast<float>(y) < hy; ++y) {
-      const float wy = covered(y, ly, hy);
-      for (int x = ix0; x <= p.sx1 && static_cast<float>(x) < hx; ++x) {
-        const float w = __fmul_rn(covered(x, lx, hx), wy);
-        if (w != 0.0F) {
-          s = accumulate(s, load_px<kSrc>(p.src, x, y), w);
-          total = __fadd_rn(total, w);
-        }
-      }
-    }
-    if (total <= 0.0F) return load_px<kSrc>(p.src, ix0, iy0);
-    return {__fdiv_rn(s.c0, total), __fdiv_rn(s.c1, total), __fdiv_rn(s.c2, total), __fdiv_rn(s.a, total)};
-  }
-}
-
-__device__ __forceinline__ bool in_content(const Plan& p, int x, int y) {
-  return x >= p.cx0 && x < p.cx1 && y >= p.cy0 && y < p.cy1;
-}
-
 #endif  // __CUDACC__
 
 // Host side (cc_plan.cpp): names, geometry, checks and the plan.

@@ -8,9 +8,10 @@
 // blocks) with both formats known at compile time, and writes each row's
 // segment with 32-bit stores where it is aligned.
 //
-// Resample path: one thread per destination block (a pixel, or the pixels
-// sharing a chroma sample), the source format and resize mode known at
-// compile time, the destination's stores chosen at run time.
+// Resample path: a thread samples four destination pixels of a row (of two rows
+// into 4:2:0 formats: two whole chroma blocks), two at a time in the lanes of
+// f32x2 instructions, the source format and resize mode known at compile time,
+// the destination's stores chosen at run time (cc_resample.cuh).
 #pragma once
 
 #include "../isp_ops.cuh"
@@ -401,77 +402,10 @@ __global__ void __launch_bounds__(kThreadsX* kThreadsY, kDirectBlocksPerSm) cc_d
   }
 }
 
-// Resample path helpers: the destination's stores chosen at run time.
-__device__ __forceinline__ void store_any(const Image& img, int x, int y, const Px& v) {
-  switch (img.format) {
-    case CC_NV12: store_px<CC_NV12>(img, x, y, v); break;
-    case CC_NV16: store_px<CC_NV16>(img, x, y, v); break;
-    case CC_I420: store_px<CC_I420>(img, x, y, v); break;
-    case CC_YUYV: store_px<CC_YUYV>(img, x, y, v); break;
-    case CC_UYVY: store_px<CC_UYVY>(img, x, y, v); break;
-    case CC_RGB8: store_px<CC_RGB8>(img, x, y, v); break;
-    case CC_BGR8: store_px<CC_BGR8>(img, x, y, v); break;
-    case CC_RGBA8: store_px<CC_RGBA8>(img, x, y, v); break;
-    case CC_BGRA8: store_px<CC_BGRA8>(img, x, y, v); break;
-    case CC_MONO8: store_px<CC_MONO8>(img, x, y, v); break;
-    case CC_MONO16: store_px<CC_MONO16>(img, x, y, v); break;
-    default: store_px<CC_RGB16>(img, x, y, v); break;
-  }
-}
-
-__device__ __forceinline__ void store_chroma_any(const Image& img, int cx, int cy, float cb, float cr) {
-  switch (img.format) {
-    case CC_NV12: store_chroma<CC_NV12>(img, cx, cy, cb, cr); break;
-    case CC_NV16: store_chroma<CC_NV16>(img, cx, cy, cb, cr); break;
-    case CC_I420: store_chroma<CC_I420>(img, cx, cy, cb, cr); break;
-    case CC_YUYV: store_chroma<CC_YUYV>(img, cx, cy, cb, cr); break;
-    default: store_chroma<CC_UYVY>(img, cx, cy, cb, cr); break;
-  }
-}
-
-template <int kSrc, int kMode>
-__device__ __forceinline__ Px pixel_at(const Plan& p, int x, int y) {
-  if (!in_content(p, x, y)) return Px{p.fill[0], p.fill[1], p.fill[2], p.fill[3]};
-  return apply_affine(p, sample_px<kSrc, kMode>(p, x, y));
-}
-
-// Resample path: thread (bx, by) converts destination block (bx, by)
-// (kernel_math.hpp:345-370).
-template <int kSrc, int kMode>
-__global__ void __launch_bounds__(kThreadsX* kThreadsY) cc_resample_kernel(const __grid_constant__ Plan p, int across,
-                                                                           int down) {
-  const int bx = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
-  const int by = static_cast<int>(blockIdx.y * blockDim.y + threadIdx.y);
-  if (bx >= across || by >= down) return;
-  if (!yuv_dst(p.dst.format)) {
-    store_any(p.dst, bx, by, pixel_at<kSrc, kMode>(p, bx, by));
-    return;
-  }
-  const int x0 = bx << p.bsx;
-  const int y0 = by << p.bsy;
-  const int x1 = min(x0 + (1 << p.bsx), p.dst.width);
-  const int y1 = min(y0 + (1 << p.bsy), p.dst.height);
-  float cb = 0.0F, cr = 0.0F;
-  int n = 0;
-  for (int y = y0; y < y1; ++y) {
-    for (int x = x0; x < x1; ++x) {
-      const Px v = pixel_at<kSrc, kMode>(p, x, y);
-      store_any(p.dst, x, y, v);
-      cb = __fadd_rn(cb, v.c1);
-      cr = __fadd_rn(cr, v.c2);
-      ++n;
-    }
-  }
-  const float cnt = static_cast<float>(n);
-  store_chroma_any(p.dst, bx, by, __fdiv_rn(cb, cnt), __fdiv_rn(cr, cnt));
-}
-
-// Launchers of each source format's direct kernels (cc_direct_*.cu) and of
-// the resample kernels (cc_resample.cu): a kernel pointer or null.
+// Each source format's direct kernels (cc_direct_*.cu): a kernel pointer or null.
 const void* direct_kernel(int src, int dst);
 const void* direct_kernel_yuv(int src, int dst);
 const void* direct_kernel_rgb(int src, int dst);
 const void* direct_kernel_gray(int src, int dst);
-const void* resample_kernel(int src, int mode);
 
 }  // namespace cc_b200

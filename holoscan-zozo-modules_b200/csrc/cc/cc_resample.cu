@@ -1,22 +1,13 @@
-// cc_resample.cu - the colour converter's resample kernels (one per source
-// format and resize mode), the synthetic camera pattern kernel, and the
-// launcher that picks the direct or the resample path for a plan.
+// cc_resample.cu - the synthetic camera pattern kernel, and the launcher that
+// picks the direct or the resample path for a plan.
 #include <cuda_runtime.h>
 
-#include "cc_kernels.cuh"
+#include <algorithm>
+
+#include "cc_resample.cuh"
 
 namespace cc_b200 {
 namespace {
-
-template <int kSrc>
-const void* for_mode(int mode) {
-  switch (mode) {
-    case CC_NEAREST: return reinterpret_cast<const void*>(&cc_resample_kernel<kSrc, CC_NEAREST>);
-    case CC_BILINEAR: return reinterpret_cast<const void*>(&cc_resample_kernel<kSrc, CC_BILINEAR>);
-    case CC_AREA: return reinterpret_cast<const void*>(&cc_resample_kernel<kSrc, CC_AREA>);
-    default: return nullptr;
-  }
-}
 
 // The synthetic camera's picture (modules/color-convert/include/holoscan/
 // color_convert/reference.hpp:34-55): eight full-intensity bars, white,
@@ -51,22 +42,13 @@ __global__ void cc_pattern_kernel(uint8_t* data, size_t pitch, int width, int he
 
 }  // namespace
 
-const void* resample_kernel(int src, int mode) {
-  switch (src) {
-    case CC_NV12: return for_mode<CC_NV12>(mode);
-    case CC_NV16: return for_mode<CC_NV16>(mode);
-    case CC_I420: return for_mode<CC_I420>(mode);
-    case CC_YUYV: return for_mode<CC_YUYV>(mode);
-    case CC_UYVY: return for_mode<CC_UYVY>(mode);
-    case CC_RGB8: return for_mode<CC_RGB8>(mode);
-    case CC_BGR8: return for_mode<CC_BGR8>(mode);
-    case CC_RGBA8: return for_mode<CC_RGBA8>(mode);
-    case CC_BGRA8: return for_mode<CC_BGRA8>(mode);
-    case CC_MONO8: return for_mode<CC_MONO8>(mode);
-    case CC_MONO16: return for_mode<CC_MONO16>(mode);
-    case CC_RGB16: return for_mode<CC_RGB16>(mode);
-    default: return nullptr;
-  }
+static const void* resample_kernel(const Plan& p) {
+  const int src = p.src.format;
+  const ResampleKey key{p.dst.format, resample_alpha(p), whole_scale(p), fast_source(p)};
+  if (src <= CC_I420) return resample_kernel_planar(src, p.mode, key);
+  if (src <= CC_UYVY) return resample_kernel_packed(src, p.mode, key);
+  if (src <= CC_BGRA8) return resample_kernel_rgb(src, p.mode, key);
+  return resample_kernel_other(src, p.mode, key);
 }
 
 const void* direct_kernel(int src, int dst) {
@@ -87,28 +69,30 @@ static bool direct_path(const Plan& p) {
 }
 
 int launch_convert(const Plan& plan, void* stream) {
-  const dim3 block(kThreadsX, kThreadsY);
   Plan p = plan;
   const bool direct = direct_path(p);
-  int across, down, per_block_x;
+  const dim3 block(kThreadsX, direct ? kThreadsY : kResampleThreadsY);
+  int across = (p.dst.width + kGroupX - 1) / kGroupX;  // four-pixel groups
+  int down, per_block_x;
   const void* fn;
   if (direct) {
-    // Four-pixel groups across; a block's warp covers kSub x 32 of them.
+    // A block's warp covers kSub x 32 groups.
     const FormatInfo fi = info_of(p.dst.format);
     const int rows = fi.model == kYuv ? (1 << fi.shift_y) : 1;
-    across = (p.dst.width + kGroupX - 1) / kGroupX;
     down = (p.dst.height + rows - 1) / rows;
     per_block_x = kThreadsX * direct_subgroups(p.dst.format);
     fn = direct_kernel(p.src.format, p.dst.format);
   } else {
-    across = (p.dst.width + (1 << p.bsx) - 1) >> p.bsx;
-    down = (p.dst.height + (1 << p.bsy) - 1) >> p.bsy;
+    const int rows = resample_rows(p.dst.format);
+    down = (p.dst.height + rows - 1) / rows;
     per_block_x = kThreadsX;
-    fn = resample_kernel(p.src.format, p.mode);
+    fn = resample_kernel(p);
   }
-  if (fn == nullptr || (down + kThreadsY - 1) / kThreadsY > 65535) return static_cast<int>(cudaErrorInvalidValue);
-  const dim3 grid(static_cast<unsigned>((across + per_block_x - 1) / per_block_x),
-                  static_cast<unsigned>((down + kThreadsY - 1) / kThreadsY));
+  // Refused: more than 65,535 x 8 rows of pixels (of chroma, where rows share it).
+  const int rows = direct ? down : (p.dst.height + (1 << p.bsy) - 1) >> p.bsy;
+  if (fn == nullptr || (rows + kThreadsY - 1) / kThreadsY > 65535) return static_cast<int>(cudaErrorInvalidValue);
+  const int blocks_down = std::min((down + static_cast<int>(block.y) - 1) / static_cast<int>(block.y), 65535);
+  const dim3 grid(static_cast<unsigned>((across + per_block_x - 1) / per_block_x), static_cast<unsigned>(blocks_down));
   void* args[] = {&p, &across, &down};
   return static_cast<int>(cudaLaunchKernel(fn, grid, block, args, 0, static_cast<cudaStream_t>(stream)));
 }
