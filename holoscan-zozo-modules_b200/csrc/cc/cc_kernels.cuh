@@ -220,6 +220,9 @@ __host__ __device__ constexpr int direct_subgroups(int dst) {
 template <int kSrc, int kDst>
 __global__ void __launch_bounds__(kThreadsX* kThreadsY, kDirectBlocksPerSm) cc_direct_kernel(const __grid_constant__ Plan p, int groups_x,
                                                                          int groups_y) {
+  // A programmatic dependent (launch_dependent): no memory before the wait.
+  isp_b200::griddep_launch_dependents();
+  isp_b200::griddep_wait();
   const int gy = static_cast<int>(blockIdx.y * blockDim.y + threadIdx.y);
   if (gy >= groups_y) return;
   constexpr FormatInfo fi = info_of(kDst);

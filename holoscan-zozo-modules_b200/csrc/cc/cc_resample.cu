@@ -4,6 +4,7 @@
 
 #include <algorithm>
 
+#include "../isp_host.hpp"
 #include "cc_resample.cuh"
 
 namespace cc_b200 {
@@ -94,7 +95,7 @@ int launch_convert(const Plan& plan, void* stream) {
   const int blocks_down = std::min((down + static_cast<int>(block.y) - 1) / static_cast<int>(block.y), 65535);
   const dim3 grid(static_cast<unsigned>((across + per_block_x - 1) / per_block_x), static_cast<unsigned>(blocks_down));
   void* args[] = {&p, &across, &down};
-  return static_cast<int>(cudaLaunchKernel(fn, grid, block, args, 0, static_cast<cudaStream_t>(stream)));
+  return static_cast<int>(isp_b200::launch_dependent(fn, grid, block, args, static_cast<cudaStream_t>(stream)));
 }
 
 int launch_pattern(uint8_t* data, size_t pitch, int width, int height, uint32_t frame, void* stream) {

@@ -543,6 +543,9 @@ __host__ __device__ constexpr int resample_blocks(int mode, int rows, int scale)
 template <int kF, int kMode, bool kAlpha, int kRows, int kScale, bool kFast>
 __global__ void __launch_bounds__(kThreadsX* kResampleThreadsY, resample_blocks(kMode, kRows, kScale)) cc_resample_kernel(const __grid_constant__ Plan p, int across,
                                                                                    int down) {
+  // A programmatic dependent (launch_dependent): no memory before the wait.
+  isp_b200::griddep_launch_dependents();
+  isp_b200::griddep_wait();
   const int gx = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
   if (gx >= across) return;
   const int x = gx * kGroupX;

@@ -71,7 +71,10 @@ void set_stream_tail(isp_b200_pipeline& pl) {
   g_tails[pl.tail_stream_id] = &pl;
 }
 
-cudaError_t wait_for_stream_tail(cudaStream_t stream, isp_b200_pipeline& pl) {
+// Waits as described above. `overlap` is cleared when the raw frame lies in
+// the image that the stream's last frame writes: its statistics pass must then
+// not start under that frame's end.
+cudaError_t wait_for_stream_tail(cudaStream_t stream, isp_b200_pipeline& pl, const isp_raw_view_c& raw, bool* overlap) {
   // A capturing stream waits for the pipeline's own event as it always did:
   // that decides what the capture may depend on.
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
@@ -81,7 +84,11 @@ cudaError_t wait_for_stream_tail(cudaStream_t stream, isp_b200_pipeline& pl) {
   }
   std::lock_guard<std::mutex> lock(g_tails_mutex);  // keeps the event's pipeline alive
   const auto it = g_tails.find(pl.last_stream_id);
-  return cudaStreamWaitEvent(stream, it != g_tails.end() ? it->second->done : pl.done, 0);
+  const isp_b200_pipeline& tail = it != g_tails.end() ? *it->second : pl;
+  const auto begin = reinterpret_cast<uintptr_t>(raw.data);
+  const uintptr_t end = begin + raw.pitch * static_cast<size_t>(raw.height);
+  if (begin < tail.last_out_end && tail.last_out_begin < end) *overlap = false;
+  return cudaStreamWaitEvent(stream, tail.done, 0);
 }
 
 std::mutex g_shapes_mutex;
@@ -324,6 +331,24 @@ cudaError_t blocks_per_sm(LaunchShapes& shapes, const void* kernel, size_t smem_
   return cudaSuccess;
 }
 
+cudaError_t launch_dependent(const void* kernel, dim3 grid, dim3 block, void** args, cudaStream_t stream) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {
+    static_cast<void>(cudaGetLastError());
+    capture = cudaStreamCaptureStatusActive;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = capture == cudaStreamCaptureStatusNone ? 1 : 0;
+  return cudaLaunchKernelExC(&cfg, kernel, args);
+}
+
 cudaError_t launch_frame(const FrameDesc& d, const isp_params_c& p, LaunchShapes& shapes, cudaStream_t stream,
                          cudaEvent_t before_main, cudaEvent_t after_main, const char** step, bool after_previous,
                          int tile_rows) {
@@ -547,18 +572,21 @@ int isp_b200_process(isp_b200_pipeline* pl, const isp_raw_view_c* raw, const isp
   // next frame's statistics pass may still overlap this one's end
   // (frame_overlap): it follows the tile pass as its programmatic dependent.
   const bool same_stream = pl->follows_on(stream);
+  bool overlap = same_stream && pl->frame_overlap;
   if (pl->queued) {
-    error = same_stream ? wait_for_stream_tail(stream, *pl) : cudaStreamWaitEvent(stream, pl->done, 0);
+    error = same_stream ? wait_for_stream_tail(stream, *pl, *raw, &overlap) : cudaStreamWaitEvent(stream, pl->done, 0);
     if (error != cudaSuccess) return fail_cuda(error, "cudaStreamWaitEvent");
   }
   const char* step = "launch";
   error = launch_frame(d, pl->params.c, shapes, stream, pl->before_main, pl->after_main, &step,
-                       same_stream && pl->frame_overlap, pl->rows_for(*raw));
+                       overlap, pl->rows_for(*raw));
   if (error == cudaSuccess) error = cudaGetLastError();
   if (error != cudaSuccess) return fail_cuda(error, (std::string("IspPipeline (cuda) ") + step).c_str());
   error = cudaEventRecord(pl->done, stream);
   if (error != cudaSuccess) return fail_cuda(error, "cudaEventRecord");
   pl->queued = true;
+  pl->last_out_begin = reinterpret_cast<uintptr_t>(out->data);
+  pl->last_out_end = pl->last_out_begin + out->pitch * static_cast<size_t>(raw->height);
   pl->set_last_stream(stream);
   set_stream_tail(*pl);
   clear_error();

@@ -124,4 +124,14 @@ __device__ __forceinline__ float2 magic_to_float2(unsigned int a_bits, unsigned 
 __device__ __forceinline__ float2 mul_sat2(float2 a, float2 b) { return make_float2(mul_sat(a.x, b.x), mul_sat(a.y, b.y)); }
 __device__ __forceinline__ float2 add_sat2(float2 a, float2 b) { return make_float2(add_sat(a.x, b.x), add_sat(a.y, b.y)); }
 
+// ---- Programmatic dependent launch ------------------------------------------
+
+// Lets the grid launched after this one (as a programmatic dependent) start
+// before this grid finishes.
+__device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Waits until the grid this one depends on has completed and its memory
+// writes are visible; returns at once when there is no such dependency.
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 }  // namespace isp_b200
