@@ -1,13 +1,25 @@
 // isp_view.cu - the demo's side-by-side view of raw and processed frames
 // (applications/isp/src/view_op.cu:35-75), as a headless device image: the
 // raw mosaic as square-rooted gray on the left, the ISP's RGB8 image on the
-// right. One thread converts a run of sixteen pixels of a row and copies
-// the sixteen RGB pixels beside them.
+// right. One thread converts a run of sixteen pixels of a row.
+//
+// The bytes that move (9 per pixel and the raw frame) take 13.2 us of a
+// 3840x2160 RAW10 frame at the measured copy bandwidth. What kept the kernel at
+// twice that was instruction issue (71 % of the slots, 62 instructions per
+// pixel: two byte loads and an exact square root for every sample), so that
+//   - a warp takes 32 runs of a row and moves their bytes in whole, contiguous
+//     words of the row: the RGB pixels straight across, the raw samples and the
+//     gray pixels by way of shared memory (three 16-byte accesses 48 bytes apart
+//     per thread left the load and store units the limit);
+//   - the gray codes of 8- to 12-bit samples, at most 4096 of them, are worked
+//     out once per block into shared memory, and blocks stay for several rows
+//     (kTableMax; deeper samples are computed one by one).
 #include <cuda_runtime.h>
 
 #include <string>
 
 #include "isp_host.hpp"
+#include "isp_ops.cuh"
 #include "isp_trace.hpp"
 
 namespace isp_b200 {
@@ -48,55 +60,153 @@ __device__ __forceinline__ uint32_t view_gray(int s, float black, float scale) {
   return __float2uint_rz(__fadd_rn(__fmul_rn(__fsqrt_rn(v), 255.0F), 0.5F));
 }
 
-// One thread per run of 16 pixels of a row (x0 = 16 g): their 16 gray codes
-// and the 16 RGB pixels beside them. Where the rows allow it (16-byte aligned
-// RGB and view rows, a whole run inside the frame) the 48-byte runs move as
-// three 16-byte words each and the raw samples come as 32-bit words; else
-// byte by byte.
-__global__ void __launch_bounds__(256) isp_view_kernel(const __grid_constant__ ViewArgs a) {
-  constexpr int kRun = 16;
-  const int x0 = kRun * static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
-  const int y = static_cast<int>(blockIdx.y * blockDim.y + threadIdx.y);
-  if (x0 >= a.width || y >= a.height) return;
-  const int n = a.width - x0 < kRun ? a.width - x0 : kRun;
-  const uint8_t* raw = a.raw + static_cast<size_t>(y) * a.raw_pitch;
-  const uint8_t* rgb = a.rgb + static_cast<size_t>(y) * a.rgb_pitch + 3 * static_cast<size_t>(x0);
-  uint8_t* left = a.out + static_cast<size_t>(y) * a.out_pitch + 3 * static_cast<size_t>(x0);
-  uint8_t* right = left + 3 * static_cast<size_t>(a.width);
-  const bool vec = n == kRun && ((reinterpret_cast<uintptr_t>(rgb) | reinterpret_cast<uintptr_t>(left) |
-                                  reinterpret_cast<uintptr_t>(right)) & 15U) == 0U;
-  if (vec) {
-    // The RGB run: three 16-byte words, loaded before the arithmetic.
-    const uint4 c0 = __ldg(reinterpret_cast<const uint4*>(rgb));
-    const uint4 c1 = __ldg(reinterpret_cast<const uint4*>(rgb) + 1);
-    const uint4 c2 = __ldg(reinterpret_cast<const uint4*>(rgb) + 2);
-    uint32_t g[kRun];
+constexpr int kRun = 16;             // pixels of a thread
+constexpr int kTableMax = 4096;      // gray codes kept per block
+constexpr int kViewThreads = 256;
+
+// 32-bit words of sixteen samples.
+__host__ __device__ constexpr int run_words(int format) {
+  return format == ISP_RAW_U8 ? 4 : format == ISP_RAW_U16 ? 8 : format == ISP_RAW_RAW10 ? 5 : 6;
+}
+
+// The sixteen samples of a run's words. Packed formats as in load_raw: RAW10
+// holds four pixels in five bytes, RAW12 two in three.
+template <int kFormat>
+__device__ __forceinline__ void view_samples(const uint32_t (&w)[run_words(kFormat)], uint32_t (&s)[kRun]) {
+  const auto byte_of = [&](int i) { return (w[i >> 2] >> (8 * (i & 3))) & 0xFFU; };
 #pragma unroll
-    for (int i = 0; i < kRun; ++i) g[i] = view_gray(view_sample(raw, a.format, x0 + i), a.black, a.scale);
-    // Gray pixels: bytes g, g, g per pixel, 48 bytes as 12 words.
-    uint32_t w[12];
-#pragma unroll
-    for (int k = 0; k < 12; ++k) {
-      uint32_t v = 0U;
-#pragma unroll
-      for (int b = 0; b < 4; ++b) v |= g[(4 * k + b) / 3] << (8 * b);
-      w[k] = v;
+  for (int i = 0; i < kRun; ++i) {
+    if constexpr (kFormat == ISP_RAW_U8) {
+      s[i] = byte_of(i);
+    } else if constexpr (kFormat == ISP_RAW_U16) {
+      s[i] = (w[i >> 1] >> (16 * (i & 1))) & 0xFFFFU;
+    } else if constexpr (kFormat == ISP_RAW_RAW10) {
+      const int g = 5 * (i >> 2);
+      s[i] = (byte_of(g + (i & 3)) << 2) | ((w[(g + 4) >> 2] >> (8 * ((g + 4) & 3) + 2 * (i & 3))) & 3U);
+    } else {
+      const int g = 3 * (i >> 1);
+      s[i] = (byte_of(g + (i & 1)) << 4) | ((w[(g + 2) >> 2] >> (8 * ((g + 2) & 3) + 4 * (i & 1))) & 15U);
     }
-    uint4* l = reinterpret_cast<uint4*>(left);
-    l[0] = make_uint4(w[0], w[1], w[2], w[3]);
-    l[1] = make_uint4(w[4], w[5], w[6], w[7]);
-    l[2] = make_uint4(w[8], w[9], w[10], w[11]);
-    uint4* r = reinterpret_cast<uint4*>(right);
-    r[0] = c0;
-    r[1] = c1;
-    r[2] = c2;
-    return;
   }
-  for (int i = 0; i < n; ++i) {
-    const uint8_t g = static_cast<uint8_t>(view_gray(view_sample(raw, a.format, x0 + i), a.black, a.scale));
-    left[3 * i] = left[3 * i + 1] = left[3 * i + 2] = g;
+}
+
+// A warp takes `tiles` of 32 runs of 16 pixels (tiles_x across the frame's
+// runs_x runs), striding over the frame with the grid's other warps. Where the
+// rows allow it (16-byte aligned RGB and view rows, 4-byte aligned raw rows)
+// whole runs move as described above; a row's last, shorter run and the runs of
+// other rows byte by byte.
+template <int kFormat, bool kTable>
+__global__ void __launch_bounds__(kViewThreads) isp_view_kernel(const __grid_constant__ ViewArgs a, int runs_x, int tiles_x,
+                                                                int tiles, int table_size) {
+  constexpr int kWords = run_words(kFormat);
+  __shared__ uint8_t table[kTable ? kTableMax : 4];
+  __shared__ uint4 staged[kViewThreads / 32][96];  // a tile's gray pixels; its raw words before them
+  // A programmatic dependent (launch_dependent): no global memory before the wait.
+  griddep_launch_dependents();
+  if constexpr (kTable) {
+    for (int i = threadIdx.x; i < table_size; i += kViewThreads) table[i] = static_cast<uint8_t>(view_gray(i, a.black, a.scale));
+    __syncthreads();
+  }
+  griddep_wait();
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  const int warp = static_cast<int>(threadIdx.x) >> 5;
+  uint4* const stage = staged[warp];
+  uint32_t* const words = reinterpret_cast<uint32_t*>(stage);
+  const auto gray = [&](uint32_t s) -> uint32_t {
+    if constexpr (kTable) {
+      // A 16-bit container may hold more than its bit depth says.
+      if (kFormat != ISP_RAW_U16 || s < static_cast<uint32_t>(table_size)) return table[s];
+    }
+    return view_gray(static_cast<int>(s), a.black, a.scale);
+  };
+  constexpr int kWarps = kViewThreads / 32;
+  for (int tile = static_cast<int>(blockIdx.x) * kWarps + warp; tile < tiles; tile += static_cast<int>(gridDim.x) * kWarps) {
+    const int y = tile / tiles_x;
+    const int run0 = 32 * (tile - y * tiles_x);
+    const uint8_t* raw = a.raw + static_cast<size_t>(y) * a.raw_pitch;
+    const uint8_t* rgb = a.rgb + static_cast<size_t>(y) * a.rgb_pitch;
+    uint8_t* left = a.out + static_cast<size_t>(y) * a.out_pitch;
+    uint8_t* right = left + 3 * static_cast<size_t>(a.width);
+    const bool vec = ((reinterpret_cast<uintptr_t>(rgb) | reinterpret_cast<uintptr_t>(left) |
+                       reinterpret_cast<uintptr_t>(right)) & 15U) == 0U && (reinterpret_cast<uintptr_t>(raw) & 3U) == 0U;
+    const int whole = vec ? min(a.width / kRun - run0, 32) : 0;  // the tile's runs moved as words
+    if (whole > 0) {
+      const uint32_t* from = reinterpret_cast<const uint32_t*>(raw) + static_cast<size_t>(run0) * kWords;
+      const uint4* pixels = reinterpret_cast<const uint4*>(rgb) + static_cast<size_t>(run0) * 3;
+      uint4* beside = reinterpret_cast<uint4*>(right) + static_cast<size_t>(run0) * 3;
+      uint4* below = reinterpret_cast<uint4*>(left) + static_cast<size_t>(run0) * 3;
+      uint32_t w[kWords];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) right[3 * i + k] = __ldg(rgb + 3 * i + k);
+      for (int k = 0; k < kWords; ++k) w[k] = lane + 32 * k < whole * kWords ? __ldg(from + lane + 32 * k) : 0U;
+      uint4 c[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) c[k] = lane + 32 * k < 3 * whole ? __ldg(pixels + lane + 32 * k) : make_uint4(0U, 0U, 0U, 0U);
+#pragma unroll
+      for (int k = 0; k < kWords; ++k) words[lane + 32 * k] = w[k];
+      __syncwarp();
+      if constexpr (kWords % 4 == 0) {
+#pragma unroll
+        for (int k = 0; k < kWords / 4; ++k) {
+          const uint4 v = stage[lane * (kWords / 4) + k];
+          w[4 * k] = v.x;
+          w[4 * k + 1] = v.y;
+          w[4 * k + 2] = v.z;
+          w[4 * k + 3] = v.w;
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < kWords; ++k) w[k] = words[lane * kWords + k];
+      }
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        if (lane + 32 * k < 3 * whole) beside[lane + 32 * k] = c[k];
+      }
+      uint32_t g[kRun];
+      view_samples<kFormat>(w, g);
+#pragma unroll
+      for (int i = 0; i < kRun; ++i) g[i] = gray(g[i]);
+      // Gray pixels: bytes g, g, g per pixel; four of them, a b c d, as the
+      // words aaab bbcc cddd.
+      uint32_t o[12];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        o[3 * k] = __byte_perm(g[4 * k], g[4 * k + 1], 0x4000U);
+        o[3 * k + 1] = __byte_perm(g[4 * k + 1], g[4 * k + 2], 0x4400U);
+        o[3 * k + 2] = __byte_perm(g[4 * k + 2], g[4 * k + 3], 0x4440U);
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k) stage[3 * lane + k] = make_uint4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        if (lane + 32 * k < 3 * whole) below[lane + 32 * k] = stage[lane + 32 * k];
+      }
+      __syncwarp();
+    }
+    if (lane >= whole && run0 + lane < runs_x) {
+      const int x0 = kRun * (run0 + lane);
+      const int x1 = min(x0 + kRun, a.width);
+      for (int x = x0; x < x1; ++x) {
+        const uint8_t g = static_cast<uint8_t>(gray(static_cast<uint32_t>(view_sample(raw, kFormat, x))));
+        left[3 * static_cast<size_t>(x)] = left[3 * static_cast<size_t>(x) + 1] = left[3 * static_cast<size_t>(x) + 2] = g;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) right[3 * static_cast<size_t>(x) + k] = __ldg(rgb + 3 * static_cast<size_t>(x) + k);
+      }
+    }
+  }
+}
+
+const void* view_kernel(int format, bool table) {
+  switch (format) {
+    case ISP_RAW_U8: return reinterpret_cast<const void*>(&isp_view_kernel<ISP_RAW_U8, true>);
+    case ISP_RAW_U16:
+      return table ? reinterpret_cast<const void*>(&isp_view_kernel<ISP_RAW_U16, true>)
+                   : reinterpret_cast<const void*>(&isp_view_kernel<ISP_RAW_U16, false>);
+    case ISP_RAW_RAW10: return reinterpret_cast<const void*>(&isp_view_kernel<ISP_RAW_RAW10, true>);
+    default:
+      return table ? reinterpret_cast<const void*>(&isp_view_kernel<ISP_RAW_RAW12, true>)
+                   : reinterpret_cast<const void*>(&isp_view_kernel<ISP_RAW_RAW12, false>);
   }
 }
 
@@ -126,10 +236,30 @@ extern "C" ISP_B200_API int isp_b200_view_compose(const isp_raw_view_c* raw, flo
   ViewArgs a{static_cast<const uint8_t*>(raw->data), raw->pitch, raw->width, raw->height, raw->format, black_level,
              1.0F / (white - black_level), static_cast<const uint8_t*>(rgb8), rgb8_pitch,
              static_cast<uint8_t*>(view), view_pitch};
-  const dim3 block(32, 8);
-  const dim3 grid(static_cast<unsigned>((raw->width + 511) / 512), static_cast<unsigned>((raw->height + 7) / 8));
-  isp_view_kernel<<<grid, block, 0, static_cast<cudaStream_t>(stream)>>>(a);
-  const cudaError_t e = cudaGetLastError();
+  // Rows beyond this were never taken (a grid of one block per eight rows).
+  if ((static_cast<int64_t>(raw->height) + 7) / 8 > 65535) return fail_cuda(cudaErrorInvalidConfiguration, "view kernel");
+  cudaError_t e = cudaSuccess;
+  const LaunchShapes& shapes = shapes_for_current_device(&e);
+  if (e != cudaSuccess) return fail_cuda(e, "view kernel");
+  // As many blocks as are resident at once, each with the same number of
+  // rounds over the frame's tiles.
+  constexpr int64_t kBlocksPerSm = 5;
+  constexpr int64_t kWarps = kViewThreads / 32;
+  int runs_x = (raw->width + kRun - 1) / kRun;
+  int tiles_x = (runs_x + 31) / 32;
+  const int64_t total = static_cast<int64_t>(tiles_x) * raw->height;
+  const int64_t needed = (total + kWarps - 1) / kWarps;
+  const int64_t rounds = (needed + shapes.sm_count * kBlocksPerSm - 1) / (shapes.sm_count * kBlocksPerSm);
+  const int64_t blocks = (needed + rounds - 1) / rounds;
+  // The table costs each thread table_size / 256 codes; a 12-bit one pays from
+  // the second round on (of two: 16 codes instead of 32). Every sample a packed
+  // format can hold has its entry, whatever the bit depth.
+  int table_size = 1 << (raw->format == ISP_RAW_U16 ? raw->bit_depth : max_bits);
+  const bool table = table_size <= kTableMax && (table_size <= 1024 || rounds >= 2);
+  int tiles = static_cast<int>(total);
+  void* args[] = {&a, &runs_x, &tiles_x, &tiles, &table_size};
+  e = launch_dependent(view_kernel(raw->format, table), dim3(static_cast<unsigned>(blocks)), dim3(kViewThreads), args,
+                       static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail_cuda(e, "view kernel");
   return ISP_OK;
 }
