@@ -10,79 +10,6 @@
 namespace isp_b200 {
 namespace {
 
-
-// ---- White balance statistics ----------------------------------------------
-
-// A band's lens shading maps and table: build_lsc's columns, rows, grid-row
-// range and table (the same arithmetic: top + (bottom - top) * ty from
-// T[k] = g + (g' - g) * tx, isp_math.hpp:121-140), for 64 columns and up to
-// kAwbBandRows rows, the rows looped over the block's threads.
-__device__ LscTile build_band_lsc(const FrameDesc& p, Span<const float> grid, int pattern, int x_first, int y_first,
-                                  int nrows, Span<int> col_mx, Span<int> col_ix, Span<float> col_tx, Span<int> row_my, Span<int> row_k,
-                                  Span<float> row_ty, Span<float> table, int* minmax) {
-  constexpr int kCols = 64;
-  const int t = threadIdx.x;
-  if (t == 0) {
-    minmax[0] = 0x7FFFFFFF;
-    minmax[1] = -1;
-  }
-  __syncthreads();
-  if (t < kCols) {
-    const int x = x_first + t;
-    col_mx[t] = x;
-    if (p.lsc != nullptr) {
-      const float fx = static_cast<float>(x) * p.lsc_sx;
-      int ix = static_cast<int>(fx);
-      ix = ix > p.lsc_width - 2 ? p.lsc_width - 2 : ix;
-      col_ix[t] = ix;
-      col_tx[t] = fx - static_cast<float>(ix);
-    }
-  }
-  int iy_lo = 0x7FFFFFFF;
-  int iy_hi = -1;
-  for (int j = t; j < nrows; j += kThreads) {
-    const int y = y_first + j;
-    row_my[j] = y;
-    if (p.lsc != nullptr) {
-      const float fy = static_cast<float>(y) * p.lsc_sy;
-      int iy = static_cast<int>(fy);
-      iy = iy > p.lsc_height - 2 ? p.lsc_height - 2 : iy;
-      row_k[j] = iy;
-      row_ty[j] = fy - static_cast<float>(iy);
-      iy_lo = iy < iy_lo ? iy : iy_lo;
-      iy_hi = iy > iy_hi ? iy : iy_hi;
-    }
-  }
-  if (p.lsc != nullptr) {
-    iy_lo = __reduce_min_sync(0xFFFFFFFFU, iy_lo);
-    iy_hi = __reduce_max_sync(0xFFFFFFFFU, iy_hi);
-    if ((t & 31) == 0 && iy_hi >= 0) {
-      atomicMin(&minmax[0], iy_lo);
-      atomicMax(&minmax[1], iy_hi);
-    }
-  }
-  __syncthreads();
-  LscTile lt{0, 0};
-  if (p.lsc == nullptr) return lt;
-  lt.iy0 = minmax[0];
-  lt.rows = minmax[1] - minmax[0] + 2;
-  if (lt.rows > kLscTableRows) return lt;
-  const int step = p.lsc_channels;
-  const int planes = step == 4 ? 2 : 1;
-  for (int e = t; e < lt.rows * planes * kCols; e += kThreads) {
-    const int i = e % kCols;
-    const int kp = e / kCols;
-    const int par = kp % planes;
-    const int k = kp / planes;
-    const int ch = step == 4 ? cfa_of(pattern, (par << 1) | (col_mx[i] & 1)) : 0;
-    Span<const float> g = grid + ((lt.iy0 + k) * p.lsc_width + col_ix[i]) * step + ch;
-    table[(k * 2 + par) * kSW + i] = g[0] + (g[step] - g[0]) * col_tx[i];
-  }
-  for (int j = t; j < nrows; j += kThreads) row_k[j] -= lt.iy0;
-  __syncthreads();
-  return lt;
-}
-
 // One CTA per band of a strip: columns [64 s, 64 s + 64) of the complete
 // quads, tiles [b band_tiles, (b + 1) band_tiles) of 64 rows. The band's lens
 // shading maps and table are built once; its tiles then stream through a
@@ -93,22 +20,9 @@ __global__ void __launch_bounds__(kThreads, 3) isp_awb_kernel(const __grid_const
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((128U - (smem_u32(smem_raw) & 127U)) & 127U);
   constexpr int kBoxRows = 64;
-  constexpr int kTableAt = 2 * 64 * 128;                          // boxes: [2][64][128], a double buffer
-  constexpr int kColsAt = kTableAt + kLscTableRows * 2 * kSW * 4;  // table: [kLscTableRows][2][kSW]
-  constexpr int kRowsAt = kColsAt + 3 * 64 * 4;                    // col_mx, col_ix, col_tx: [64] each
-  constexpr int kHistAt = kRowsAt + 3 * kAwbBandRows * 4;          // row_my, row_k, row_ty: [kAwbBandRows] each
-  constexpr int kGridAt = kHistAt + 3 * kAwbBins * 4;              // hist: [3][1024]; grid_s: [kGridSmemGains]
-  CheckRecord* rec = span_rec(p.scratch);
-  Span<uint8_t> boxes = carve_span<uint8_t>(smem, 0, kTableAt, rec);
-  Span<float> table = carve_span<float>(smem, kTableAt, kColsAt - kTableAt, rec);
-  Span<int> col_mx = carve_span<int>(smem, kColsAt, 64 * 4, rec);
-  Span<int> col_ix = carve_span<int>(smem, kColsAt + 64 * 4, 64 * 4, rec);
-  Span<float> col_tx = carve_span<float>(smem, kColsAt + 128 * 4, 64 * 4, rec);
-  Span<int> row_my = carve_span<int>(smem, kRowsAt, kAwbBandRows * 4, rec);
-  Span<int> row_k = carve_span<int>(smem, kRowsAt + kAwbBandRows * 4, kAwbBandRows * 4, rec);
-  Span<float> row_ty = carve_span<float>(smem, kRowsAt + 2 * kAwbBandRows * 4, kAwbBandRows * 4, rec);
-  Span<unsigned int> hist = carve_span<unsigned int>(smem, kHistAt, kGridAt - kHistAt, rec);
-  Span<float> grid_s = carve_span<float>(smem, kGridAt, kGridSmemGains * 4, rec);
+  const AwbSmem m = carve_awb(smem, span_rec(p.scratch));
+  const Span<uint8_t> boxes = m.boxes;
+  const Span<unsigned int> hist = m.hist;
   __shared__ uint64_t bars[2];
   __shared__ u64 red[4 * kWarps];
   __shared__ int minmax[2];
@@ -127,8 +41,8 @@ __global__ void __launch_bounds__(kThreads, 3) isp_awb_kernel(const __grid_const
   Span<const float> grid = p.lsc;
   const int gains = p.lsc_width * p.lsc_height * p.lsc_channels;
   if (p.lsc != nullptr && gains <= kGridSmemGains) {
-    for (int i = tid; i < gains; i += kThreads) cp_async4(&grid_s[i], &p.lsc[i]);
-    grid = grid_s;
+    for (int i = tid; i < gains; i += kThreads) cp_async4(&m.grid[i], &p.lsc[i]);
+    grid = m.grid;
   }
   if (tid == 0 && use_tma) {
     mbar_init(&bars[0]);
@@ -159,8 +73,7 @@ __global__ void __launch_bounds__(kThreads, 3) isp_awb_kernel(const __grid_const
   if (ty0 < ty1) issue(ty0, 0);
   // The band's maps and table (block-synchronised inside), while the first
   // box is in flight.
-  const LscTile lt = build_band_lsc(p, grid, kPat, x0, ty0 * 64, (ty1 - ty0) * 64, col_mx, col_ix, col_tx, row_my,
-                                    row_k, row_ty, table, minmax);
+  const LscTile lt = build_band_lsc(p, grid, kPat, x0, ty0 * 64, (ty1 - ty0) * 64, m, minmax);
   u64 acc[4] = {0, 0, 0, 0};
   uint32_t phases = 0;  // bit b: parity of buffer b's next completion
   AwbCell cell;
@@ -180,8 +93,8 @@ __global__ void __launch_bounds__(kThreads, 3) isp_awb_kernel(const __grid_const
     const int rows = (ty - ty0) * 64;  // the tile's first row within the band
     unsigned int sum[3] = {0U, 0U, 0U};
     unsigned int quads = 0;
-    awb_tile<kWhitePatch, kPat>(p, grid, boxes + buf * 64 * 128, box_bytes, x0, ty * 64, lt, row_k + rows, row_ty + rows,
-                                table, black, inv, hist, cell, sum, quads);
+    awb_tile<kWhitePatch, kPat>(p, grid, boxes + buf * 64 * 128, box_bytes, x0, ty * 64, lt, m.row_k + rows, m.row_ty + rows,
+                                m.table, black, inv, hist, cell, sum, quads);
 #pragma unroll
     for (int k = 0; k < 3; ++k) acc[k] += sum[k];
     acc[3] += quads;

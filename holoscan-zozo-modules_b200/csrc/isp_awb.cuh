@@ -19,6 +19,108 @@ __device__ __forceinline__ int awb_box_x(int fmt, int x0) {
   return fmt == kRawRaw10 ? 5 * (x0 >> 2) : fmt == kRawRaw12 ? 3 * (x0 >> 1) : x0;
 }
 
+// ---- Shared memory of a CTA of the statistics pass ---------------------------
+
+constexpr int kAwbTableAt = 2 * 64 * 128;                             // boxes: [2][64][128], a double buffer
+constexpr int kAwbColsAt = kAwbTableAt + kLscTableRows * 2 * kSW * 4;  // table: [kLscTableRows][2][kSW]
+constexpr int kAwbRowsAt = kAwbColsAt + 2 * 64 * 4;                    // col_ix, col_tx: [64] each
+constexpr int kAwbHistAt = kAwbRowsAt + 2 * kAwbBandRows * 4;          // row_k, row_ty: [kAwbBandRows] each
+constexpr int kAwbGridAt = kAwbHistAt + 3 * kAwbBins * 4;              // hist: [3][kAwbBins]
+constexpr int kAwbSmem = kAwbGridAt + kGridSmemGains * 4;              // grid: [kGridSmemGains]
+
+struct AwbSmem {
+  Span<uint8_t> boxes;
+  Span<float> table;
+  Span<int> col_ix;
+  Span<float> col_tx;
+  Span<int> row_k;
+  Span<float> row_ty;
+  Span<unsigned int> hist;
+  Span<float> grid;
+};
+
+__device__ __forceinline__ AwbSmem carve_awb(unsigned char* smem, CheckRecord* rec) {
+  AwbSmem m;
+  m.boxes = carve_span<uint8_t>(smem, 0, kAwbTableAt, rec);
+  m.table = carve_span<float>(smem, kAwbTableAt, kAwbColsAt - kAwbTableAt, rec);
+  m.col_ix = carve_span<int>(smem, kAwbColsAt, 64 * 4, rec);
+  m.col_tx = carve_span<float>(smem, kAwbColsAt + 64 * 4, 64 * 4, rec);
+  m.row_k = carve_span<int>(smem, kAwbRowsAt, kAwbBandRows * 4, rec);
+  m.row_ty = carve_span<float>(smem, kAwbRowsAt + kAwbBandRows * 4, kAwbBandRows * 4, rec);
+  m.hist = carve_span<unsigned int>(smem, kAwbHistAt, 3 * kAwbBins * 4, rec);
+  m.grid = carve_span<float>(smem, kAwbGridAt, kGridSmemGains * 4, rec);
+  return m;
+}
+
+// A band's lens shading maps and table: build_lsc's columns, rows, grid-row
+// range and table (the same arithmetic: top + (bottom - top) * ty from
+// T[k] = g + (g' - g) * tx, isp_math.hpp:121-140), for 64 columns and up to
+// kAwbBandRows rows, the rows looped over the block's threads.
+__device__ LscTile build_band_lsc(const FrameDesc& p, Span<const float> grid, int pattern, int x_first, int y_first,
+                                  int nrows, const AwbSmem& m, int* minmax) {
+  constexpr int kCols = 64;
+  const Span<int> col_ix = m.col_ix, row_k = m.row_k;
+  const Span<float> col_tx = m.col_tx, row_ty = m.row_ty, table = m.table;
+  const int t = threadIdx.x;
+  if (t == 0) {
+    minmax[0] = 0x7FFFFFFF;
+    minmax[1] = -1;
+  }
+  __syncthreads();
+  if (t < kCols) {
+    const int x = x_first + t;
+    if (p.lsc != nullptr) {
+      const float fx = static_cast<float>(x) * p.lsc_sx;
+      int ix = static_cast<int>(fx);
+      ix = ix > p.lsc_width - 2 ? p.lsc_width - 2 : ix;
+      col_ix[t] = ix;
+      col_tx[t] = fx - static_cast<float>(ix);
+    }
+  }
+  int iy_lo = 0x7FFFFFFF;
+  int iy_hi = -1;
+  for (int j = t; j < nrows; j += kThreads) {
+    const int y = y_first + j;
+    if (p.lsc != nullptr) {
+      const float fy = static_cast<float>(y) * p.lsc_sy;
+      int iy = static_cast<int>(fy);
+      iy = iy > p.lsc_height - 2 ? p.lsc_height - 2 : iy;
+      row_k[j] = iy;
+      row_ty[j] = fy - static_cast<float>(iy);
+      iy_lo = iy < iy_lo ? iy : iy_lo;
+      iy_hi = iy > iy_hi ? iy : iy_hi;
+    }
+  }
+  if (p.lsc != nullptr) {
+    iy_lo = __reduce_min_sync(0xFFFFFFFFU, iy_lo);
+    iy_hi = __reduce_max_sync(0xFFFFFFFFU, iy_hi);
+    if ((t & 31) == 0 && iy_hi >= 0) {
+      atomicMin(&minmax[0], iy_lo);
+      atomicMax(&minmax[1], iy_hi);
+    }
+  }
+  __syncthreads();
+  LscTile lt{0, 0};
+  if (p.lsc == nullptr) return lt;
+  lt.iy0 = minmax[0];
+  lt.rows = minmax[1] - minmax[0] + 2;
+  if (lt.rows > kLscTableRows) return lt;
+  const int step = p.lsc_channels;
+  const int odd = step == 4 ? 1 : 0;  // two rows of the table per grid row, or one
+  for (int e = t; e < (lt.rows << odd) * kCols; e += kThreads) {
+    const int i = e % kCols;
+    const int kp = e / kCols;
+    const int par = kp & odd;
+    const int k = kp >> odd;
+    const int ch = step == 4 ? cfa_of(pattern, (par << 1) | (i & 1)) : 0;
+    Span<const float> g = grid + ((lt.iy0 + k) * p.lsc_width + col_ix[i]) * step + ch;
+    table[(k * 2 + par) * kSW + i] = g[0] + (g[step] - g[0]) * col_tx[i];
+  }
+  for (int j = t; j < nrows; j += kThreads) row_k[j] -= lt.iy0;
+  __syncthreads();
+  return lt;
+}
+
 // The two rows of the lens shading table that a thread's current samples lie
 // between: T[k] and T[k + 1] - T[k] per row parity and column pair. A thread
 // keeps its four columns through a band, so they are read again only where

@@ -4,7 +4,10 @@
 
 namespace isp_b200 {
 
-const void* batch_kernel_shared_lut() { return reinterpret_cast<const void*>(&isp_batch_kernel<true, kTH>); }
+const void* batch_kernel_shared_lut(bool sharpen) {
+  return sharpen ? reinterpret_cast<const void*>(&isp_batch_kernel<true, kTH, true>)
+                 : reinterpret_cast<const void*>(&isp_batch_kernel<true, kTH, false>);
+}
 
 const void* awb_batch_kernel() { return reinterpret_cast<const void*>(&isp_awb_batch_kernel); }
 
@@ -24,10 +27,5 @@ __global__ void isp_batch_stage_kernel(const uint4* __restrict__ frames_src, uin
 }
 
 const void* batch_stage_kernel() { return reinterpret_cast<const void*>(&isp_batch_stage_kernel); }
-
-size_t batch_kernel_smem(bool lut_smem, int tile_rows) {
-  return static_cast<size_t>(layout_of(true, box_row_bytes(kRawU16), lut_smem ? kBatchLutEntries : 0, tile_rows).total) +
-         128U;
-}
 
 }  // namespace isp_b200

@@ -4,7 +4,8 @@
 //
 // Each pass is a persistent kernel over a work list: CTA i owns the
 // contiguous items ranges[i] (sized by the host so the estimated cost is
-// even), walks them frame by frame, keeps the frame's FrameDesc and tone
+// even; the last part of the work is claimed range by range from a queue
+// instead), walks them frame by frame, keeps the frame's FrameDesc and tone
 // table in shared memory, prefetches the next item's raw box by TMA
 // (whichever frame it belongs to), and flushes a frame's sums when it leaves
 // it; the CTA that completes a frame's count of tiles finishes that frame
@@ -40,23 +41,64 @@ __device__ __forceinline__ int frame_of_item(Span<const BatchFrame> frames, int 
   return f;
 }
 
+// The item after `item` for a CTA (one thread calls): the next of its range
+// r, or the first of a range claimed from the queue, which is left in `claim`
+// (empty when none is left). -1: none. Queued items come after every CTA's own,
+// and claims only move forward.
+__device__ __forceinline__ int next_item(BatchQueue* queue, int item, int2 r, int2& claim, CheckRecord* rec) {
+  if (item + 1 < r.y) return item + 1;
+  claim = make_int2(0, 0);
+  const int count = queue->count;
+  if (count > 0) {
+    const unsigned int c = atomicAdd(&queue->claimed, 1U);
+    if (c < static_cast<unsigned int>(count)) {
+      claim = make_span(reinterpret_cast<const int2*>(queue + 1), static_cast<size_t>(count), rec)[static_cast<int>(c)];
+    }
+  }
+  return claim.x < claim.y ? claim.x : -1;
+}
+
+// Adds a tile's four sums over the warp to the totals its lanes 0..3 keep: two
+// registers a thread across the tiles instead of eight. A tile has at most
+// 16 samples a thread of at most 2^22, so a warp's sum is below 2^32.
+__device__ __forceinline__ void add_tile_sums(u64& acc, unsigned int a, unsigned int b, unsigned int c, unsigned int d) {
+  a = __reduce_add_sync(0xffffffffU, a);
+  b = __reduce_add_sync(0xffffffffU, b);
+  c = __reduce_add_sync(0xffffffffU, c);
+  d = __reduce_add_sync(0xffffffffU, d);
+  const int lane = threadIdx.x & 31;
+  const unsigned int lo = (lane & 1) ? b : a, hi = (lane & 1) ? d : c;
+  acc += (lane & 2) ? hi : lo;
+}
+
+// The warp's totals as the flushes take them: per thread, summed over the block.
+__device__ __forceinline__ void totals_of(u64 acc, u64 (&total)[4]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) total[k] = lane == k ? acc : 0;
+}
+
 // One tile of a frame of any settings (BatchFrame::variant). Only what differs
 // between the variants is compiled per variant: the demosaics. With one copy
 // of the whole tile per variant (eight, each with the finish of four output
 // formats) the CTAs of an SM, at work on different variants, waited for
 // instructions more than for anything else (1.3 of 7.4 cycles per
-// instruction).
-template <bool kLutSmem, int kTileH, class AfterA>
+// instruction). kSharpen: whether any frame of the batch sharpens.
+template <bool kLutSmem, int kTileH, bool kSharpen, class AfterA>
 __device__ __forceinline__ void run_tile_any(const FrameDesc& p, const FrameSetup& f, const TileSmem& m, int* minmax,
                                              int variant, int x0, int y0, bool use_tma, uint64_t* bar, uint32_t& phase,
-                                             u64 (&acc)[4], AfterA after_a) {
-  const bool sharpen = (variant & 2) != 0;
+                                             u64& acc, AfterA after_a) {
+  const bool sharpen = kSharpen && (variant & 2) != 0;
+  unsigned int saturated = 0;
   const auto no_wait = [] {};
-  acc[3] += sharpen ? tile_samples<Geom<true, kTileH>::kHalo, kTileH>(p, f, m, minmax, x0, y0, use_tma, bar, phase, no_wait)
-                    : tile_samples<Geom<false, kTileH>::kHalo, kTileH>(p, f, m, minmax, x0, y0, use_tma, bar, phase, no_wait);
+  if (kSharpen && sharpen) {
+    saturated = tile_samples<Geom<true, kTileH>::kHalo, kTileH>(p, f, m, minmax, x0, y0, use_tma, bar, phase, no_wait);
+  } else {
+    saturated = tile_samples<Geom<false, kTileH>::kHalo, kTileH>(p, f, m, minmax, x0, y0, use_tma, bar, phase, no_wait);
+  }
   __syncthreads();
   after_a();
-  if (sharpen) {
+  if (kSharpen && sharpen) {
     const Span<float2> red = f.swap_rb ? m.B : m.R, blue = f.swap_rb ? m.R : m.B;
     switch (variant) {
       case 2: phase_b2<false, 0, kTileH>(m.P, red, m.G, blue); break;
@@ -73,7 +115,7 @@ __device__ __forceinline__ void run_tile_any(const FrameDesc& p, const FrameSetu
     int r, uc;
     unit_rc(threadIdx.x + k * kThreads, r, uc);
     float2 rgb[4][3];
-    if (sharpen) {
+    if (kSharpen && sharpen) {
       sharpened_row(m, r, uc, p.sharpen, rgb);
     } else {
       switch (variant) {
@@ -86,15 +128,18 @@ __device__ __forceinline__ void run_tile_any(const FrameDesc& p, const FrameSetu
     }
     finish_row<-1, kLutSmem>(p, f, m.hist, rgb, x0 + 4 * uc, y0 + r, sums, npix);
   }
-#pragma unroll
-  for (int k = 0; k < 3; ++k) acc[k] += sums[k] - npix * kTwo23Bits;  // mod 2^32: the true sum
+  add_tile_sums(acc, sums[0] - npix * kTwo23Bits, sums[1] - npix * kTwo23Bits, sums[2] - npix * kTwo23Bits,
+                saturated);  // mod 2^32: the true sums
   __syncthreads();  // the next tile overwrites the tables, P and the planes
 }
 
-template <bool kLutSmem, int kTileH>
-__global__ void __launch_bounds__(kThreads, kTileH == kTH ? 2 : 3)
-    isp_batch_kernel(const BatchFrame* frames_in, int nframes, const int2* ranges_in) {
-  using GS = Geom<true, kTileH>;  // the sharpening geometry holds every variant's
+// Without sharpening three CTAs share an SM (80 registers a thread, no RGB
+// planes), with it two. A 5472x3648 frame's tile pass takes 103 us at three and
+// 115 at two.
+template <bool kLutSmem, int kTileH, bool kSharpen>
+__global__ void __launch_bounds__(kThreads, kSharpen && kTileH == kTH ? 2 : 3)
+    isp_batch_kernel(const BatchFrame* frames_in, int nframes, const int2* ranges_in, BatchQueue* queue) {
+  using GS = Geom<kSharpen, kTileH>;  // the sharpening geometry holds every variant's
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((128U - (smem_u32(smem_raw) & 127U)) & 127U);
 #ifdef ISP_CHECKED
@@ -105,7 +150,8 @@ __global__ void __launch_bounds__(kThreads, kTileH == kTH ? 2 : 3)
   const Span<const BatchFrame> frames = make_span(frames_in, static_cast<size_t>(nframes), rec);
   const Span<const int2> ranges = make_span(ranges_in, static_cast<size_t>(gridDim.x), rec);
   const TileSmem m =
-      carve(smem, layout_of(true, box_row_bytes(kRawU16), kLutSmem ? kBatchLutEntries : 0, kTileH), GS::kSH, rec);
+      carve(smem, layout_of(kSharpen, box_row_bytes(kRawU16), kLutSmem ? kBatchLutEntries : 0, kTileH), GS::kSH, rec);
+  __shared__ int2 next_range;
   __shared__ uint64_t bar;
   __shared__ u64 red[4 * kWarps];
   __shared__ int minmax[2];
@@ -114,14 +160,14 @@ __global__ void __launch_bounds__(kThreads, kTileH == kTH ? 2 : 3)
   // A programmatic dependent of the statistics batch: resident early, it
   // waits here for that batch's completion (and the gains it wrote).
   griddep_wait();
-  const int2 r = ranges[blockIdx.x];
+  int2 r = ranges[blockIdx.x];
   if (r.x >= r.y) return;
   const int tid = threadIdx.x;
   if (tid == 0) mbar_init(&bar);
   int f = frame_of_item(frames, nframes, 0, r.x, false);
   load_desc(&fd, &frames[f].desc);
   __syncthreads();
-  FrameSetup fs = setup_frame<kLutSmem>(fd, m);
+  setup_frame<kLutSmem>(fd, m);
   __syncthreads();
 
   const auto issue = [&](int g, int item) {
@@ -137,19 +183,24 @@ __global__ void __launch_bounds__(kThreads, kTileH == kTH ? 2 : 3)
   };
   if (tid == 0 && frames[f].use_tma) issue(f, r.x);
   uint32_t phase = 0;
-  u64 acc[4] = {0, 0, 0, 0};
+  u64 acc = 0;
   unsigned int done = 0;
-  for (int item = r.x; item < r.y; ++item) {
+  const auto flush = [&] {
+    u64 total[4];
+    totals_of(acc, total);
+    flush_frame(fd, frame_setup<kLutSmem>(fd, m), total, m, red, &last, done, static_cast<unsigned int>(frames[f].tiles));
+  };
+  int item = r.x;
+  while (true) {
     if (item >= frames[f].tile_begin + frames[f].tiles) {
-      flush_frame(fd, fs, acc, m, red, &last, done, static_cast<unsigned int>(frames[f].tiles));
+      flush();
       __syncthreads();
       f = frame_of_item(frames, nframes, f, item, false);
       load_desc(&fd, &frames[f].desc);
       __syncthreads();
-      fs = setup_frame<kLutSmem>(fd, m);
+      setup_frame<kLutSmem>(fd, m);
       __syncthreads();
-#pragma unroll
-      for (int k = 0; k < 4; ++k) acc[k] = 0;
+      acc = 0;
       done = 0;
     }
     const BatchFrame& bf = frames[f];
@@ -158,27 +209,33 @@ __global__ void __launch_bounds__(kThreads, kTileH == kTH ? 2 : 3)
     const int x0 = (local - ty * bf.tiles_x) * kTW;
     const bool use_tma = bf.use_tma != 0;
     const auto prefetch = [&] {
-      if (tid == 0 && item + 1 < r.y) {
-        const int g = frame_of_item(frames, nframes, f, item + 1, false);
-        if (frames[g].use_tma) {
-          fence_async_shared();
-          issue(g, item + 1);
-        }
+      if (tid != 0) return;
+      const int next = next_item(queue, item, r, next_range, rec);
+      if (next < 0) return;
+      const int g = frame_of_item(frames, nframes, f, next, false);
+      if (frames[g].use_tma) {
+        fence_async_shared();
+        issue(g, next);
       }
     };
-    run_tile_any<kLutSmem, kTileH>(fd, fs, m, minmax, bf.variant, x0, ty * kTileH, use_tma, &bar, phase, acc, prefetch);
+    run_tile_any<kLutSmem, kTileH, kSharpen>(fd, frame_setup<kLutSmem>(fd, m), m, minmax, bf.variant, x0, ty * kTileH, use_tma, &bar, phase, acc,
+                                             prefetch);
     ++done;
+    if (++item == r.y) {
+      r = next_range;  // written before run_tile_any's closing barrier
+      if (r.x >= r.y) break;
+      item = r.x;
+    }
   }
-  flush_frame(fd, fs, acc, m, red, &last, done, static_cast<unsigned int>(frames[f].tiles));
+  flush();
 }
 
 // The statistics tile of a frame for its Bayer pattern and mode.
 __device__ __forceinline__ void awb_tile_any(const FrameDesc& p, int pattern, bool white_patch, Span<const uint8_t> box,
                                              int box_bytes, int x0, int y0, const LscTile& lt, Span<const int> row_k,
                                              Span<const float> row_ty, Span<const float> table, const float (&black)[4],
-                                             const float (&inv)[4], Span<unsigned int> hist, unsigned int (&sum)[3],
-                                             unsigned int& quads) {
-  AwbCell cell;  // the table is the tile's own
+                                             const float (&inv)[4], Span<unsigned int> hist, AwbCell& cell,
+                                             unsigned int (&sum)[3], unsigned int& quads) {
 #define ISP_AWB_CASE(P, W) \
   awb_tile<W, P>(p, p.lsc, box, box_bytes, x0, y0, lt, row_k, row_ty, table, black, inv, hist, cell, sum, quads)
   switch (pattern * 2 + (white_patch ? 1 : 0)) {
@@ -195,7 +252,7 @@ __device__ __forceinline__ void awb_tile_any(const FrameDesc& p, int pattern, bo
 }
 
 __global__ void __launch_bounds__(kThreads, 3) isp_awb_batch_kernel(const BatchFrame* frames_in, int nframes,
-                                                               const int2* ranges_in) {
+                                                               const int2* ranges_in, BatchQueue* queue) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((128U - (smem_u32(smem_raw) & 127U)) & 127U);
 #ifdef ISP_CHECKED
@@ -205,26 +262,17 @@ __global__ void __launch_bounds__(kThreads, 3) isp_awb_batch_kernel(const BatchF
 #endif
   const Span<const BatchFrame> frames = make_span(frames_in, static_cast<size_t>(nframes), rec);
   const Span<const int2> ranges = make_span(ranges_in, static_cast<size_t>(gridDim.x), rec);
-  constexpr int kTableAt = 2 * 64 * 128;                          // boxes: [2][64][128], a double buffer
-  constexpr int kColsAt = kTableAt + kLscTableRows * 2 * kSW * 4;  // table: [kLscTableRows][2][kSW]
-  constexpr int kRowsAt = kColsAt + 3 * 64 * 4;                    // col_mx, col_ix, col_tx: [64] each
-  constexpr int kHistAt = kRowsAt + 3 * 64 * 4;                    // row_my, row_k, row_ty: [64] each
-  Span<uint8_t> boxes = carve_span<uint8_t>(smem, 0, kTableAt, rec);
-  Span<float> table = carve_span<float>(smem, kTableAt, kColsAt - kTableAt, rec);
-  Span<int> col_mx = carve_span<int>(smem, kColsAt, 64 * 4, rec);
-  Span<int> col_ix = carve_span<int>(smem, kColsAt + 64 * 4, 64 * 4, rec);
-  Span<float> col_tx = carve_span<float>(smem, kColsAt + 128 * 4, 64 * 4, rec);
-  Span<int> row_my = carve_span<int>(smem, kRowsAt, 64 * 4, rec);
-  Span<int> row_k = carve_span<int>(smem, kRowsAt + 64 * 4, 64 * 4, rec);
-  Span<float> row_ty = carve_span<float>(smem, kRowsAt + 128 * 4, 64 * 4, rec);
-  Span<unsigned int> hist = carve_span<unsigned int>(smem, kHistAt, 3 * kAwbBins * 4, rec);  // [3][1024]
+  const AwbSmem m = carve_awb(smem, rec);
+  const Span<uint8_t> boxes = m.boxes;
+  const Span<unsigned int> hist = m.hist;
   __shared__ uint64_t bars[2];
   __shared__ u64 red[4 * kWarps];
   __shared__ int minmax[2];
   __shared__ bool last;
   __shared__ __align__(16) FrameDesc fd;
   griddep_launch_dependents();  // the tile batch may become resident as this one finishes
-  const int2 r = ranges[blockIdx.x];
+  __shared__ int2 next_range[2];
+  int2 r = ranges[blockIdx.x];
   if (r.x >= r.y) return;
   const int tid = threadIdx.x;
   if (tid == 0) {
@@ -237,54 +285,76 @@ __global__ void __launch_bounds__(kThreads, 3) isp_awb_batch_kernel(const BatchF
   __syncthreads();
   const auto issue = [&](int g, int item, int b) {
     const BatchFrame& bf = frames[g];
-    const int local = item - bf.awb_begin;
-    const int ty = local / bf.awb_tiles_x;
-    const int x0 = (local - ty * bf.awb_tiles_x) * 64;
+    const int tiles_y = bf.awb_tiles / bf.awb_tiles_x;
+    const int strip = (item - bf.awb_begin) / tiles_y;
+    const int ty = item - bf.awb_begin - strip * tiles_y;
+    const int x0 = strip * 64;
     const int fmt = bf.desc.raw_format;
     tensormap_acquire(&bf.awb_map);
     tma_load_2d(&bf.awb_map, boxes + b * 64 * 128, &bars[b], awb_box_x(fmt, x0), ty * 64,
                 static_cast<unsigned int>(64 * awb_box_bytes(fmt)));
   };
   if (tid == 0 && frames[f].use_tma) issue(f, r.x, 0);
-  // Item i of the range uses buffer (i - r.x) & 1, whether or not its frame
-  // uses TMA, so the prefetching thread and the waiting block always agree.
+  // Items alternate between the buffers, whether or not their frame uses TMA,
+  // so the prefetching thread and the waiting block always agree.
   uint32_t phases = 0;  // bit b: parity of buffer b's next completion
-  u64 acc[4] = {0, 0, 0, 0};
+  u64 acc = 0;
   unsigned int done = 0;
-  for (int item = r.x; item < r.y; ++item) {
+  // Tiles run down the 64-column strips of a frame; the lens shading maps and
+  // table are built for as many rows of a strip as come next (a band).
+  int band_begin = 0, band_end = 0;
+  LscTile lt{0, 0};
+  AwbCell cell;
+  const auto flush = [&] {
+    u64 total[4];
+    totals_of(acc, total);
+    awb_flush(fd, total, hist, fd.awb_mode == kWbWhitePatch, red, &last, done,
+              static_cast<unsigned int>(frames[f].awb_tiles));
+  };
+  int item = r.x;
+  int buf = 0;
+  while (true) {
     if (item >= frames[f].awb_begin + frames[f].awb_tiles) {
-      awb_flush(fd, acc, hist, fd.awb_mode == kWbWhitePatch, red, &last, done,
-                static_cast<unsigned int>(frames[f].awb_tiles));
+      flush();
       f = frame_of_item(frames, nframes, f, item, true);
       load_desc(&fd, &frames[f].desc);
       for (int i = tid; i < 3 * kAwbBins; i += kThreads) hist[i] = 0U;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) acc[k] = 0;
+      acc = 0;
       done = 0;
       __syncthreads();
     }
     const BatchFrame& bf = frames[f];
-    const int buf = (item - r.x) & 1;
     // The other buffer was read by the previous item (the block synchronised
-    // since): load the next item into it while this one is summed.
-    if (tid == 0 && item + 1 < r.y) {
-      const int g = frame_of_item(frames, nframes, f, item + 1, true);
-      if (frames[g].use_tma) {
-        fence_async_shared();
-        issue(g, item + 1, buf ^ 1);
+    // since): load the next item into it while this one is summed. The claimed
+    // range's slot alternates too: the next claim may follow within the next
+    // item, before every thread has read this one.
+    if (tid == 0) {
+      const int next = next_item(queue, item, r, next_range[buf], rec);
+      if (next >= 0) {
+        const int g = frame_of_item(frames, nframes, f, next, true);
+        if (frames[g].use_tma) {
+          fence_async_shared();
+          issue(g, next, buf ^ 1);
+        }
       }
     }
-    const int local = item - bf.awb_begin;
-    const int ty = local / bf.awb_tiles_x;
-    const int x0 = (local - ty * bf.awb_tiles_x) * 64;
+    const int tiles_y = bf.awb_tiles / bf.awb_tiles_x;
+    const int strip = (item - bf.awb_begin) / tiles_y;
+    const int ty = item - bf.awb_begin - strip * tiles_y;
+    const int x0 = strip * 64;
     const int y0 = ty * 64;
     const bool use_tma = bf.use_tma != 0;
     const int box_bytes = awb_box_bytes(fd.raw_format);
     if (!use_tma) {
       fill_box(fd, boxes + buf * 64 * 128, box_bytes, 64, awb_box_x(fd.raw_format, x0) * (fd.raw_format == kRawU16 ? 2 : 1), y0);
     }
-    const LscTile lt = build_lsc(fd, fd.lsc, fd.pattern, x0, 64, y0, 64, false, 0, 0, col_mx, col_ix, col_tx, row_my, row_k,
-                                 row_ty, table, minmax);
+    if (item >= band_end) {
+      band_begin = item;
+      band_end = min(min(item + tiles_y - ty, r.y), item + kAwbBandRows / 64);
+      lt = build_band_lsc(fd, fd.lsc, fd.pattern, x0, y0, (band_end - band_begin) * 64, m, minmax);
+      cell.k = -1;
+    }
+    const int rows = (item - band_begin) * 64;
     if (use_tma) {
       if (!mbar_wait(&bars[buf], (phases >> buf) & 1U) && tid == 0) report_wait_timeout(fd.scratch);
       phases ^= 1U << buf;
@@ -300,16 +370,19 @@ __global__ void __launch_bounds__(kThreads, 3) isp_awb_batch_kernel(const BatchF
     }
     unsigned int sum[3] = {0U, 0U, 0U};
     unsigned int quads = 0;
-    awb_tile_any(fd, fd.pattern, fd.awb_mode == kWbWhitePatch, boxes + buf * 64 * 128, box_bytes, x0, y0, lt, row_k, row_ty,
-                 table, black, inv, hist, sum, quads);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) acc[k] += sum[k];
-    acc[3] += quads;
+    awb_tile_any(fd, fd.pattern, fd.awb_mode == kWbWhitePatch, boxes + buf * 64 * 128, box_bytes, x0, y0, lt, m.row_k + rows,
+                 m.row_ty + rows, m.table, black, inv, hist, cell, sum, quads);
+    add_tile_sums(acc, sum[0], sum[1], sum[2], quads);
     __syncthreads();
     ++done;
+    if (++item == r.y) {
+      r = next_range[buf];
+      if (r.x >= r.y) break;
+      item = r.x;
+    }
+    buf ^= 1;
   }
-  awb_flush(fd, acc, hist, fd.awb_mode == kWbWhitePatch, red, &last, done,
-            static_cast<unsigned int>(frames[f].awb_tiles));
+  flush();
 }
 
 }  // namespace

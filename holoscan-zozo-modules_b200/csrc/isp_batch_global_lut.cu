@@ -5,6 +5,9 @@
 
 namespace isp_b200 {
 
-const void* batch_kernel_global_lut() { return reinterpret_cast<const void*>(&isp_batch_kernel<false, kTH>); }
+const void* batch_kernel_global_lut(bool sharpen) {
+  return sharpen ? reinterpret_cast<const void*>(&isp_batch_kernel<false, kTH, true>)
+                 : reinterpret_cast<const void*>(&isp_batch_kernel<false, kTH, false>);
+}
 
 }  // namespace isp_b200

@@ -17,7 +17,9 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
+#include <limits>
 #include <string>
 #include <vector>
 
@@ -42,9 +44,78 @@ struct Entry {
   isp_exposure_c exposure;
 };
 
+// Ranges of work items of a launch, in 8-byte entries from the start of a
+// slot's (and the device's) range memory: one per CTA of the tile pass, one per
+// CTA of the statistics pass, then each pass's BatchQueue with its ranges.
+constexpr int kQueuePerCta = 4;
+size_t queue_capacity(int max_ctas) { return static_cast<size_t>(kQueuePerCta) * static_cast<size_t>(max_ctas); }
+size_t queue_entries(int max_ctas) { return sizeof(BatchQueue) / sizeof(int2) + queue_capacity(max_ctas); }
+size_t range_entries(int max_ctas) { return 2U * static_cast<size_t>(max_ctas) + 2U * queue_entries(max_ctas); }
+BatchQueue* tile_queue(int2* ranges, int max_ctas) { return reinterpret_cast<BatchQueue*>(ranges + 2 * max_ctas); }
+BatchQueue* awb_queue(int2* ranges, int max_ctas) {
+  return reinterpret_cast<BatchQueue*>(ranges + 2 * max_ctas + queue_entries(max_ctas));
+}
+
+// Items of one cost each, in item order.
+struct CostRun {
+  int items;
+  double cost;
+};
+
+// Deals work items out: to each of `ctas` CTAs one contiguous range of even
+// cost, together the share `dealt` of the cost, and the rest to the queue in
+// ranges that shrink as it empties. CTAs then finish together although the costs
+// are estimates: with all of the work dealt out beforehand the SMs of a
+// 48-camera batch were idle for a tenth of the tile pass and a quarter of the
+// statistics pass. A frame's first item on a CTA costs a flush of its sums, so
+// few items per CTA, and claims of less than kLeast items, are not worth it.
+void deal(const std::vector<CostRun>& runs, int ctas, double dealt, int2* ranges, BatchQueue* queue, int capacity) {
+  constexpr int kLeast = 4;
+  double total = 0.0;
+  int items = 0;
+  for (const CostRun& r : runs) {
+    total += r.items * r.cost;
+    items += r.items;
+  }
+  const bool use_queue = items >= 4 * kLeast * ctas;
+  if (use_queue) total *= dealt;
+  int item = 0;
+  double acc = 0.0;
+  size_t run = 0;
+  int used = 0;  // of the run
+  for (int k = 0; k < ctas; ++k) {
+    const int begin = item;
+    const double goal = total * (k + 1) / ctas;
+    const bool all = k == ctas - 1 && !use_queue;
+    // An item belongs to the range its middle lies in.
+    while (run < runs.size()) {
+      const CostRun& r = runs[run];
+      const int left = r.items - used;
+      const double fit = std::floor((goal - acc) / r.cost + 0.5);
+      const int n = all || fit >= left ? left : fit > 0.0 ? static_cast<int>(fit) : 0;
+      item += n;
+      used += n;
+      acc += n * r.cost;
+      if (used < r.items) break;
+      ++run;
+      used = 0;
+    }
+    ranges[k] = make_int2(begin, item);
+  }
+  *queue = BatchQueue{};
+  auto* queued = reinterpret_cast<int2*>(queue + 1);
+  while (item < items) {
+    const int left = items - item;
+    const int room = capacity - queue->count;
+    const int size = std::min(left, std::max({kLeast, left / (2 * ctas), (left + room - 1) / room}));
+    queued[queue->count++] = make_int2(item, item + size);
+    item += size;
+  }
+}
+
 struct Slot {
   BatchFrame* frames = nullptr;  // pinned
-  int2* ranges = nullptr;        // pinned: tile pass then statistics pass
+  int2* ranges = nullptr;        // pinned
   const uint4* frames_dev = nullptr;  // the same memory as the device reads it
   const uint4* ranges_dev = nullptr;
   cudaEvent_t consumed = nullptr;
@@ -58,9 +129,10 @@ struct Shape {
   int awb_ctas = 0;
   bool lut_smem = false;
   int tile_rows = 64;
+  bool sharpen = false;  // some frame sharpens
   bool operator==(const Shape& o) const {
     return nframes == o.nframes && main_ctas == o.main_ctas && awb_ctas == o.awb_ctas && lut_smem == o.lut_smem &&
-           tile_rows == o.tile_rows;
+           tile_rows == o.tile_rows && sharpen == o.sharpen;
   }
 };
 
@@ -99,7 +171,9 @@ cudaError_t build(isp_b200_batch* b, const Slot& slot, Shape* shape) {
   const int n = static_cast<int>(b->entries.size());
   bool lut_smem = true;
   for (const Entry& e : b->entries) lut_smem = lut_smem && e.camera->state.tone_size <= kBatchLutEntries;
-  std::vector<float> tile_cost;
+  bool any_sharpen = false;
+  for (const Entry& e : b->entries) any_sharpen = any_sharpen || e.camera->params.c.sharpen > 0.0F;
+  std::vector<CostRun> tile_cost, awb_cost;
   int tiles = 0;
   int awb_tiles = 0;
   for (int i = 0; i < n; ++i) {
@@ -121,15 +195,17 @@ cudaError_t build(isp_b200_batch* b, const Slot& slot, Shape* shape) {
       f.awb_tiles = awb_kernel_tiles(e.raw.width, e.raw.height, &f.awb_tiles_x);
       tma_awb = encode_raw_map(f.desc, awb_box_row_bytes(e.raw.format), 64, &f.awb_map);
     }
+    awb_cost.push_back({f.awb_tiles, 1.0});
     f.awb_begin = awb_tiles;
     awb_tiles += f.awb_tiles;
     f.use_tma = tma_main && tma_awb ? 1 : 0;
-    tile_cost.insert(tile_cost.end(), static_cast<size_t>(f.tiles), b->weights[f.variant & 3]);
+    // Weights are positive, infinity included; the sums of costs are finite.
+    tile_cost.push_back({f.tiles, std::min(b->weights[f.variant & 3], std::numeric_limits<float>::max())});
   }
   // CTAs: as many as fit (or the tuned count) per SM, never more than items.
   int bpsm = 0;
-  const size_t smem = batch_kernel_smem(lut_smem, b->tile_rows);
-  error = blocks_per_sm(dev, batch_kernel(lut_smem, b->tile_rows), smem, smem, &bpsm);
+  const size_t smem = batch_kernel_smem(lut_smem, b->tile_rows, any_sharpen);
+  error = blocks_per_sm(dev, batch_kernel(lut_smem, b->tile_rows, any_sharpen), smem, smem, &bpsm);
   if (error != cudaSuccess) return error;
   if (b->ctas_per_sm > 0) bpsm = std::min(bpsm, b->ctas_per_sm);
   const int main_ctas = std::max(1, std::min({tiles, dev.sm_count * bpsm, b->max_ctas}));
@@ -137,30 +213,15 @@ cudaError_t build(isp_b200_batch* b, const Slot& slot, Shape* shape) {
   error = blocks_per_sm(dev, awb_batch_kernel(), awb_kernel_smem(), awb_kernel_smem(), &awb_bpsm);
   if (error != cudaSuccess) return error;
   const int awb_ctas = awb_tiles == 0 ? 0 : std::max(1, std::min({awb_tiles, dev.sm_count * awb_bpsm, b->max_ctas}));
-  // Contiguous ranges of even cost.
-  double total = 0.0;
-  for (const float c : tile_cost) total += c;
-  int item = 0;
-  double acc = 0.0;
-  for (int k = 0; k < main_ctas; ++k) {
-    const int begin = item;
-    const double goal = total * (k + 1) / main_ctas;
-    while (item < tiles && (acc + tile_cost[static_cast<size_t>(item)] * 0.5 <= goal || k == main_ctas - 1)) {
-      acc += tile_cost[static_cast<size_t>(item)];
-      ++item;
-    }
-    slot.ranges[k] = make_int2(begin, item);
-  }
-  for (int k = 0; k < awb_ctas; ++k) {
-    slot.ranges[b->max_ctas + k] =
-        make_int2(static_cast<int>(static_cast<int64_t>(awb_tiles) * k / awb_ctas),
-                  static_cast<int>(static_cast<int64_t>(awb_tiles) * (k + 1) / awb_ctas));
-  }
+  const int capacity = static_cast<int>(queue_capacity(b->max_ctas));
+  deal(tile_cost, main_ctas, 0.8, slot.ranges, tile_queue(slot.ranges, b->max_ctas), capacity);
+  deal(awb_cost, awb_ctas, 0.6, slot.ranges + b->max_ctas, awb_queue(slot.ranges, b->max_ctas), capacity);
   shape->nframes = n;
   shape->main_ctas = main_ctas;
   shape->awb_ctas = awb_ctas;
   shape->lut_smem = lut_smem;
   shape->tile_rows = b->tile_rows;
+  shape->sharpen = any_sharpen;
   return cudaSuccess;
 }
 
@@ -181,7 +242,7 @@ struct StageArgs {
         frame_words(static_cast<int>(sizeof(BatchFrame) / sizeof(uint4)) * s.nframes),
         ranges_src(slot.ranges_dev),
         ranges_dst(reinterpret_cast<uint4*>(b->d_ranges)),
-        range_words(b->max_ctas),  // 2 x max_ctas int2
+        range_words(static_cast<int>(range_entries(b->max_ctas) * sizeof(int2) / sizeof(uint4))),
         args{&frames_src, &frames_dst, &frame_words, &ranges_src, &ranges_dst, &range_words},
         grid((frame_words + range_words + kStageThreads - 1) / kStageThreads) {}
   StageArgs(const StageArgs&) = delete;
@@ -206,24 +267,26 @@ cudaError_t enqueue(isp_b200_batch* b, const Slot& slot, const Shape& s, cudaStr
   int nframes = s.nframes;
   const int2* awb_ranges = b->d_ranges + b->max_ctas;
   if (s.awb_ctas > 0) {
-    void* args[] = {&b->d_frames, &nframes, &awb_ranges};
+    auto* queue = awb_queue(b->d_ranges, b->max_ctas);
+    void* args[] = {&b->d_frames, &nframes, &awb_ranges, &queue};
     e = cudaLaunchKernel(awb_batch_kernel(), dim3(s.awb_ctas), dim3(kernel_threads()), args, awb_kernel_smem(), stream);
     if (e != cudaSuccess) return e;
   }
-  void* args[] = {&b->d_frames, &nframes, &b->d_ranges};
+  auto* queue = tile_queue(b->d_ranges, b->max_ctas);
+  void* args[] = {&b->d_frames, &nframes, &b->d_ranges, &queue};
   // After the statistics batch, as its programmatic dependent (the tile
   // batch waits for it in the kernel).
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(s.main_ctas);
   cfg.blockDim = dim3(kernel_threads());
-  cfg.dynamicSmemBytes = batch_kernel_smem(s.lut_smem, s.tile_rows);
+  cfg.dynamicSmemBytes = batch_kernel_smem(s.lut_smem, s.tile_rows, s.sharpen);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = s.awb_ctas > 0 ? 1 : 0;
-  return cudaLaunchKernelExC(&cfg, batch_kernel(s.lut_smem, s.tile_rows), args);
+  return cudaLaunchKernelExC(&cfg, batch_kernel(s.lut_smem, s.tile_rows, s.sharpen), args);
 }
 
 // Builds the graph of a shape: the descriptor staging, then the passes.
@@ -242,7 +305,8 @@ cudaError_t make_graph(isp_b200_batch* b, const Slot& slot, const Shape& s) {
   const int2* awb_ranges = b->d_ranges + b->max_ctas;
   cudaGraphNode_t awb = nullptr;
   if (s.awb_ctas > 0) {
-    void* args[] = {&b->d_frames, &nframes, &awb_ranges};
+    auto* queue = awb_queue(b->d_ranges, b->max_ctas);
+    void* args[] = {&b->d_frames, &nframes, &awb_ranges, &queue};
     cudaKernelNodeParams kp{};
     kp.func = const_cast<void*>(awb_batch_kernel());
     kp.gridDim = dim3(s.awb_ctas);
@@ -252,12 +316,13 @@ cudaError_t make_graph(isp_b200_batch* b, const Slot& slot, const Shape& s) {
     e = cudaGraphAddKernelNode(&awb, b->graph, &b->stage, 1, &kp);
     if (e != cudaSuccess) return e;
   }
-  void* args[] = {&b->d_frames, &nframes, &b->d_ranges};
+  auto* queue = tile_queue(b->d_ranges, b->max_ctas);
+  void* args[] = {&b->d_frames, &nframes, &b->d_ranges, &queue};
   cudaKernelNodeParams kp{};
-  kp.func = const_cast<void*>(batch_kernel(s.lut_smem, s.tile_rows));
+  kp.func = const_cast<void*>(batch_kernel(s.lut_smem, s.tile_rows, s.sharpen));
   kp.gridDim = dim3(s.main_ctas);
   kp.blockDim = dim3(kernel_threads());
-  kp.sharedMemBytes = static_cast<unsigned int>(batch_kernel_smem(s.lut_smem, s.tile_rows));
+  kp.sharedMemBytes = static_cast<unsigned int>(batch_kernel_smem(s.lut_smem, s.tile_rows, s.sharpen));
   kp.kernelParams = args;
   cudaGraphNode_t main = nullptr;
   if (awb != nullptr) {
@@ -309,10 +374,10 @@ int isp_b200_batch_create(int32_t capacity, isp_b200_batch** out) {
     b->max_ctas = dev.sm_count * 4;
     e = cudaMalloc(&b->d_frames, sizeof(BatchFrame) * static_cast<size_t>(capacity));
   }
-  if (e == cudaSuccess) e = cudaMalloc(&b->d_ranges, sizeof(int2) * 2 * static_cast<size_t>(b->max_ctas));
+  if (e == cudaSuccess) e = cudaMalloc(&b->d_ranges, sizeof(int2) * range_entries(b->max_ctas));
   for (Slot& s : b->slots) {
     if (e == cudaSuccess) e = cudaMallocHost(&s.frames, sizeof(BatchFrame) * static_cast<size_t>(capacity));
-    if (e == cudaSuccess) e = cudaMallocHost(&s.ranges, sizeof(int2) * 2 * static_cast<size_t>(b->max_ctas));
+    if (e == cudaSuccess) e = cudaMallocHost(&s.ranges, sizeof(int2) * range_entries(b->max_ctas));
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s.consumed, cudaEventDisableTiming);
     void* dev = nullptr;
     if (e == cudaSuccess) e = cudaHostGetDevicePointer(&dev, s.frames, 0);

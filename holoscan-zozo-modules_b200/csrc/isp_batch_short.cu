@@ -4,8 +4,9 @@
 
 namespace isp_b200 {
 
-const void* batch_kernel_shared_lut_short() {
-  return reinterpret_cast<const void*>(&isp_batch_kernel<true, kTHShort>);
+const void* batch_kernel_shared_lut_short(bool sharpen) {
+  return sharpen ? reinterpret_cast<const void*>(&isp_batch_kernel<true, kTHShort, true>)
+                 : reinterpret_cast<const void*>(&isp_batch_kernel<true, kTHShort, false>);
 }
 
 }  // namespace isp_b200

@@ -4,8 +4,9 @@
 
 namespace isp_b200 {
 
-const void* batch_kernel_global_lut_short() {
-  return reinterpret_cast<const void*>(&isp_batch_kernel<false, kTHShort>);
+const void* batch_kernel_global_lut_short(bool sharpen) {
+  return sharpen ? reinterpret_cast<const void*>(&isp_batch_kernel<false, kTHShort, true>)
+                 : reinterpret_cast<const void*>(&isp_batch_kernel<false, kTHShort, false>);
 }
 
 }  // namespace isp_b200

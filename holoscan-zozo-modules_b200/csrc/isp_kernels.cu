@@ -2,7 +2,7 @@
 // kernels (isp_main_*.cu, isp_awb.cu).
 #include <algorithm>
 
-#include "isp_common.cuh"
+#include "isp_awb.cuh"
 
 namespace isp_b200 {
 
@@ -41,16 +41,23 @@ const void* main_kernel_bn_short(int layout, bool lut_smem, int out_format);
 const void* main_kernel_bs_short(int layout, bool lut_smem, int out_format);
 const void* main_kernel_mn_short(int layout, bool lut_smem, int out_format);
 const void* main_kernel_ms_short(int layout, bool lut_smem, int out_format);
-const void* batch_kernel_shared_lut();
-const void* batch_kernel_global_lut();
-const void* batch_kernel_shared_lut_short();
-const void* batch_kernel_global_lut_short();
+const void* batch_kernel_shared_lut(bool sharpen);
+const void* batch_kernel_global_lut(bool sharpen);
+const void* batch_kernel_shared_lut_short(bool sharpen);
+const void* batch_kernel_global_lut_short(bool sharpen);
 
 int tile_rows_valid(int tile_rows) { return tile_rows == kTH ? kTH : tile_rows == kTHShort ? kTHShort : 0; }
 
-const void* batch_kernel(bool lut_smem, int tile_rows) {
-  if (tile_rows == kTHShort) return lut_smem ? batch_kernel_shared_lut_short() : batch_kernel_global_lut_short();
-  return lut_smem ? batch_kernel_shared_lut() : batch_kernel_global_lut();
+const void* batch_kernel(bool lut_smem, int tile_rows, bool sharpen) {
+  if (tile_rows == kTHShort) {
+    return lut_smem ? batch_kernel_shared_lut_short(sharpen) : batch_kernel_global_lut_short(sharpen);
+  }
+  return lut_smem ? batch_kernel_shared_lut(sharpen) : batch_kernel_global_lut(sharpen);
+}
+
+size_t batch_kernel_smem(bool lut_smem, int tile_rows, bool sharpen) {
+  return static_cast<size_t>(layout_of(sharpen, box_row_bytes(kRawU16), lut_smem ? kBatchLutEntries : 0, tile_rows).total) +
+         128U;
 }
 
 const void* main_kernel(bool malvar, bool sharpen, int pattern, bool lut_smem, int out_format, int tile_rows) {
@@ -85,12 +92,7 @@ int main_kernel_tiles(int width, int height, int* tiles_x, int tile_rows) {
 
 int kernel_threads() { return kThreads; }
 
-size_t awb_kernel_smem() {
-  // two boxes of 64 x 128, lens shading table, column maps (64) and row maps
-  // (a band's rows), white-patch histogram, the frame's lens shading grid.
-  return 2U * 64U * 128U + kLscTableRows * 2U * kSW * 4U + 3U * 64U * 4U + 3U * kAwbBandRows * 4U +
-         3U * kAwbBins * 4U + kGridSmemGains * 4U + 128U;
-}
+size_t awb_kernel_smem() { return static_cast<size_t>(kAwbSmem) + 128U; }
 
 int awb_kernel_bands(int width, int height, int ctas, int* strips, int* tiles_y, int* band_tiles) {
   // Strips of 64 columns over the complete quads, cut into bands of whole

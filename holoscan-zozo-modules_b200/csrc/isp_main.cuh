@@ -94,20 +94,9 @@ __device__ __forceinline__ Span<const float> frame_grid(const FrameDesc& p, cons
   return p.lsc != nullptr && gains <= kGridSmemGains ? Span<const float>(m.grid) : p.lsc;
 }
 
-// Reads the frame's gains (its estimate, for auto white balance) into m.quad and, with
-// kFill, fills the frame's shared memory (fill_frame_smem, its copies waited
-// for; without kFill the caller filled it before and waits for the copies).
-// The caller synchronises the block before the first tile.
-template <bool kLutSmem, bool kFill = true>
-__device__ __forceinline__ FrameSetup setup_frame(const FrameDesc& p, const TileSmem& m) {
-  if constexpr (kFill) fill_frame_smem<kLutSmem>(p, m);
+template <bool kLutSmem>
+__device__ __forceinline__ FrameSetup frame_setup(const FrameDesc& p, const TileSmem& m) {
   FrameSetup f;
-  if (threadIdx.x < kQuadFloats) {
-    const int t = threadIdx.x;
-    const int ch = t < 12 ? cfa_of(p.pattern, t & 3) : 0;
-    const int color = t < 12 ? color_of(ch) : t - 12;
-    m.quad[t] = t < 4 ? p.black[ch] : t < 8 ? p.inv_range[ch] : p.auto_wb ? __ldcg(&p.scratch->awb_gains[color]) : p.wb[color];
-  }
   f.grid = frame_grid(p, m);
   f.lut = kLutSmem ? m.lut_s : p.tone;
   f.lut_scale = static_cast<float>(p.tone_size - 1);
@@ -117,8 +106,24 @@ __device__ __forceinline__ FrameSetup setup_frame(const FrameDesc& p, const Tile
   f.swap_rb = (p.pattern & 1) != 0;
   f.want_hist = p.hist_out != nullptr;
   f.want_stats = p.stats_out != nullptr;
-  if constexpr (kFill) cp_async_wait_all();
   return f;
+}
+
+// Reads the frame's gains (its estimate, for auto white balance) into m.quad and, with
+// kFill, fills the frame's shared memory (fill_frame_smem, its copies waited
+// for; without kFill the caller filled it before and waits for the copies).
+// The caller synchronises the block before the first tile.
+template <bool kLutSmem, bool kFill = true>
+__device__ __forceinline__ FrameSetup setup_frame(const FrameDesc& p, const TileSmem& m) {
+  if constexpr (kFill) fill_frame_smem<kLutSmem>(p, m);
+  if (threadIdx.x < kQuadFloats) {
+    const int t = threadIdx.x;
+    const int ch = t < 12 ? cfa_of(p.pattern, t & 3) : 0;
+    const int color = t < 12 ? color_of(ch) : t - 12;
+    m.quad[t] = t < 4 ? p.black[ch] : t < 8 ? p.inv_range[ch] : p.auto_wb ? __ldcg(&p.scratch->awb_gains[color]) : p.wb[color];
+  }
+  if constexpr (kFill) cp_async_wait_all();
+  return frame_setup<kLutSmem>(p, m);
 }
 
 // Output units u (0..511) of phase C: an output row r and group uc of four

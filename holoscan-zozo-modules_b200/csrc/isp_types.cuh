@@ -115,4 +115,13 @@ struct alignas(64) BatchFrame {
   int use_tma;
 };
 
+// The end of a batch's tile pass: ranges of work items that CTAs claim when
+// they are done with their own, so that they finish together whatever the
+// frames' real costs. Followed in memory by the ranges.
+struct alignas(16) BatchQueue {
+  int count;             // ranges in the queue
+  unsigned int claimed;  // so far; the descriptor staging sets it to 0
+  int pad[2];
+};
+
 }  // namespace isp_b200
