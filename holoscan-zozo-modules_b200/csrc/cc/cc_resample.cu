@@ -52,10 +52,10 @@ static const void* resample_kernel(const Plan& p) {
   return resample_kernel_other(src, p.mode, key);
 }
 
-const void* direct_kernel(int src, int dst) {
-  if (src <= CC_UYVY) return direct_kernel_yuv(src, dst);
-  if (src <= CC_BGRA8) return direct_kernel_rgb(src, dst);
-  return direct_kernel_gray(src, dst);
+const void* direct_kernel(int src, int dst, bool wide) {
+  if (src <= CC_UYVY) return direct_kernel_yuv(src, dst, wide);
+  if (src <= CC_BGRA8) return direct_kernel_rgb(src, dst, wide);
+  return direct_kernel_gray(src, dst, wide);
 }
 
 // Whether every content pixel reads exactly the source pixel under it: the
@@ -77,12 +77,16 @@ int launch_convert(const Plan& plan, void* stream) {
   int down, per_block_x;
   const void* fn;
   if (direct) {
-    // A block's warp covers kSub x 32 groups.
     const FormatInfo fi = info_of(p.dst.format);
     const int rows = fi.model == kYuv ? (1 << fi.shift_y) : 1;
     down = (p.dst.height + rows - 1) / rows;
-    per_block_x = kThreadsX * direct_subgroups(p.dst.format);
-    fn = direct_kernel(p.src.format, p.dst.format);
+    // Few large blocks once they still fill the chip twice over.
+    constexpr int kWave = kSms * kDirectBlocksPerSm;
+    per_block_x = kThreadsX * direct_subgroups(p.dst.format, true);
+    const long long blocks = static_cast<long long>((across + per_block_x - 1) / per_block_x) * ((down + kThreadsY - 1) / kThreadsY);
+    const bool wide = blocks >= 2 * kWave;
+    per_block_x = kThreadsX * direct_subgroups(p.dst.format, wide);
+    fn = direct_kernel(p.src.format, p.dst.format, wide);
   } else {
     const int rows = resample_rows(p.dst.format);
     down = (p.dst.height + rows - 1) / rows;
@@ -93,7 +97,8 @@ int launch_convert(const Plan& plan, void* stream) {
   const int rows = direct ? down : (p.dst.height + (1 << p.bsy) - 1) >> p.bsy;
   if (fn == nullptr || (rows + kThreadsY - 1) / kThreadsY > 65535) return static_cast<int>(cudaErrorInvalidValue);
   const int blocks_down = std::min((down + static_cast<int>(block.y) - 1) / static_cast<int>(block.y), 65535);
-  const dim3 grid(static_cast<unsigned>((across + per_block_x - 1) / per_block_x), static_cast<unsigned>(blocks_down));
+  const int blocks_across = (across + per_block_x - 1) / per_block_x;
+  const dim3 grid(static_cast<unsigned>(blocks_across), static_cast<unsigned>(blocks_down));
   void* args[] = {&p, &across, &down};
   return static_cast<int>(isp_b200::launch_dependent(fn, grid, block, args, static_cast<cudaStream_t>(stream)));
 }
