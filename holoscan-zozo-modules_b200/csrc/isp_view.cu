@@ -36,20 +36,10 @@ struct ViewArgs {
   size_t out_pitch;
 };
 
-// One raw sample's counts (view_op.cu:35-51; isp_math.hpp:101-119).
-__device__ __forceinline__ int view_sample(const uint8_t* row, int format, int x) {
-  switch (format) {
-    case ISP_RAW_U8: return __ldg(row + x);
-    case ISP_RAW_U16: return __ldg(row + 2 * x) | (__ldg(row + 2 * x + 1) << 8);
-    case ISP_RAW_RAW10: {
-      const uint8_t* g = row + 5 * (x >> 2);
-      return (__ldg(g + (x & 3)) << 2) | ((__ldg(g + 4) >> (2 * (x & 3))) & 3);
-    }
-    default: {
-      const uint8_t* g = row + 3 * (x >> 1);
-      return (__ldg(g + (x & 1)) << 4) | ((__ldg(g + 2) >> (4 * (x & 1))) & 15);
-    }
-  }
+// Bytes of n samples of a row, from a run's start.
+template <int kFormat>
+__device__ __forceinline__ int raw_bytes(int n) {
+  return kFormat == ISP_RAW_U8 ? n : kFormat == ISP_RAW_U16 ? 2 * n : kFormat == ISP_RAW_RAW10 ? (n + 3) / 4 * 5 : (n + 1) / 2 * 3;
 }
 
 // The gray code of one sample: (s - black) * scale clamped to [0, 1], its
@@ -63,13 +53,14 @@ __device__ __forceinline__ uint32_t view_gray(int s, float black, float scale) {
 constexpr int kRun = 16;             // pixels of a thread
 constexpr int kTableMax = 4096;      // gray codes kept per block
 constexpr int kViewThreads = 256;
+constexpr int kViewBlocksPerSm = 5;
 
 // 32-bit words of sixteen samples.
 __host__ __device__ constexpr int run_words(int format) {
   return format == ISP_RAW_U8 ? 4 : format == ISP_RAW_U16 ? 8 : format == ISP_RAW_RAW10 ? 5 : 6;
 }
 
-// The sixteen samples of a run's words. Packed formats as in load_raw: RAW10
+// The sixteen samples of a run's words (view_op.cu:35-51; isp_math.hpp:101-119). Packed formats as in load_raw: RAW10
 // holds four pixels in five bytes, RAW12 two in three.
 template <int kFormat>
 __device__ __forceinline__ void view_samples(const uint32_t (&w)[run_words(kFormat)], uint32_t (&s)[kRun]) {
@@ -90,13 +81,34 @@ __device__ __forceinline__ void view_samples(const uint32_t (&w)[run_words(kForm
   }
 }
 
+// The 32-bit word at any address, from the aligned words that hold its bytes.
+__device__ __forceinline__ uint32_t word_at(const uint8_t* p) {
+  const unsigned int s = static_cast<unsigned int>(reinterpret_cast<uintptr_t>(p)) & 3U;
+  const uint32_t* base = reinterpret_cast<const uint32_t*>(p - s);
+  return __funnelshift_r(__ldg(base), s != 0U ? __ldg(base + 1) : 0U, 8U * s);
+}
+
+// A warp writes `bytes` bytes at dst, wherever it starts: aligned words from
+// word(offset), the few bytes before and after them from byte(offset).
+template <class Word, class Byte>
+__device__ __forceinline__ void put_bytes(uint8_t* dst, int bytes, Word word, Byte byte) {
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  const int head = min(static_cast<int>(-reinterpret_cast<uintptr_t>(dst) & 3U), bytes);
+  const int n = (bytes - head) >> 2;
+  const int end = head + 4 * n;
+#pragma unroll 2
+  for (int j = lane; j < n; j += 32) *reinterpret_cast<uint32_t*>(dst + head + 4 * j) = word(head + 4 * j);
+  if (lane < head) dst[lane] = byte(lane);
+  if (lane < bytes - end) dst[end + lane] = byte(end + lane);
+}
+
 // A warp takes `tiles` of 32 runs of 16 pixels (tiles_x across the frame's
-// runs_x runs), striding over the frame with the grid's other warps. Where the
-// rows allow it (16-byte aligned RGB and view rows, 4-byte aligned raw rows)
-// whole runs move as described above; a row's last, shorter run and the runs of
-// other rows byte by byte.
+// width), striding over the frame with the grid's other warps. Where the rows
+// allow it (16-byte aligned RGB and view rows, 4-byte aligned raw rows) the
+// runs move as 16-byte words; elsewhere as the aligned 4-byte words that hold
+// them, shifted on the way (1646x1647 U8: 139 us pixel by pixel).
 template <int kFormat, bool kTable>
-__global__ void __launch_bounds__(kViewThreads) isp_view_kernel(const __grid_constant__ ViewArgs a, int runs_x, int tiles_x,
+__global__ void __launch_bounds__(kViewThreads, kViewBlocksPerSm) isp_view_kernel(const __grid_constant__ ViewArgs a, int tiles_x,
                                                                 int tiles, int table_size) {
   constexpr int kWords = run_words(kFormat);
   __shared__ uint8_t table[kTable ? kTableMax : 4];
@@ -129,71 +141,91 @@ __global__ void __launch_bounds__(kViewThreads) isp_view_kernel(const __grid_con
     uint8_t* right = left + 3 * static_cast<size_t>(a.width);
     const bool vec = ((reinterpret_cast<uintptr_t>(rgb) | reinterpret_cast<uintptr_t>(left) |
                        reinterpret_cast<uintptr_t>(right)) & 15U) == 0U && (reinterpret_cast<uintptr_t>(raw) & 3U) == 0U;
-    const int whole = vec ? min(a.width / kRun - run0, 32) : 0;  // the tile's runs moved as words
-    if (whole > 0) {
-      const uint32_t* from = reinterpret_cast<const uint32_t*>(raw) + static_cast<size_t>(run0) * kWords;
-      const uint4* pixels = reinterpret_cast<const uint4*>(rgb) + static_cast<size_t>(run0) * 3;
-      uint4* beside = reinterpret_cast<uint4*>(right) + static_cast<size_t>(run0) * 3;
-      uint4* below = reinterpret_cast<uint4*>(left) + static_cast<size_t>(run0) * 3;
-      uint32_t w[kWords];
+    const int pixels_here = min(a.width - kRun * run0, 32 * kRun);
+    const int whole = pixels_here / kRun;  // all of the tile's, where vec
+    raw += static_cast<size_t>(run0) * (4 * kWords);
+    rgb += static_cast<size_t>(run0) * (3 * kRun);
+    left += static_cast<size_t>(run0) * (3 * kRun);
+    right += static_cast<size_t>(run0) * (3 * kRun);
+    const uint4* pixels = reinterpret_cast<const uint4*>(rgb);
+    uint4* beside = reinterpret_cast<uint4*>(right);
+    uint4* below = reinterpret_cast<uint4*>(left);
+    uint32_t w[kWords];
+    uint4 c[3];
+    if (vec) {
+      const uint32_t* from = reinterpret_cast<const uint32_t*>(raw);
 #pragma unroll
       for (int k = 0; k < kWords; ++k) w[k] = lane + 32 * k < whole * kWords ? __ldg(from + lane + 32 * k) : 0U;
-      uint4 c[3];
 #pragma unroll
       for (int k = 0; k < 3; ++k) c[k] = lane + 32 * k < 3 * whole ? __ldg(pixels + lane + 32 * k) : make_uint4(0U, 0U, 0U, 0U);
+    } else {
+      // Aligned words that hold at least a byte of the row's; zeros past its end.
+      const int bytes = raw_bytes<kFormat>(pixels_here);
+      const unsigned int s = static_cast<unsigned int>(reinterpret_cast<uintptr_t>(raw)) & 3U;
+      const uint32_t* from = reinterpret_cast<const uint32_t*>(raw - s);
 #pragma unroll
-      for (int k = 0; k < kWords; ++k) words[lane + 32 * k] = w[k];
-      __syncwarp();
-      if constexpr (kWords % 4 == 0) {
-#pragma unroll
-        for (int k = 0; k < kWords / 4; ++k) {
-          const uint4 v = stage[lane * (kWords / 4) + k];
-          w[4 * k] = v.x;
-          w[4 * k + 1] = v.y;
-          w[4 * k + 2] = v.z;
-          w[4 * k + 3] = v.w;
-        }
-      } else {
-#pragma unroll
-        for (int k = 0; k < kWords; ++k) w[k] = words[lane * kWords + k];
+      for (int k = 0; k < kWords; ++k) {
+        const int i = lane + 32 * k;
+        const uint32_t lo = 4 * i < bytes + static_cast<int>(s) ? __ldg(from + i) : 0U;
+        const uint32_t hi = s != 0U && 4 * i + 4 < bytes + static_cast<int>(s) ? __ldg(from + i + 1) : 0U;
+        w[k] = __funnelshift_r(lo, hi, 8U * s);
       }
-      __syncwarp();
+    }
+#pragma unroll
+    for (int k = 0; k < kWords; ++k) words[lane + 32 * k] = w[k];
+    __syncwarp();
+    if constexpr (kWords % 4 == 0) {
+#pragma unroll
+      for (int k = 0; k < kWords / 4; ++k) {
+        const uint4 v = stage[lane * (kWords / 4) + k];
+        w[4 * k] = v.x;
+        w[4 * k + 1] = v.y;
+        w[4 * k + 2] = v.z;
+        w[4 * k + 3] = v.w;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < kWords; ++k) w[k] = words[lane * kWords + k];
+    }
+    __syncwarp();
+    if (vec) {
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         if (lane + 32 * k < 3 * whole) beside[lane + 32 * k] = c[k];
       }
-      uint32_t g[kRun];
-      view_samples<kFormat>(w, g);
+    }
+    uint32_t g[kRun];
+    view_samples<kFormat>(w, g);
 #pragma unroll
-      for (int i = 0; i < kRun; ++i) g[i] = gray(g[i]);
-      // Gray pixels: bytes g, g, g per pixel; four of them, a b c d, as the
-      // words aaab bbcc cddd.
-      uint32_t o[12];
+    for (int i = 0; i < kRun; ++i) g[i] = gray(g[i]);
+    // Gray pixels: bytes g, g, g per pixel; four of them, a b c d, as the
+    // words aaab bbcc cddd.
+    uint32_t o[12];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        o[3 * k] = __byte_perm(g[4 * k], g[4 * k + 1], 0x4000U);
-        o[3 * k + 1] = __byte_perm(g[4 * k + 1], g[4 * k + 2], 0x4400U);
-        o[3 * k + 2] = __byte_perm(g[4 * k + 2], g[4 * k + 3], 0x4440U);
-      }
+    for (int k = 0; k < 4; ++k) {
+      o[3 * k] = __byte_perm(g[4 * k], g[4 * k + 1], 0x4000U);
+      o[3 * k + 1] = __byte_perm(g[4 * k + 1], g[4 * k + 2], 0x4400U);
+      o[3 * k + 2] = __byte_perm(g[4 * k + 2], g[4 * k + 3], 0x4440U);
+    }
 #pragma unroll
-      for (int k = 0; k < 3; ++k) stage[3 * lane + k] = make_uint4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
-      __syncwarp();
+    for (int k = 0; k < 3; ++k) stage[3 * lane + k] = make_uint4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
+    __syncwarp();
+    if (vec) {
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         if (lane + 32 * k < 3 * whole) below[lane + 32 * k] = stage[lane + 32 * k];
       }
-      __syncwarp();
+    } else {
+      put_bytes(right, 3 * pixels_here, [&](int at) { return word_at(rgb + at); }, [&](int at) { return __ldg(rgb + at); });
+      put_bytes(
+          left, 3 * pixels_here,
+          [&](int at) {
+            const int k = at >> 2;
+            return (at & 3) == 0 ? words[k] : __funnelshift_r(words[k], words[k + 1], 8U * (static_cast<unsigned int>(at) & 3U));
+          },
+          [&](int at) { return static_cast<uint8_t>(words[at >> 2] >> (8 * (at & 3))); });
     }
-    if (lane >= whole && run0 + lane < runs_x) {
-      const int x0 = kRun * (run0 + lane);
-      const int x1 = min(x0 + kRun, a.width);
-      for (int x = x0; x < x1; ++x) {
-        const uint8_t g = static_cast<uint8_t>(gray(static_cast<uint32_t>(view_sample(raw, kFormat, x))));
-        left[3 * static_cast<size_t>(x)] = left[3 * static_cast<size_t>(x) + 1] = left[3 * static_cast<size_t>(x) + 2] = g;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) right[3 * static_cast<size_t>(x) + k] = __ldg(rgb + 3 * static_cast<size_t>(x) + k);
-      }
-    }
+    __syncwarp();
   }
 }
 
@@ -243,13 +275,11 @@ extern "C" ISP_B200_API int isp_b200_view_compose(const isp_raw_view_c* raw, flo
   if (e != cudaSuccess) return fail_cuda(e, "view kernel");
   // As many blocks as are resident at once, each with the same number of
   // rounds over the frame's tiles.
-  constexpr int64_t kBlocksPerSm = 5;
   constexpr int64_t kWarps = kViewThreads / 32;
-  int runs_x = (raw->width + kRun - 1) / kRun;
-  int tiles_x = (runs_x + 31) / 32;
+  int tiles_x = (raw->width + 32 * kRun - 1) / (32 * kRun);
   const int64_t total = static_cast<int64_t>(tiles_x) * raw->height;
   const int64_t needed = (total + kWarps - 1) / kWarps;
-  const int64_t rounds = (needed + shapes.sm_count * kBlocksPerSm - 1) / (shapes.sm_count * kBlocksPerSm);
+  const int64_t rounds = (needed + shapes.sm_count * int64_t{kViewBlocksPerSm} - 1) / (shapes.sm_count * int64_t{kViewBlocksPerSm});
   const int64_t blocks = (needed + rounds - 1) / rounds;
   // The table costs each thread table_size / 256 codes; a 12-bit one pays from
   // the second round on (of two: 16 codes instead of 32). Every sample a packed
@@ -257,7 +287,7 @@ extern "C" ISP_B200_API int isp_b200_view_compose(const isp_raw_view_c* raw, flo
   int table_size = 1 << (raw->format == ISP_RAW_U16 ? raw->bit_depth : max_bits);
   const bool table = table_size <= kTableMax && (table_size <= 1024 || rounds >= 2);
   int tiles = static_cast<int>(total);
-  void* args[] = {&a, &runs_x, &tiles_x, &tiles, &table_size};
+  void* args[] = {&a, &tiles_x, &tiles, &table_size};
   e = launch_dependent(view_kernel(raw->format, table), dim3(static_cast<unsigned>(blocks)), dim3(kViewThreads), args,
                        static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail_cuda(e, "view kernel");
