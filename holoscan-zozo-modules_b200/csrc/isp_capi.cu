@@ -579,7 +579,7 @@ int isp_b200_process(isp_b200_pipeline* pl, const isp_raw_view_c* raw, const isp
   }
   const char* step = "launch";
   error = launch_frame(d, pl->params.c, shapes, stream, pl->before_main, pl->after_main, &step,
-                       overlap, pl->rows_for(*raw));
+                       overlap, pl->rows_for(*raw, shapes.sm_count));
   if (error == cudaSuccess) error = cudaGetLastError();
   if (error != cudaSuccess) return fail_cuda(error, (std::string("IspPipeline (cuda) ") + step).c_str());
   error = cudaEventRecord(pl->done, stream);

@@ -139,14 +139,22 @@ struct isp_b200_pipeline {
   };
   ShapePick picks[8] = {};  // isp_b200_autotune's choices, oldest replaced first
   int npicks = 0;
-  // The tile height for a frame: the forced one, the shape's pick, else 64.
-  int rows_for(const isp_raw_view_c& raw) const {
+  // The tile height for a frame: the forced one, the shape's pick, else 64 or,
+  // for a frame of so few tiles that SMs would stay idle, 32. Frames back to back
+  // on one stream, 64 / 32 rows (U16, gray world when sharpened): sharpened
+  // 96x64 21.8 / 13.7 us, 640x480 17.1 / 16.0, 960x540 (135 tiles) 19.9 / 16.3,
+  // 1000x700 (176) 22.0 / 22.9; not sharpened 96x64 13.5 / 9.4 us, 320x240 10.4 /
+  // 9.2, 640x360 (120 short tiles) 10.3 / 10.0, 640x480 (150) 10.6 / 10.8, 800x600
+  // 11.2 / 12.2.
+  int rows_for(const isp_raw_view_c& raw, int sms) const {
     if (tile_rows != 0) return tile_rows;
     for (int i = 0; i < npicks && i < 8; ++i) {
       const ShapePick& k = picks[i];
       if (k.format == raw.format && k.width == raw.width && k.height == raw.height) return k.rows;
     }
-    return 64;
+    const int64_t across = (static_cast<int64_t>(raw.width) + 63) / 64;
+    const int rows = params.c.sharpen > 0.0F ? 64 : 32;  // of the tiles counted
+    return across * ((static_cast<int64_t>(raw.height) + rows - 1) / rows) <= sms ? 32 : 64;
   }
   // Staging for isp_b200_process_host, grown on demand.
   cudaStream_t host_stream = nullptr;

@@ -428,7 +428,8 @@ ISP_B200_API int isp_b200_noalloc_status(void* stream, int32_t* status);
  * The pass is compiled for 64-row tiles (two CTAs per SM) and 32-row tiles
  * (three CTAs per SM: a frame of few tiles spreads over more SMs). 0 (the
  * default) uses the height isp_b200_autotune picked for the frame's raw
- * format and size, else 64; 64 or 32 force it for every frame. Outputs are
+ * format and size, else 32 for frames of few tiles and 64 for others; 64 or 32
+ * force it for every frame. Outputs are
  * bit-identical either way. ISP_EINVAL for any other value. */
 ISP_B200_API int isp_b200_set_tile_rows(isp_b200_pipeline* pipeline, int32_t tile_rows);
 
