@@ -512,8 +512,14 @@ __device__ __noinline__ void edge_group(const Plan& p, int xs, int y0) {
 // groups are read first; then each is converted and stored. groups_x =
 // ceil(width / 4).
 //
-// At 3840x2160 what bounds it is instruction issue, then memory: RGB8 -> NV12
-// moves 37.3 MB (5.8 us at the copy bandwidth).
+// What bounds it at 3840x2160 is the FP32 pipes and instruction issue: RGB8 ->
+// NV12, 37.3 MB (5.8 us at the copy bandwidth), executes 28 instructions a pixel,
+// 12.8 of them two-lane FP32 ones that hold both pipes two cycles each (72 % of
+// the active cycles). Passes before groups were lane pairs, and now (inputs
+// in L2): RGB8 -> NV12 12.1 and 10.6 us, NV12 -> RGB8 13.5 and 10.7, YUYV ->
+// NV12 8.0 and 5.7; rows at any byte: 3839x2159 NV12 -> RGB8 32.7 and 17.1 us,
+// 2001x1500 MONO16 -> RGB16 52.5 and 12.2. The checks come before the loads, once
+// for the warp: between them they cost 10 % (12.0 against 10.7 us).
 template <int kSrc, int kDst, int kSub>
 __global__ void __launch_bounds__(kThreadsX* kThreadsY, kDirectBlocksPerSm)
     cc_direct_kernel(const __grid_constant__ Plan p, int groups_x, int groups_y) {
