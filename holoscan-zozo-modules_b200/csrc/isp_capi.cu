@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -50,14 +51,32 @@ constexpr int kCfa[4][4] = {
 // (frame_overlap), whichever camera it belongs to. With the cameras of a rig
 // in turn on one stream, each waiting for its own last frame, no two frames
 // overlapped. If the caller queued other work since, the wait keeps the
-// frame behind all of it.
+// frame behind all of it; this library's own kernels that signal their
+// dependents early (launch_dependent) take the stream's entry away, and a
+// frame that finds none does not overlap: it may read what they write.
 std::mutex g_tails_mutex;
 std::map<unsigned long long, isp_b200_pipeline*> g_tails;
+std::atomic<size_t> g_tail_count{0};  // of g_tails, for a look without the lock
 
 void drop_stream_tail(isp_b200_pipeline& pl) {
   std::lock_guard<std::mutex> lock(g_tails_mutex);
   const auto it = g_tails.find(pl.tail_stream_id);
   if (it != g_tails.end() && it->second == &pl) g_tails.erase(it);
+  g_tail_count = g_tails.size();
+}
+
+void forget_stream_tail(cudaStream_t stream) {
+  if (g_tail_count == 0) return;
+  unsigned long long id = 0;
+  const bool known = cudaStreamGetId(stream, &id) == cudaSuccess;
+  if (!known) static_cast<void>(cudaGetLastError());
+  std::lock_guard<std::mutex> lock(g_tails_mutex);
+  if (known) {
+    g_tails.erase(id);
+  } else {
+    g_tails.clear();
+  }
+  g_tail_count = g_tails.size();
 }
 
 void set_stream_tail(isp_b200_pipeline& pl) {
@@ -69,11 +88,12 @@ void set_stream_tail(isp_b200_pipeline& pl) {
     pl.tail_stream_id = pl.last_stream_id;
   }
   g_tails[pl.tail_stream_id] = &pl;
+  g_tail_count = g_tails.size();
 }
 
-// Waits as described above. `overlap` is cleared when the raw frame lies in
-// the image that the stream's last frame writes: its statistics pass must then
-// not start under that frame's end.
+// Waits as described above. `overlap` is cleared when the stream has no entry,
+// and when the raw frame lies in the image that the stream's last frame writes:
+// its statistics pass must then not start under that frame's end.
 cudaError_t wait_for_stream_tail(cudaStream_t stream, isp_b200_pipeline& pl, const isp_raw_view_c& raw, bool* overlap) {
   // A capturing stream waits for the pipeline's own event as it always did:
   // that decides what the capture may depend on.
@@ -84,7 +104,11 @@ cudaError_t wait_for_stream_tail(cudaStream_t stream, isp_b200_pipeline& pl, con
   }
   std::lock_guard<std::mutex> lock(g_tails_mutex);  // keeps the event's pipeline alive
   const auto it = g_tails.find(pl.last_stream_id);
-  const isp_b200_pipeline& tail = it != g_tails.end() ? *it->second : pl;
+  if (it == g_tails.end()) {
+    *overlap = false;
+    return cudaStreamWaitEvent(stream, pl.done, 0);
+  }
+  const isp_b200_pipeline& tail = *it->second;
   const auto begin = reinterpret_cast<uintptr_t>(raw.data);
   const uintptr_t end = begin + raw.pitch * static_cast<size_t>(raw.height);
   if (begin < tail.last_out_end && tail.last_out_begin < end) *overlap = false;
@@ -346,6 +370,7 @@ cudaError_t launch_dependent(const void* kernel, dim3 grid, dim3 block, void** a
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = capture == cudaStreamCaptureStatusNone ? 1 : 0;
+  if (capture == cudaStreamCaptureStatusNone) forget_stream_tail(stream);
   return cudaLaunchKernelExC(&cfg, kernel, args);
 }
 

@@ -444,7 +444,7 @@ ISP_B200_API int isp_b200_autotune(isp_b200_pipeline* pipeline, const isp_raw_vi
                                    int32_t* tile_rows);
 
 /* Frame overlap, no reference counterpart (on by default): when frames of
- * one pipeline follow each other on one stream, the next frame's white
+ * any pipelines follow each other on one stream, the next frame's white
  * balance statistics pass may begin while the previous frame's tile pass
  * finishes (a programmatic dependent launch); its estimate still waits for
  * that pass, so every output is the one the frames give alone. The pass reads
