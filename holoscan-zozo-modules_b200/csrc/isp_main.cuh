@@ -491,9 +491,21 @@ __global__ void __launch_bounds__(kThreads, kTileH == kTH ? 2 : 3)
     // claim's round trip hidden behind phase B, the copy behind phase C), so
     // that claims are made as late as the box allows and the frame's last
     // tiles go to the CTAs that are free first; without sharpening (no phase
-    // B) it is claimed at the tile's start and its box requested after A.
+    // B) it is claimed at the tile's start and its box requested after A. The
+    // first claim comes after wait_frame: the counter is the pipeline's, and
+    // until then its previous frame may still count by it and clear it at its
+    // end. (Claimed before the wait, the frame of another size that followed on
+    // the stream skipped tiles by the old count and did others twice.)
     unsigned int claim = 0;
-    if (!kSharpen && threadIdx.x == 0) claim = gridDim.x + atomicAdd(&p.scratch->tile_next, 1U);
+    const auto claim_next = [&] {
+      if (threadIdx.x == 0) claim = gridDim.x + atomicAdd(&p.scratch->tile_next, 1U);
+    };
+    if (!kSharpen && waited) claim_next();
+    const auto begin = [&] {
+      if (waited) return;
+      wait_frame();
+      if constexpr (!kSharpen) claim_next();
+    };
     const auto request = [&] {
       if (threadIdx.x == 0) {
         next_tile = static_cast<int>(claim);
@@ -505,7 +517,7 @@ __global__ void __launch_bounds__(kThreads, kTileH == kTH ? 2 : 3)
     };
     const auto after_a = [&] {
       if constexpr (kSharpen) {
-        if (threadIdx.x == 0) claim = gridDim.x + atomicAdd(&p.scratch->tile_next, 1U);
+        claim_next();
       } else {
         request();
       }
@@ -514,7 +526,7 @@ __global__ void __launch_bounds__(kThreads, kTileH == kTH ? 2 : 3)
       if constexpr (kSharpen) request();
     };
     run_tile<kMalvar, kSharpen, kLayout, kLutSmem, kOut, kTileH>(p, f, m, minmax, x0, ty * kTileH, use_tma != 0, &bar,
-                                                                 phase, acc, after_a, before_c, wait_frame);
+                                                                 phase, acc, after_a, before_c, begin);
     ++done;
     tile = next_tile;  // written before run_tile's closing barrier
   }
