@@ -91,17 +91,23 @@ void set_stream_tail(isp_b200_pipeline& pl) {
   g_tail_count = g_tails.size();
 }
 
+// Whether work queued on the stream now is captured (or may be). A capturing
+// stream's id must not be asked for (that ends the capture with an error), and a
+// captured frame is none of the stream's work: its event was recorded in the
+// capture, and no frame outside may wait for it. So captured frames stay out of
+// the map, and each waits for its pipeline's own event, which decides what the
+// capture may depend on.
+bool is_capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusActive;
+  if (cudaStreamIsCapturing(stream, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
+  static_cast<void>(cudaGetLastError());
+  return true;
+}
+
 // Waits as described above. `overlap` is cleared when the stream has no entry,
 // and when the raw frame lies in the image that the stream's last frame writes:
 // its statistics pass must then not start under that frame's end.
 cudaError_t wait_for_stream_tail(cudaStream_t stream, isp_b200_pipeline& pl, const isp_raw_view_c& raw, bool* overlap) {
-  // A capturing stream waits for the pipeline's own event as it always did:
-  // that decides what the capture may depend on.
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
-  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
-    static_cast<void>(cudaGetLastError());
-    return cudaStreamWaitEvent(stream, pl.done, 0);
-  }
   std::lock_guard<std::mutex> lock(g_tails_mutex);  // keeps the event's pipeline alive
   const auto it = g_tails.find(pl.last_stream_id);
   if (it == g_tails.end()) {
@@ -356,11 +362,7 @@ cudaError_t blocks_per_sm(LaunchShapes& shapes, const void* kernel, size_t smem_
 }
 
 cudaError_t launch_dependent(const void* kernel, dim3 grid, dim3 block, void** args, cudaStream_t stream) {
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
-  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {
-    static_cast<void>(cudaGetLastError());
-    capture = cudaStreamCaptureStatusActive;
-  }
+  const bool captured = is_capturing(stream);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -369,8 +371,8 @@ cudaError_t launch_dependent(const void* kernel, dim3 grid, dim3 block, void** a
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = capture == cudaStreamCaptureStatusNone ? 1 : 0;
-  if (capture == cudaStreamCaptureStatusNone) forget_stream_tail(stream);
+  cfg.numAttrs = captured ? 0 : 1;
+  if (!captured) forget_stream_tail(stream);
   return cudaLaunchKernelExC(&cfg, kernel, args);
 }
 
@@ -596,7 +598,8 @@ int isp_b200_process(isp_b200_pipeline* pl, const isp_raw_view_c* raw, const isp
   // previous frame first (cuda_pipeline.cu:304-310). On the same stream the
   // next frame's statistics pass may still overlap this one's end
   // (frame_overlap): it follows the tile pass as its programmatic dependent.
-  const bool same_stream = pl->follows_on(stream);
+  const bool captured = is_capturing(stream);
+  const bool same_stream = !captured && pl->follows_on(stream);
   bool overlap = same_stream && pl->frame_overlap;
   if (pl->queued) {
     error = same_stream ? wait_for_stream_tail(stream, *pl, *raw, &overlap) : cudaStreamWaitEvent(stream, pl->done, 0);
@@ -612,7 +615,7 @@ int isp_b200_process(isp_b200_pipeline* pl, const isp_raw_view_c* raw, const isp
   pl->queued = true;
   pl->last_out_begin = reinterpret_cast<uintptr_t>(out->data);
   pl->last_out_end = pl->last_out_begin + out->pitch * static_cast<size_t>(raw->height);
-  pl->set_last_stream(stream);
+  pl->set_last_stream(stream, captured);
   set_stream_tail(*pl);
   clear_error();
   return ISP_OK;
@@ -760,7 +763,7 @@ int isp_b200_check_bounded_wait(isp_b200_pipeline* pl, uint32_t polls, void* str
   if (error == cudaSuccess) error = cudaEventRecord(pl->done, stream);
   if (error != cudaSuccess) return fail_cuda(error, "isp_b200_check_bounded_wait");
   pl->queued = true;
-  pl->set_last_stream(stream);
+  pl->set_last_stream(stream, is_capturing(stream));
   clear_error();
   return ISP_OK;
 }

@@ -123,11 +123,11 @@ struct isp_b200_pipeline {
   bool last_stream_known = false;
   uintptr_t last_out_begin = 0, last_out_end = 0;  // the image of the last queued frame
   unsigned long long tail_stream_id = 0;  // the stream it may stand as the last frame of (isp_capi.cu)
-  void set_last_stream(cudaStream_t stream) {
-    last_stream_known = cudaStreamGetId(stream, &last_stream_id) == cudaSuccess;
+  void set_last_stream(cudaStream_t stream, bool captured) {
+    last_stream_known = !captured && cudaStreamGetId(stream, &last_stream_id) == cudaSuccess;
   }
-  // Whether `stream` is the one of the last queued frame, so that its order is
-  // the frames' order.
+  // Whether `stream`, which does not capture, is the one of the last queued
+  // frame, so that its order is the frames' order.
   bool follows_on(cudaStream_t stream) const {
     unsigned long long id = 0;
     return queued && last_stream_known && cudaStreamGetId(stream, &id) == cudaSuccess && id == last_stream_id;
