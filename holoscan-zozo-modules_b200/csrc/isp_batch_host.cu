@@ -493,7 +493,7 @@ int isp_b200_batch_launch(isp_b200_batch* b, void* stream_ptr, int32_t use_graph
     e = cudaEventRecord(en.camera->done, stream);
     if (e != cudaSuccess) return fail_cuda(e, "cudaEventRecord");
     en.camera->queued = true;
-    en.camera->last_stream_known = false;  // its next frame waits for the event
+    en.camera->last = {};  // its next frame waits for the event
   }
   clear_error();
   return ISP_OK;

@@ -10,7 +10,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -41,84 +40,51 @@ constexpr int kCfa[4][4] = {
     {kChGb, kChB, kChR, kChGr},
 };
 
-// The pipeline whose frame was queued last on each stream (by stream id): at
-// most one entry per live pipeline, removed when the pipeline moves to
-// another stream or is destroyed. A frame that follows on its stream waits
-// for that frame's event instead of its own pipeline's last one. Both come
-// earlier in the stream, so either order is right; but when nothing was queued
-// since, the wait is for the stream's last operation, which costs nothing and
-// leaves the frame's kernels free to start under that frame's end
-// (frame_overlap), whichever camera it belongs to. With the cameras of a rig
-// in turn on one stream, each waiting for its own last frame, no two frames
-// overlapped. If the caller queued other work since, the wait keeps the
-// frame behind all of it; this library's own kernels that signal their
-// dependents early (launch_dependent) take the stream's entry away, and a
-// frame that finds none does not overlap: it may read what they write.
-std::mutex g_tails_mutex;
-std::map<unsigned long long, isp_b200_pipeline*> g_tails;
-std::atomic<size_t> g_tail_count{0};  // of g_tails, for a look without the lock
+StreamTails<isp_b200_pipeline> g_tails;
 
-void drop_stream_tail(isp_b200_pipeline& pl) {
-  std::lock_guard<std::mutex> lock(g_tails_mutex);
-  const auto it = g_tails.find(pl.tail_stream_id);
-  if (it != g_tails.end() && it->second == &pl) g_tails.erase(it);
-  g_tail_count = g_tails.size();
-}
-
-void forget_stream_tail(cudaStream_t stream) {
-  if (g_tail_count == 0) return;
-  unsigned long long id = 0;
-  const bool known = cudaStreamGetId(stream, &id) == cudaSuccess;
-  if (!known) static_cast<void>(cudaGetLastError());
-  std::lock_guard<std::mutex> lock(g_tails_mutex);
-  if (known) {
-    g_tails.erase(id);
-  } else {
-    g_tails.clear();
-  }
-  g_tail_count = g_tails.size();
-}
-
-void set_stream_tail(isp_b200_pipeline& pl) {
-  if (!pl.last_stream_known) return drop_stream_tail(pl);
-  std::lock_guard<std::mutex> lock(g_tails_mutex);
-  if (pl.tail_stream_id != pl.last_stream_id) {
-    const auto it = g_tails.find(pl.tail_stream_id);
-    if (it != g_tails.end() && it->second == &pl) g_tails.erase(it);
-    pl.tail_stream_id = pl.last_stream_id;
-  }
-  g_tails[pl.tail_stream_id] = &pl;
-  g_tail_count = g_tails.size();
-}
-
-// Whether work queued on the stream now is captured (or may be). A capturing
-// stream's id must not be asked for (that ends the capture with an error), and a
-// captured frame is none of the stream's work: its event was recorded in the
-// capture, and no frame outside may wait for it. So captured frames stay out of
-// the map, and each waits for its pipeline's own event, which decides what the
-// capture may depend on.
-bool is_capturing(cudaStream_t stream) {
+// Where the next work on the stream will come. (A capturing stream's id must not
+// be asked for: that ends the capture with an error.)
+StreamKey place_of(cudaStream_t stream) {
+  StreamKey key;
+  int device = -1;
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusActive;
-  if (cudaStreamIsCapturing(stream, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
-  static_cast<void>(cudaGetLastError());
-  return true;
+  unsigned long long capture = 0;
+  const cudaGraphNode_t* nodes = nullptr;
+  const cudaGraphEdgeData* edges = nullptr;
+  size_t count = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e == cudaSuccess) e = cudaStreamGetCaptureInfo_v3(stream, &status, &capture, nullptr, &nodes, &edges, &count);
+  key.capturing = e != cudaSuccess || status != cudaStreamCaptureStatusNone;
+  if (e == cudaSuccess && key.capturing && count == 1) {
+    key.device = device;
+    key.capture = capture;
+    key.at = reinterpret_cast<uintptr_t>(nodes[0]);
+  } else if (!key.capturing) {
+    e = cudaStreamGetId(stream, &key.at);
+    if (e == cudaSuccess) key.device = device;
+  }
+  if (e != cudaSuccess) static_cast<void>(cudaGetLastError());
+  return key;
 }
 
-// Waits as described above. `overlap` is cleared when the stream has no entry,
-// and when the raw frame lies in the image that the stream's last frame writes:
-// its statistics pass must then not start under that frame's end.
-cudaError_t wait_for_stream_tail(cudaStream_t stream, isp_b200_pipeline& pl, const isp_raw_view_c& raw, bool* overlap) {
-  std::lock_guard<std::mutex> lock(g_tails_mutex);  // keeps the event's pipeline alive
-  const auto it = g_tails.find(pl.last_stream_id);
-  if (it == g_tails.end()) {
-    *overlap = false;
-    return cudaStreamWaitEvent(stream, pl.done, 0);
-  }
-  const isp_b200_pipeline& tail = *it->second;
-  const auto begin = reinterpret_cast<uintptr_t>(raw.data);
-  const uintptr_t end = begin + raw.pitch * static_cast<size_t>(raw.height);
-  if (begin < tail.last_out_end && tail.last_out_begin < end) *overlap = false;
-  return cudaStreamWaitEvent(stream, tail.done, 0);
+// Waits for the work that a frame at `here` follows (isp_tails.hpp): `follows`,
+// whether its pipeline's last frame comes earlier in the same order. `overlap`
+// is cleared when the frame must not start under the end of the work before it:
+// that work is no frame, or its image holds the raw samples, which the frame's
+// statistics pass reads before it waits. In a capture each frame waits for its
+// pipeline's own event, which decides what the capture may depend on.
+cudaError_t wait_for_stream_tail(cudaStream_t stream, const StreamKey& here, bool follows, isp_b200_pipeline& pl,
+                                 const isp_raw_view_c& raw, bool* overlap) {
+  cudaError_t error = cudaSuccess;
+  const auto tail = [&](const StreamTails<isp_b200_pipeline>::Tail& t) {
+    const auto begin = reinterpret_cast<uintptr_t>(raw.data);
+    const uintptr_t end = begin + raw.pitch * static_cast<size_t>(raw.height);
+    if (begin < t.out_end && t.out_begin < end) *overlap = false;
+    error = cudaStreamWaitEvent(stream, here.capturing ? pl.done : t.owner->done, 0);
+  };
+  if (follows && g_tails.find(here, tail)) return error;
+  *overlap = false;
+  return cudaStreamWaitEvent(stream, pl.done, 0);
 }
 
 std::mutex g_shapes_mutex;
@@ -362,7 +328,7 @@ cudaError_t blocks_per_sm(LaunchShapes& shapes, const void* kernel, size_t smem_
 }
 
 cudaError_t launch_dependent(const void* kernel, dim3 grid, dim3 block, void** args, cudaStream_t stream) {
-  const bool captured = is_capturing(stream);
+  const StreamKey here = place_of(stream);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -371,8 +337,8 @@ cudaError_t launch_dependent(const void* kernel, dim3 grid, dim3 block, void** a
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = captured ? 0 : 1;
-  if (!captured) forget_stream_tail(stream);
+  cfg.numAttrs = here.capturing ? 0 : 1;
+  if (!here.capturing && !g_tails.empty()) g_tails.forget(here);
   return cudaLaunchKernelExC(&cfg, kernel, args);
 }
 
@@ -534,7 +500,7 @@ int isp_b200_create(const isp_params_c* params, isp_b200_pipeline** out) {
 
 void isp_b200_destroy(isp_b200_pipeline* pl) {
   if (pl == nullptr) return;
-  drop_stream_tail(*pl);
+  g_tails.drop(pl);
   if (pl->queued) cudaEventSynchronize(pl->done);
   if (pl->host_stream != nullptr) cudaStreamSynchronize(pl->host_stream);
   device_state_free(&pl->state);
@@ -598,11 +564,11 @@ int isp_b200_process(isp_b200_pipeline* pl, const isp_raw_view_c* raw, const isp
   // previous frame first (cuda_pipeline.cu:304-310). On the same stream the
   // next frame's statistics pass may still overlap this one's end
   // (frame_overlap): it follows the tile pass as its programmatic dependent.
-  const bool captured = is_capturing(stream);
-  const bool same_stream = !captured && pl->follows_on(stream);
-  bool overlap = same_stream && pl->frame_overlap;
+  const StreamKey here = place_of(stream);
+  const bool follows = pl->follows(here);
+  bool overlap = follows && pl->frame_overlap;
   if (pl->queued) {
-    error = same_stream ? wait_for_stream_tail(stream, *pl, *raw, &overlap) : cudaStreamWaitEvent(stream, pl->done, 0);
+    error = wait_for_stream_tail(stream, here, follows, *pl, *raw, &overlap);
     if (error != cudaSuccess) return fail_cuda(error, "cudaStreamWaitEvent");
   }
   const char* step = "launch";
@@ -613,10 +579,9 @@ int isp_b200_process(isp_b200_pipeline* pl, const isp_raw_view_c* raw, const isp
   error = cudaEventRecord(pl->done, stream);
   if (error != cudaSuccess) return fail_cuda(error, "cudaEventRecord");
   pl->queued = true;
-  pl->last_out_begin = reinterpret_cast<uintptr_t>(out->data);
-  pl->last_out_end = pl->last_out_begin + out->pitch * static_cast<size_t>(raw->height);
-  pl->set_last_stream(stream, captured);
-  set_stream_tail(*pl);
+  pl->last = here.capturing ? place_of(stream) : here;
+  const auto image = reinterpret_cast<uintptr_t>(out->data);
+  g_tails.set(pl->last, {pl, image, image + out->pitch * static_cast<size_t>(raw->height)});
   clear_error();
   return ISP_OK;
 }
@@ -763,7 +728,7 @@ int isp_b200_check_bounded_wait(isp_b200_pipeline* pl, uint32_t polls, void* str
   if (error == cudaSuccess) error = cudaEventRecord(pl->done, stream);
   if (error != cudaSuccess) return fail_cuda(error, "isp_b200_check_bounded_wait");
   pl->queued = true;
-  pl->set_last_stream(stream, is_capturing(stream));
+  pl->last = place_of(stream);
   clear_error();
   return ISP_OK;
 }

@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "isp_b200.h"
+#include "isp_tails.hpp"
 #include "isp_types.cuh"
 
 namespace isp_b200 {
@@ -117,20 +118,11 @@ struct isp_b200_pipeline {
   int device = 0;
   cudaEvent_t done = nullptr;
   bool queued = false;
-  // The stream of the last queued frame: its id, which unlike a handle is
-  // never used again, when known.
-  unsigned long long last_stream_id = 0;
-  bool last_stream_known = false;
-  uintptr_t last_out_begin = 0, last_out_end = 0;  // the image of the last queued frame
-  unsigned long long tail_stream_id = 0;  // the stream it may stand as the last frame of (isp_capi.cu)
-  void set_last_stream(cudaStream_t stream, bool captured) {
-    last_stream_known = !captured && cudaStreamGetId(stream, &last_stream_id) == cudaSuccess;
-  }
-  // Whether `stream`, which does not capture, is the one of the last queued
-  // frame, so that its order is the frames' order.
-  bool follows_on(cudaStream_t stream) const {
-    unsigned long long id = 0;
-    return queued && last_stream_known && cudaStreamGetId(stream, &id) == cudaSuccess && id == last_stream_id;
+  isp_b200::StreamKey last;  // where the last queued frame went
+  // Whether work at `here` comes after the last queued frame in its order.
+  bool follows(const isp_b200::StreamKey& here) const {
+    return queued && here.known() && last.known() && here.device == last.device && here.capture == last.capture &&
+           (here.capturing || here.at == last.at);
   }
   bool frame_overlap = true;           // isp_b200_set_frame_overlap
   int tile_rows = 0;                   // isp_b200_set_tile_rows: 0 = per shape (isp_b200_autotune), else 64 / 32

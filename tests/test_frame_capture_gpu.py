@@ -4,7 +4,7 @@ import pytest
 
 import isp_b200
 from gpu_support import DeviceFrame, same_bits, torch_cuda
-from isp_b200 import abi, scene
+from isp_b200 import abi, cc, scene
 
 pytestmark = pytest.mark.gpu
 
@@ -85,3 +85,51 @@ def test_a_captured_frame_is_not_waited_for_by_others():
     for i, f in enumerate(frames):
         same(f, want[i], i)
     same(inside, captured_want[0], "captured")
+
+
+@pytest.mark.parametrize("balance", [abi.MANUAL, abi.GRAY_WORLD])
+def test_captured_cameras_in_turn(balance):
+    """Frames of two cameras in one graph, each behind the other's."""
+    torch = torch_cuda()
+    raws = [raw_frame(i) for i in range(3)]
+    want = alone(raws + raws, balance)
+    pipes, stream = [isp_b200.Pipeline(params(balance)) for _ in range(2)], torch.cuda.Stream()
+    frames = [[DeviceFrame(raw, abi.RGB8) for raw in raws] for _ in pipes]
+    torch.cuda.synchronize()
+    graph = capture(stream, lambda: [f[i].run(pipe, stream=stream.cuda_stream) for i in range(3)
+                                     for f, pipe in zip(frames, pipes)])
+    for k in (0, 3):
+        with torch.cuda.stream(stream):
+            graph.replay()
+        for camera in frames:
+            for i, f in enumerate(camera):
+                same(f, want[k + i], k + i)
+
+
+@pytest.mark.parametrize("balance", [abi.MANUAL, abi.GRAY_WORLD])
+def test_a_captured_frame_waits_for_the_conversion_before_it(balance):
+    """frame, conversion into the raw samples of the next, frame: in one graph, replayed with changing sources."""
+    torch = torch_cuda()
+    raws = [raw_frame(i) for i in range(4)]
+    want = alone([raws[i] for i in (0, 1, 2, 3)], balance)
+    pipe, converter, stream = isp_b200.Pipeline(params(balance)), cc.Converter(), torch.cuda.Stream()
+    sources = [torch.zeros_like(DeviceFrame(raws[0], abi.RGB8).raw) for _ in range(2)]
+    frames = [DeviceFrame(raws[0], abi.RGB8) for _ in range(2)]
+    copy = cc.params(cc.BT709, mode=cc.NEAREST)
+
+    def queue():
+        for source, f in zip(sources, frames):
+            converter.convert(cc.packed_view(source.data_ptr(), cc.MONO16, W, H),
+                              cc.packed_view(f.raw.data_ptr(), cc.MONO16, W, H), copy, stream.cuda_stream)
+            f.run(pipe, stream=stream.cuda_stream)
+
+    torch.cuda.synchronize()
+    graph = capture(stream, queue)
+    for k in (0, 2):
+        for i, source in enumerate(sources):
+            source.copy_(torch.from_numpy(raws[k + i].data))
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            graph.replay()
+        for i, f in enumerate(frames):
+            same(f, want[k + i], k + i)
