@@ -328,7 +328,12 @@ cudaError_t blocks_per_sm(LaunchShapes& shapes, const void* kernel, size_t smem_
 }
 
 cudaError_t launch_dependent(const void* kernel, dim3 grid, dim3 block, void** args, cudaStream_t stream) {
-  const StreamKey here = place_of(stream);
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusActive;
+  if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
+    static_cast<void>(cudaGetLastError());
+    status = cudaStreamCaptureStatusActive;
+  }
+  const bool capturing = status != cudaStreamCaptureStatusNone;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -337,9 +342,10 @@ cudaError_t launch_dependent(const void* kernel, dim3 grid, dim3 block, void** a
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = here.capturing ? 0 : 1;
-  if (!here.capturing && !g_tails.empty()) g_tails.forget(here);
-  return cudaLaunchKernelExC(&cfg, kernel, args);
+  cfg.numAttrs = capturing ? 0 : 1;
+  const cudaError_t e = cudaLaunchKernelExC(&cfg, kernel, args);
+  if (!capturing && !g_tails.idle()) g_tails.forget(place_of(stream));
+  return e;
 }
 
 cudaError_t launch_frame(const FrameDesc& d, const isp_params_c& p, LaunchShapes& shapes, cudaStream_t stream,
@@ -565,6 +571,7 @@ int isp_b200_process(isp_b200_pipeline* pl, const isp_raw_view_c* raw, const isp
   // next frame's statistics pass may still overlap this one's end
   // (frame_overlap): it follows the tile pass as its programmatic dependent.
   const StreamKey here = place_of(stream);
+  StreamTails<isp_b200_pipeline>::Call call(g_tails, here);
   const bool follows = pl->follows(here);
   bool overlap = follows && pl->frame_overlap;
   if (pl->queued) {
@@ -581,7 +588,7 @@ int isp_b200_process(isp_b200_pipeline* pl, const isp_raw_view_c* raw, const isp
   pl->queued = true;
   pl->last = here.capturing ? place_of(stream) : here;
   const auto image = reinterpret_cast<uintptr_t>(out->data);
-  g_tails.set(pl->last, {pl, image, image + out->pitch * static_cast<size_t>(raw->height)});
+  call.finish({pl, image, image + out->pitch * static_cast<size_t>(raw->height)}, pl->last);
   clear_error();
   return ISP_OK;
 }

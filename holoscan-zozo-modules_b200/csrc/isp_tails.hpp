@@ -40,12 +40,66 @@ struct StreamKey {
 
 // At most one entry per frame owner (a live pipeline), removed when its next
 // frame goes elsewhere or it is destroyed.
+//
+// Several threads may queue work on one stream, and an entry must not outlive
+// work queued behind its frame by another thread. So a frame is queued within a
+// Call, other work is announced after its launch (forget), and a frame in whose
+// Call anything else was announced at the same place gets no entry: which of the
+// two came last on the stream is not known.
 template <class Owner>
 class StreamTails {
  public:
   struct Tail {
     Owner* owner;
     uintptr_t out_begin, out_end;  // the frame's image
+  };
+
+  // From before a frame's first operation until its event is recorded. A Call
+  // that ends without that may have queued a part of the frame: no entry stays.
+  class Call {
+   public:
+    Call(StreamTails& tails, const StreamKey& key) : tails_(tails), key_(key) {
+      std::lock_guard<std::mutex> lock(tails_.mutex_);
+      next_ = tails_.calls_;
+      tails_.calls_ = this;
+      tails_.recount();
+    }
+    ~Call() {
+      std::lock_guard<std::mutex> lock(tails_.mutex_);
+      leave();
+      if (!finished_) tails_.announce(key_);
+      tails_.recount();
+    }
+    Call(const Call&) = delete;
+    Call& operator=(const Call&) = delete;
+
+    // The frame is queued, and the next work will come at `place` (the Call's
+    // own outside captures).
+    void finish(const Tail& tail, const StreamKey& place) {
+      std::lock_guard<std::mutex> lock(tails_.mutex_);
+      leave();
+      finished_ = true;
+      tails_.announce(key_);
+      tails_.remove(tail.owner);
+      if (!disturbed_ && place.known()) tails_.put(place, tail);
+      tails_.recount();
+    }
+
+   private:
+    friend class StreamTails;
+    void leave() {
+      for (Call** c = &tails_.calls_; *c != nullptr; c = &(*c)->next_) {
+        if (*c == this) {
+          *c = next_;
+          break;
+        }
+      }
+    }
+    StreamTails& tails_;
+    const StreamKey key_;
+    Call* next_ = nullptr;
+    bool disturbed_ = false;
+    bool finished_ = false;
   };
 
   // Calls f(tail) with the register locked, so that the owner stays alive;
@@ -59,41 +113,31 @@ class StreamTails {
     return true;
   }
 
-  void set(const StreamKey& key, const Tail& tail) {
-    std::lock_guard<std::mutex> lock(mutex_);
-    remove(tail.owner);
-    if (key.known()) {
-      const auto it = tails_.find(key);
-      if (it != tails_.end()) places_.erase(it->second.owner);
-      tails_[key] = tail;
-      places_[tail.owner] = key;
-    }
-    count_ = tails_.size();
-  }
-
   void drop(Owner* owner) {
     std::lock_guard<std::mutex> lock(mutex_);
     remove(owner);
-    count_ = tails_.size();
+    recount();
   }
 
-  // Takes the entry at `key` away, or every entry when the place is unknown.
+  // Without the lock: whether there is nothing to forget. Asked after the launch
+  // of other work, since a frame's Call that begins later queues behind it.
+  bool idle() const { return count_ == 0; }
+
+  // Work other than a frame was queued at `key`, by a call that returns after this.
   void forget(const StreamKey& key) {
     std::lock_guard<std::mutex> lock(mutex_);
-    if (key.known()) {
-      const auto it = tails_.find(key);
-      if (it != tails_.end()) remove(it->second.owner);
-    } else {
-      tails_.clear();
-      places_.clear();
-    }
-    count_ = tails_.size();
+    announce(key);
+    recount();
   }
 
-  // Without the lock: whether there is anything to forget.
-  bool empty() const { return count_ == 0; }
-
  private:
+  void put(const StreamKey& key, const Tail& tail) {
+    const auto it = tails_.find(key);
+    if (it != tails_.end()) places_.erase(it->second.owner);
+    tails_[key] = tail;
+    places_[tail.owner] = key;
+  }
+
   void remove(Owner* owner) {
     const auto it = places_.find(owner);
     if (it == places_.end()) return;
@@ -101,10 +145,30 @@ class StreamTails {
     places_.erase(it);
   }
 
+  // Work was queued at `key`, or, when that is unknown, anywhere. (At an unknown
+  // place of a capture there is no entry.)
+  void announce(const StreamKey& key) {
+    if (!key.known() && key.capturing) return;
+    for (Call* c = calls_; c != nullptr; c = c->next_) {
+      if (!key.known() || !c->key_.known() || same(c->key_, key)) c->disturbed_ = true;
+    }
+    if (key.known()) {
+      const auto it = tails_.find(key);
+      if (it != tails_.end()) remove(it->second.owner);
+    } else {
+      tails_.clear();
+      places_.clear();
+    }
+  }
+
+  static bool same(const StreamKey& a, const StreamKey& b) { return !(a < b) && !(b < a); }
+  void recount() { count_ = tails_.size() + (calls_ != nullptr ? 1 : 0); }
+
   std::mutex mutex_;
   std::map<StreamKey, Tail> tails_;
   std::map<Owner*, StreamKey> places_;
-  std::atomic<size_t> count_{0};
+  Call* calls_ = nullptr;
+  std::atomic<size_t> count_{0};  // entries, and one more while there are Calls
 };
 
 }  // namespace isp_b200
