@@ -327,6 +327,8 @@ cudaError_t blocks_per_sm(LaunchShapes& shapes, const void* kernel, size_t smem_
   return cudaSuccess;
 }
 
+void drop_stream_tail(isp_b200_pipeline* pl) { g_tails.drop(pl); }
+
 cudaError_t launch_dependent(const void* kernel, dim3 grid, dim3 block, void** args, cudaStream_t stream) {
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusActive;
   if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
@@ -506,7 +508,7 @@ int isp_b200_create(const isp_params_c* params, isp_b200_pipeline** out) {
 
 void isp_b200_destroy(isp_b200_pipeline* pl) {
   if (pl == nullptr) return;
-  g_tails.drop(pl);
+  drop_stream_tail(pl);
   if (pl->queued) cudaEventSynchronize(pl->done);
   if (pl->host_stream != nullptr) cudaStreamSynchronize(pl->host_stream);
   device_state_free(&pl->state);
@@ -732,10 +734,11 @@ int isp_b200_check_bounded_wait(isp_b200_pipeline* pl, uint32_t polls, void* str
     void* args[] = {&scratch, &n};
     error = cudaLaunchKernel(wait_check_kernel(), dim3(1), dim3(32), args, 0, stream);
   }
+  drop_stream_tail(pl);
+  pl->last = {};  // its next frame waits for the event
   if (error == cudaSuccess) error = cudaEventRecord(pl->done, stream);
   if (error != cudaSuccess) return fail_cuda(error, "isp_b200_check_bounded_wait");
   pl->queued = true;
-  pl->last = place_of(stream);
   clear_error();
   return ISP_OK;
 }

@@ -15,6 +15,8 @@
 #include "isp_tails.hpp"
 #include "isp_types.cuh"
 
+struct isp_b200_pipeline;
+
 namespace isp_b200 {
 
 void params_default(isp_params_c* p);
@@ -101,6 +103,10 @@ LaunchShapes& shapes_for_current_device(cudaError_t* error);
 // kernel of 6.5 us takes 8.2, one of 11.2 us 14.3). While the stream captures,
 // a plain launch: the graph gets the full dependency it always had.
 cudaError_t launch_dependent(const void* kernel, dim3 grid, dim3 block, void** args, cudaStream_t stream);
+
+// For whoever records a pipeline's `done` elsewhere than behind a single frame:
+// frames of other pipelines no longer wait for it.
+void drop_stream_tail(isp_b200_pipeline* pl);
 
 // Queues one frame's kernels on `stream` (no host synchronisation).
 // before_main / after_main (may be null) are recorded around the fused tile kernel.
