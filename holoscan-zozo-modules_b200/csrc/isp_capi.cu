@@ -329,6 +329,10 @@ cudaError_t blocks_per_sm(LaunchShapes& shapes, const void* kernel, size_t smem_
 
 void drop_stream_tail(isp_b200_pipeline* pl) { g_tails.drop(pl); }
 
+void forget_stream_tail(cudaStream_t stream) {
+  if (!g_tails.idle()) g_tails.forget(place_of(stream));
+}
+
 cudaError_t launch_dependent(const void* kernel, dim3 grid, dim3 block, void** args, cudaStream_t stream) {
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusActive;
   if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
@@ -346,7 +350,7 @@ cudaError_t launch_dependent(const void* kernel, dim3 grid, dim3 block, void** a
   cfg.attrs = attr;
   cfg.numAttrs = capturing ? 0 : 1;
   const cudaError_t e = cudaLaunchKernelExC(&cfg, kernel, args);
-  if (!capturing && !g_tails.idle()) g_tails.forget(place_of(stream));
+  if (!capturing) forget_stream_tail(stream);
   return e;
 }
 

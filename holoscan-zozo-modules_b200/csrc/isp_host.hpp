@@ -107,6 +107,10 @@ cudaError_t launch_dependent(const void* kernel, dim3 grid, dim3 block, void** a
 // For whoever records a pipeline's `done` elsewhere than behind a single frame:
 // frames of other pipelines no longer wait for it.
 void drop_stream_tail(isp_b200_pipeline* pl);
+// For whoever queued a kernel that lets its dependents start early, and is no
+// pipeline's single frame, after its launch on a stream that does not capture:
+// the next frame there does not overlap it. Neither allocates nor frees memory.
+void forget_stream_tail(cudaStream_t stream);
 
 // Queues one frame's kernels on `stream` (no host synchronisation).
 // before_main / after_main (may be null) are recorded around the fused tile kernel.

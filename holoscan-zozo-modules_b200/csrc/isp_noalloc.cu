@@ -239,6 +239,7 @@ extern "C" int isp_b200_process_noalloc(const isp_params_c* params, const isp_ra
   if (e != cudaSuccess) return fail_cuda(e, "isp_b200_process_noalloc: table upload");
   const FrameDesc d = make_desc(*params, state, *raw, *out, stats, exposure);
   e = launch_noalloc(d, *params, sm_count, stream);
+  forget_stream_tail(stream);  // its tile pass lets a dependent start early
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return fail_cuda(e, "isp_b200_process_noalloc");
   clear_error();

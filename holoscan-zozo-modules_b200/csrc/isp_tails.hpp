@@ -10,7 +10,7 @@
 // stream, each waiting for its own last frame, no two frames overlapped. If the
 // caller queued other work since, the wait keeps the frame behind all of it,
 // unless that work lets its dependents start early; this library's own kernels
-// that do (launch_dependent) take the stream's entry away, and a frame that finds
+// that do (launch_dependent, and the frames of isp_noalloc.cu) end the entry, and a frame that finds
 // none does not overlap: it may read what they write.
 #pragma once
 
@@ -108,8 +108,8 @@ class StreamTails {
   bool find(const StreamKey& key, F f) {
     std::lock_guard<std::mutex> lock(mutex_);
     const auto it = tails_.find(key);
-    if (!key.known() || it == tails_.end()) return false;
-    f(it->second);
+    if (!key.known() || it == tails_.end() || !it->second.last) return false;
+    f(it->second.tail);
     return true;
   }
 
@@ -123,7 +123,8 @@ class StreamTails {
   // of other work, since a frame's Call that begins later queues behind it.
   bool idle() const { return count_ == 0; }
 
-  // Work other than a frame was queued at `key`, by a call that returns after this.
+  // Work other than a frame was queued at `key`, by a call that returns after
+  // this. Neither allocates nor frees memory.
   void forget(const StreamKey& key) {
     std::lock_guard<std::mutex> lock(mutex_);
     announce(key);
@@ -131,18 +132,31 @@ class StreamTails {
   }
 
  private:
+  struct Entry {
+    Tail tail;
+    bool last;  // nothing was announced behind it
+  };
+
   void put(const StreamKey& key, const Tail& tail) {
     const auto it = tails_.find(key);
-    if (it != tails_.end()) places_.erase(it->second.owner);
-    tails_[key] = tail;
+    if (it != tails_.end()) remove(it->second.tail.owner);
+    tails_[key] = {tail, true};
     places_[tail.owner] = key;
+    ++last_;
   }
 
   void remove(Owner* owner) {
-    const auto it = places_.find(owner);
-    if (it == places_.end()) return;
-    tails_.erase(it->second);
-    places_.erase(it);
+    const auto place = places_.find(owner);
+    if (place == places_.end()) return;
+    const auto it = tails_.find(place->second);
+    bury(it->second);
+    tails_.erase(it);
+    places_.erase(place);
+  }
+
+  void bury(Entry& e) {
+    if (e.last) --last_;
+    e.last = false;
   }
 
   // Work was queued at `key`, or, when that is unknown, anywhere. (At an unknown
@@ -154,21 +168,21 @@ class StreamTails {
     }
     if (key.known()) {
       const auto it = tails_.find(key);
-      if (it != tails_.end()) remove(it->second.owner);
+      if (it != tails_.end()) bury(it->second);
     } else {
-      tails_.clear();
-      places_.clear();
+      for (auto& t : tails_) bury(t.second);
     }
   }
 
   static bool same(const StreamKey& a, const StreamKey& b) { return !(a < b) && !(b < a); }
-  void recount() { count_ = tails_.size() + (calls_ != nullptr ? 1 : 0); }
+  void recount() { count_ = last_ + (calls_ != nullptr ? 1 : 0); }
 
   std::mutex mutex_;
-  std::map<StreamKey, Tail> tails_;
+  std::map<StreamKey, Entry> tails_;
   std::map<Owner*, StreamKey> places_;
   Call* calls_ = nullptr;
-  std::atomic<size_t> count_{0};  // entries, and one more while there are Calls
+  size_t last_ = 0;               // entries that are still last
+  std::atomic<size_t> count_{0};  // these, and one more while there are Calls
 };
 
 }  // namespace isp_b200

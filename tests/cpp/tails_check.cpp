@@ -68,6 +68,19 @@ int main() {
     frame(t, a, s);
     frame(t, b, nowhere);
     expect("work at an unknown place", last(t, s), nullptr);
+    Tails u;
+    if (!u.idle()) ++failures, std::printf("idle without a frame\n");
+    frame(u, a, s);
+    frame(u, b, other);
+    u.forget(s);
+    if (u.idle()) ++failures, std::printf("idle with a frame\n");
+    frame(u, b, s);
+    expect("a camera in the place of an ended entry", last(u, s), &b);
+    frame(u, a, other);
+    expect("the camera of the ended entry", last(u, other), &a);
+    u.drop(&a);
+    u.drop(&b);
+    if (!u.idle()) ++failures, std::printf("idle again\n");
   }
   {
     // A frame's call on one thread; the other thread's conversion is launched
