@@ -15,6 +15,7 @@
 #pragma once
 
 #include "isp_awb.cuh"
+#include "isp_bands.hpp"
 #include "isp_main.cuh"
 
 namespace isp_b200 {
@@ -303,7 +304,8 @@ __global__ void __launch_bounds__(kThreads, 3) isp_awb_batch_kernel(const BatchF
   u64 acc = 0;
   unsigned int done = 0;
   // Tiles run down the 64-column strips of a frame; the lens shading maps and
-  // table are built for as many rows of a strip as come next (a band).
+  // table are built for as many of a strip's next tiles as one table serves (a
+  // band).
   int band_begin = 0, band_end = 0;
   LscTile lt{0, 0};
   AwbCell cell;
@@ -352,7 +354,9 @@ __global__ void __launch_bounds__(kThreads, 3) isp_awb_batch_kernel(const BatchF
     }
     if (item >= band_end) {
       band_begin = item;
-      band_end = min(min(item + tiles_y - ty, r.y), item + kAwbBandRows / 64);
+      int most = min(min(tiles_y - ty, r.y - item), kAwbBandRows / 64);
+      if (fd.lsc != nullptr) most = lsc_band_tiles(y0, most, fd.lsc_sy, fd.lsc_height, kLscTableRows);
+      band_end = item + most;
       lt = build_band_lsc(fd, fd.lsc, fd.pattern, x0, y0, (band_end - band_begin) * 64, m, minmax);
       cell.k = -1;
     }
