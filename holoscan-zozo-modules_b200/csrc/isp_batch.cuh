@@ -53,7 +53,8 @@ __device__ __forceinline__ int next_item(BatchQueue* queue, int item, int2 r, in
   if (count > 0) {
     const unsigned int c = atomicAdd(&queue->claimed, 1U);
     if (c < static_cast<unsigned int>(count)) {
-      claim = make_span(reinterpret_cast<const int2*>(queue + 1), static_cast<size_t>(count), rec)[static_cast<int>(c)];
+      const int2* entries = reinterpret_cast<const int2*>(queue) + queue->first;
+      claim = make_span(entries, static_cast<size_t>(count), rec)[static_cast<int>(c)];
     }
   }
   return claim.x < claim.y ? claim.x : -1;

@@ -44,17 +44,23 @@ struct Entry {
   isp_exposure_c exposure;
 };
 
-// Ranges of work items of a launch, in 8-byte entries from the start of a
-// slot's (and the device's) range memory: one per CTA of the tile pass, one per
-// CTA of the statistics pass, then each pass's BatchQueue with its ranges.
+// Ranges of work items of a launch, in 8-byte entries of a slot's (and the
+// device's) range memory: the BatchQueues of the tile and the statistics pass,
+// one range per CTA of the tile pass, one per CTA of the statistics pass, then the
+// queues' ranges. What a launch uses comes first and without gaps, since its
+// staging reads it over PCIe: with every part at the place of its largest size
+// each launch staged 47 KB, for two 640x480 cameras and for 48 of all sizes alike.
+constexpr int kQueueEntries = static_cast<int>(sizeof(BatchQueue) / sizeof(int2));  // of a BatchQueue itself
+constexpr int kTileRanges = 2 * kQueueEntries;
 constexpr int kQueuePerCta = 4;
 size_t queue_capacity(int max_ctas) { return static_cast<size_t>(kQueuePerCta) * static_cast<size_t>(max_ctas); }
-size_t queue_entries(int max_ctas) { return sizeof(BatchQueue) / sizeof(int2) + queue_capacity(max_ctas); }
-size_t range_entries(int max_ctas) { return 2U * static_cast<size_t>(max_ctas) + 2U * queue_entries(max_ctas); }
-BatchQueue* tile_queue(int2* ranges, int max_ctas) { return reinterpret_cast<BatchQueue*>(ranges + 2 * max_ctas); }
-BatchQueue* awb_queue(int2* ranges, int max_ctas) {
-  return reinterpret_cast<BatchQueue*>(ranges + 2 * max_ctas + queue_entries(max_ctas));
+size_t range_entries(int max_ctas) {
+  return kTileRanges + 2U * static_cast<size_t>(max_ctas) + 2U * queue_capacity(max_ctas);
 }
+BatchQueue* tile_queue(int2* ranges) { return reinterpret_cast<BatchQueue*>(ranges); }
+BatchQueue* awb_queue(int2* ranges) { return reinterpret_cast<BatchQueue*>(ranges + kQueueEntries); }
+int2* tile_ranges(int2* ranges) { return ranges + kTileRanges; }
+int2* awb_ranges(int2* ranges, int main_ctas) { return ranges + kTileRanges + main_ctas; }
 
 // Items of one cost each, in item order.
 struct CostRun {
@@ -63,13 +69,14 @@ struct CostRun {
 };
 
 // Deals work items out: to each of `ctas` CTAs one contiguous range of even
-// cost, together the share `dealt` of the cost, and the rest to the queue in
-// ranges that shrink as it empties. CTAs then finish together although the costs
-// are estimates: with all of the work dealt out beforehand the SMs of a
-// 48-camera batch were idle for a tenth of the tile pass and a quarter of the
-// statistics pass. A frame's first item on a CTA costs a flush of its sums, so
+// cost, together the share `dealt` of the cost, and the rest to the queue, whose
+// ranges go to `queued` and shrink as it empties. CTAs then finish together
+// although the costs are estimates: with all of the work dealt out beforehand the
+// SMs of a 48-camera batch were idle for a tenth of the tile pass and a quarter of
+// the statistics pass. A frame's first item on a CTA costs a flush of its sums, so
 // few items per CTA, and claims of less than kLeast items, are not worth it.
-void deal(const std::vector<CostRun>& runs, int ctas, double dealt, int2* ranges, BatchQueue* queue, int capacity) {
+void deal(const std::vector<CostRun>& runs, int ctas, double dealt, int2* ranges, BatchQueue* queue, int2* queued,
+          int capacity) {
   constexpr int kLeast = 4;
   double total = 0.0;
   int items = 0;
@@ -103,7 +110,7 @@ void deal(const std::vector<CostRun>& runs, int ctas, double dealt, int2* ranges
     ranges[k] = make_int2(begin, item);
   }
   *queue = BatchQueue{};
-  auto* queued = reinterpret_cast<int2*>(queue + 1);
+  queue->first = static_cast<int>(queued - reinterpret_cast<int2*>(queue));
   while (item < items) {
     const int left = items - item;
     const int room = capacity - queue->count;
@@ -116,6 +123,7 @@ void deal(const std::vector<CostRun>& runs, int ctas, double dealt, int2* ranges
 struct Slot {
   BatchFrame* frames = nullptr;  // pinned
   int2* ranges = nullptr;        // pinned
+  int range_words = 0;           // of them, the launch's, in 16-byte words
   const uint4* frames_dev = nullptr;  // the same memory as the device reads it
   const uint4* ranges_dev = nullptr;
   cudaEvent_t consumed = nullptr;
@@ -164,7 +172,7 @@ struct isp_b200_batch {
 
 namespace {
 
-cudaError_t build(isp_b200_batch* b, const Slot& slot, Shape* shape) {
+cudaError_t build(isp_b200_batch* b, Slot& slot, Shape* shape) {
   cudaError_t error = cudaSuccess;
   LaunchShapes& dev = shapes_for_current_device(&error);
   if (error != cudaSuccess) return error;
@@ -214,8 +222,13 @@ cudaError_t build(isp_b200_batch* b, const Slot& slot, Shape* shape) {
   if (error != cudaSuccess) return error;
   const int awb_ctas = awb_tiles == 0 ? 0 : std::max(1, std::min({awb_tiles, dev.sm_count * awb_bpsm, b->max_ctas}));
   const int capacity = static_cast<int>(queue_capacity(b->max_ctas));
-  deal(tile_cost, main_ctas, 0.8, slot.ranges, tile_queue(slot.ranges, b->max_ctas), capacity);
-  deal(awb_cost, awb_ctas, 0.6, slot.ranges + b->max_ctas, awb_queue(slot.ranges, b->max_ctas), capacity);
+  int2* const first = awb_ranges(slot.ranges, main_ctas);
+  int2* queued = first + awb_ctas;
+  deal(tile_cost, main_ctas, 0.8, tile_ranges(slot.ranges), tile_queue(slot.ranges), queued, capacity);
+  queued += tile_queue(slot.ranges)->count;
+  deal(awb_cost, awb_ctas, 0.6, first, awb_queue(slot.ranges), queued, capacity);
+  queued += awb_queue(slot.ranges)->count;
+  slot.range_words = static_cast<int>((queued - slot.ranges + 1) / 2);
   shape->nframes = n;
   shape->main_ctas = main_ctas;
   shape->awb_ctas = awb_ctas;
@@ -242,7 +255,7 @@ struct StageArgs {
         frame_words(static_cast<int>(sizeof(BatchFrame) / sizeof(uint4)) * s.nframes),
         ranges_src(slot.ranges_dev),
         ranges_dst(reinterpret_cast<uint4*>(b->d_ranges)),
-        range_words(static_cast<int>(range_entries(b->max_ctas) * sizeof(int2) / sizeof(uint4))),
+        range_words(slot.range_words),
         args{&frames_src, &frames_dst, &frame_words, &ranges_src, &ranges_dst, &range_words},
         grid((frame_words + range_words + kStageThreads - 1) / kStageThreads) {}
   StageArgs(const StageArgs&) = delete;
@@ -265,15 +278,16 @@ cudaError_t enqueue(isp_b200_batch* b, const Slot& slot, const Shape& s, cudaStr
   cudaError_t e = cudaLaunchKernel(batch_stage_kernel(), stage.grid, dim3(kStageThreads), stage.args, 0, stream);
   if (e != cudaSuccess) return e;
   int nframes = s.nframes;
-  const int2* awb_ranges = b->d_ranges + b->max_ctas;
+  const int2* awb = awb_ranges(b->d_ranges, s.main_ctas);
   if (s.awb_ctas > 0) {
-    auto* queue = awb_queue(b->d_ranges, b->max_ctas);
-    void* args[] = {&b->d_frames, &nframes, &awb_ranges, &queue};
+    auto* queue = awb_queue(b->d_ranges);
+    void* args[] = {&b->d_frames, &nframes, &awb, &queue};
     e = cudaLaunchKernel(awb_batch_kernel(), dim3(s.awb_ctas), dim3(kernel_threads()), args, awb_kernel_smem(), stream);
     if (e != cudaSuccess) return e;
   }
-  auto* queue = tile_queue(b->d_ranges, b->max_ctas);
-  void* args[] = {&b->d_frames, &nframes, &b->d_ranges, &queue};
+  auto* queue = tile_queue(b->d_ranges);
+  const int2* tile = tile_ranges(b->d_ranges);
+  void* args[] = {&b->d_frames, &nframes, &tile, &queue};
   // After the statistics batch, as its programmatic dependent (the tile
   // batch waits for it in the kernel).
   cudaLaunchConfig_t cfg{};
@@ -302,11 +316,11 @@ cudaError_t make_graph(isp_b200_batch* b, const Slot& slot, const Shape& s) {
   e = cudaGraphAddKernelNode(&b->stage, b->graph, nullptr, 0, &sp);
   if (e != cudaSuccess) return e;
   int nframes = s.nframes;  // kernel node arguments are copied when the node is made
-  const int2* awb_ranges = b->d_ranges + b->max_ctas;
+  const int2* awb_range = awb_ranges(b->d_ranges, s.main_ctas);
   cudaGraphNode_t awb = nullptr;
   if (s.awb_ctas > 0) {
-    auto* queue = awb_queue(b->d_ranges, b->max_ctas);
-    void* args[] = {&b->d_frames, &nframes, &awb_ranges, &queue};
+    auto* queue = awb_queue(b->d_ranges);
+    void* args[] = {&b->d_frames, &nframes, &awb_range, &queue};
     cudaKernelNodeParams kp{};
     kp.func = const_cast<void*>(awb_batch_kernel());
     kp.gridDim = dim3(s.awb_ctas);
@@ -316,8 +330,9 @@ cudaError_t make_graph(isp_b200_batch* b, const Slot& slot, const Shape& s) {
     e = cudaGraphAddKernelNode(&awb, b->graph, &b->stage, 1, &kp);
     if (e != cudaSuccess) return e;
   }
-  auto* queue = tile_queue(b->d_ranges, b->max_ctas);
-  void* args[] = {&b->d_frames, &nframes, &b->d_ranges, &queue};
+  auto* queue = tile_queue(b->d_ranges);
+  const int2* tile = tile_ranges(b->d_ranges);
+  void* args[] = {&b->d_frames, &nframes, &tile, &queue};
   cudaKernelNodeParams kp{};
   kp.func = const_cast<void*>(batch_kernel(s.lut_smem, s.tile_rows, s.sharpen));
   kp.gridDim = dim3(s.main_ctas);

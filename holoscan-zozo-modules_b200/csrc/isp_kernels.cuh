@@ -46,10 +46,9 @@ constexpr int kLutSmemEntries = 4097;
 constexpr int kBatchLutEntries = 1024;
 
 // The batch passes (isp_batch.cu): arguments (const BatchFrame* frames, int
-// nframes, const int2* ranges[, const BatchQueue* queue]), one range of work
-// items per CTA (then, in the tile pass, ranges claimed from the queue). The tile
-// pass's dynamic shared memory is batch_kernel_smem(); the statistics pass's
-// is awb_kernel_smem().
+// nframes, const int2* ranges, BatchQueue* queue), one range of work items per
+// CTA, then ranges claimed from the queue. The tile pass's dynamic shared memory
+// is batch_kernel_smem(); the statistics pass's is awb_kernel_smem().
 // sharpen: whether any frame sharpens; a kernel without the sharpening's planes
 // lets three CTAs share an SM instead of two.
 const void* batch_kernel(bool lut_smem, int tile_rows, bool sharpen);

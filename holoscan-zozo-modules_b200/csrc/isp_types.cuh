@@ -115,13 +115,14 @@ struct alignas(64) BatchFrame {
   int use_tma;
 };
 
-// The end of a batch's tile pass: ranges of work items that CTAs claim when
-// they are done with their own, so that they finish together whatever the
-// frames' real costs. Followed in memory by the ranges.
+// The end of a batch pass: ranges of work items that CTAs claim when they are
+// done with their own, so that they finish together whatever the frames' real
+// costs.
 struct alignas(16) BatchQueue {
   int count;             // ranges in the queue
   unsigned int claimed;  // so far; the descriptor staging sets it to 0
-  int pad[2];
+  int first;             // where they lie, in 8-byte entries from this queue
+  int pad;
 };
 
 }  // namespace isp_b200
