@@ -42,19 +42,23 @@ __device__ __forceinline__ int frame_of_item(Span<const BatchFrame> frames, int 
   return f;
 }
 
+// The queue's count and first: read once at a CTA's start, beside its own range,
+// and kept in shared memory, since a read at each claim holds up the thread that
+// claims, and the block behind it, for a round trip to L2.
+__device__ __forceinline__ int2 queue_head(const BatchQueue* queue) { return make_int2(queue->count, queue->first); }
+
 // The item after `item` for a CTA (one thread calls): the next of its range
 // r, or the first of a range claimed from the queue, which is left in `claim`
 // (empty when none is left). -1: none. Queued items come after every CTA's own,
 // and claims only move forward.
-__device__ __forceinline__ int next_item(BatchQueue* queue, int item, int2 r, int2& claim, CheckRecord* rec) {
+__device__ __forceinline__ int next_item(BatchQueue* queue, int2 head, int item, int2 r, int2& claim, CheckRecord* rec) {
   if (item + 1 < r.y) return item + 1;
   claim = make_int2(0, 0);
-  const int count = queue->count;
-  if (count > 0) {
+  if (head.x > 0) {
     const unsigned int c = atomicAdd(&queue->claimed, 1U);
-    if (c < static_cast<unsigned int>(count)) {
-      const int2* entries = reinterpret_cast<const int2*>(queue) + queue->first;
-      claim = make_span(entries, static_cast<size_t>(count), rec)[static_cast<int>(c)];
+    if (c < static_cast<unsigned int>(head.x)) {
+      const int2* entries = reinterpret_cast<const int2*>(queue) + head.y;
+      claim = make_span(entries, static_cast<size_t>(head.x), rec)[static_cast<int>(c)];
     }
   }
   return claim.x < claim.y ? claim.x : -1;
@@ -156,6 +160,7 @@ __global__ void __launch_bounds__(kThreads, kSharpen && kTileH == kTH ? 2 : 3)
   const TileSmem m =
       carve(smem, layout_of(kSharpen, box_row_bytes(kRawU16), kLutSmem ? kBatchLutEntries : 0, kTileH), GS::kSH, rec);
   __shared__ int2 next_range;
+  __shared__ int2 head;
   __shared__ uint64_t bar;
   __shared__ u64 red[4 * kWarps];
   __shared__ int minmax[2];
@@ -164,10 +169,14 @@ __global__ void __launch_bounds__(kThreads, kSharpen && kTileH == kTH ? 2 : 3)
   // A programmatic dependent of the statistics batch: resident early, it
   // waits here for that batch's completion (and the gains it wrote).
   griddep_wait();
+  const int2 queued = queue_head(queue);
   int2 r = ranges[blockIdx.x];
   if (r.x >= r.y) return;
   const int tid = threadIdx.x;
-  if (tid == 0) mbar_init(&bar);
+  if (tid == 0) {
+    head = queued;
+    mbar_init(&bar);
+  }
   int f = frame_of_item(frames, nframes, 0, r.x, false);
   load_desc(&fd, &frames[f].desc);
   __syncthreads();
@@ -214,7 +223,7 @@ __global__ void __launch_bounds__(kThreads, kSharpen && kTileH == kTH ? 2 : 3)
     const bool use_tma = bf.use_tma != 0;
     const auto prefetch = [&] {
       if (tid != 0) return;
-      const int next = next_item(queue, item, r, next_range, rec);
+      const int next = next_item(queue, head, item, r, next_range, rec);
       if (next < 0) return;
       const int g = frame_of_item(frames, nframes, f, next, false);
       if (frames[g].use_tma) {
@@ -276,10 +285,13 @@ __global__ void __launch_bounds__(kThreads, 3) isp_awb_batch_kernel(const BatchF
   __shared__ __align__(16) FrameDesc fd;
   griddep_launch_dependents();  // the tile batch may become resident as this one finishes
   __shared__ int2 next_range[2];
+  __shared__ int2 head;
+  const int2 queued = queue_head(queue);
   int2 r = ranges[blockIdx.x];
   if (r.x >= r.y) return;
   const int tid = threadIdx.x;
   if (tid == 0) {
+    head = queued;
     mbar_init(&bars[0]);
     mbar_init(&bars[1]);
   }
@@ -334,7 +346,7 @@ __global__ void __launch_bounds__(kThreads, 3) isp_awb_batch_kernel(const BatchF
     // range's slot alternates too: the next claim may follow within the next
     // item, before every thread has read this one.
     if (tid == 0) {
-      const int next = next_item(queue, item, r, next_range[buf], rec);
+      const int next = next_item(queue, head, item, r, next_range[buf], rec);
       if (next >= 0) {
         const int g = frame_of_item(frames, nframes, f, next, true);
         if (frames[g].use_tma) {

@@ -120,8 +120,8 @@ struct alignas(64) BatchFrame {
 // costs.
 struct alignas(16) BatchQueue {
   int count;             // ranges in the queue
-  unsigned int claimed;  // so far; the descriptor staging sets it to 0
   int first;             // where they lie, in 8-byte entries from this queue
+  unsigned int claimed;  // so far; the descriptor staging sets it to 0
   int pad;
 };
 
