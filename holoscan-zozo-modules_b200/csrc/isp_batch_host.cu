@@ -165,6 +165,7 @@ struct Shape {
   bool lut_smem = false;
   int tile_rows = 64;
   bool sharpen = false;  // some frame sharpens
+  size_t tile_smem = 0;  // of a CTA of the tile pass; follows from the rest
   bool operator==(const Shape& o) const {
     return nframes == o.nframes && main_ctas == o.main_ctas && awb_ctas == o.awb_ctas && lut_smem == o.lut_smem &&
            tile_rows == o.tile_rows && sharpen == o.sharpen;
@@ -240,7 +241,8 @@ cudaError_t build(isp_b200_batch* b, Slot& slot, Shape* shape) {
   // CTAs: as many as fit (or the tuned count) per SM, never more than items.
   int bpsm = 0;
   const size_t smem = batch_kernel_smem(lut_smem, b->tile_rows, any_sharpen);
-  error = blocks_per_sm(dev, batch_kernel(lut_smem, b->tile_rows, any_sharpen), smem, smem, &bpsm);
+  const size_t roomy = batch_kernel_smem(lut_smem, b->tile_rows, true);
+  error = blocks_per_sm(dev, batch_kernel(lut_smem, b->tile_rows, any_sharpen), roomy, smem, &bpsm);
   if (error != cudaSuccess) return error;
   if (b->ctas_per_sm > 0) bpsm = std::min(bpsm, b->ctas_per_sm);
   const int main_ctas = std::max(1, std::min({tiles, dev.sm_count * bpsm, b->max_ctas}));
@@ -262,6 +264,12 @@ cudaError_t build(isp_b200_batch* b, Slot& slot, Shape* shape) {
   shape->lut_smem = lut_smem;
   shape->tile_rows = b->tile_rows;
   shape->sharpen = any_sharpen;
+  // Little more than one tile an SM, behind a statistics pass: next to one of that
+  // pass's CTAs two small ones fit, and the tile pass would fill some SMs twice
+  // and leave others. As much shared memory as a sharpening tile's leaves room for
+  // one (two 640x480 cameras, gray world: 37.1 and 35.0 us a launch).
+  const bool spread = awb_ctas > 0 && main_ctas > dev.sm_count && main_ctas <= 2 * dev.sm_count;
+  shape->tile_smem = spread ? roomy : smem;
   return cudaSuccess;
 }
 
@@ -320,7 +328,7 @@ cudaError_t enqueue(isp_b200_batch* b, const Slot& slot, const Shape& s, cudaStr
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(s.main_ctas);
   cfg.blockDim = dim3(kernel_threads());
-  cfg.dynamicSmemBytes = batch_kernel_smem(s.lut_smem, s.tile_rows, s.sharpen);
+  cfg.dynamicSmemBytes = s.tile_smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -364,7 +372,7 @@ cudaError_t make_graph(isp_b200_batch* b, const Slot& slot, const Shape& s) {
   kp.func = const_cast<void*>(batch_kernel(s.lut_smem, s.tile_rows, s.sharpen));
   kp.gridDim = dim3(s.main_ctas);
   kp.blockDim = dim3(kernel_threads());
-  kp.sharedMemBytes = static_cast<unsigned int>(batch_kernel_smem(s.lut_smem, s.tile_rows, s.sharpen));
+  kp.sharedMemBytes = static_cast<unsigned int>(s.tile_smem);
   kp.kernelParams = args;
   cudaGraphNode_t main = nullptr;
   if (awb != nullptr) {

@@ -15,6 +15,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("sizes,weights", [
     ([(64, 40)], (1.0, 1.0, 1.0, 1.0)),
     ([(1920, 1080), (35, 67)], (1.0, 1.0, 1.0, 1.0)),
+    ([(640, 480), (640, 480), (200, 150)], (1.0, 1.0, 1.0, 1.0)),
     ([(1792, 1030), (640, 480), (200, 150)], (1.0, 3.0, 1.0, 1.0)),
     ([(1000, 700), (1920, 1080)], (1e-30, float("inf"), 1.0, 1.0)),
 ])
