@@ -184,15 +184,9 @@ __device__ __forceinline__ bool aligned4(const void* p) { return (reinterpret_ca
 __device__ __forceinline__ uint32_t ldw(const uint8_t* p) { return __ldg(reinterpret_cast<const uint32_t*>(p)); }
 
 // c = m s + o on the colour samples, each row summed left to right; alpha
-// passes through (:236-244). kKnown: whether the identity is settled at
-// compile time (kIdentity then says which), else p.identity decides.
-template <bool kKnown = false, bool kIdentity = false>
+// passes through (:236-244).
 __device__ __forceinline__ Px apply_affine(const Plan& p, Px s) {
-  if constexpr (kKnown) {
-    if constexpr (kIdentity) return s;
-  } else {
-    if (p.identity) return s;
-  }
+  if (p.identity) return s;
   Px r;
   r.c0 = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(p.m[0], s.c0), __fmul_rn(p.m[1], s.c1)), __fmul_rn(p.m[2], s.c2)),
                    p.o[0]);
@@ -269,8 +263,6 @@ __device__ __forceinline__ void store_chroma(const Image& img, int cx, int cy, f
     q[2] = static_cast<uint8_t>(code8(cr));
   }
 }
-
-__device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
 #endif  // __CUDACC__
 

@@ -26,35 +26,31 @@ constexpr int kThreadsY = 8;
 // thread): at four, a 4K frame's 2,025 CTAs ran 3.42 waves, the last 42 % full.
 constexpr int kDirectBlocksPerSm = 5;
 constexpr int kSms = 148;  // of a B200: a matter of balance only
-__device__ __forceinline__ bool yuv_dst(int f) { return f <= CC_UYVY; }
 
 // The colour map of two pixels at once: the nine products two lanes at a
 // time (mul.rn.f32x2, each lane rounded as the scalar product), every sum in
 // the definition's order; a two-lane product never feeds a plain two-lane
 // sum, which the assembler could fuse into one rounding (psum2).
-template <bool kIdentity>
 __device__ __forceinline__ void affine_pair(const Plan& p, Px& a, Px& b) {
-  if constexpr (!kIdentity) {
-    using isp_b200::add2;
-    using isp_b200::bc2;
-    using isp_b200::mul2;
-    using isp_b200::psum2;
-    const float2 s0 = make_float2(a.c0, b.c0), s1 = make_float2(a.c1, b.c1), s2 = make_float2(a.c2, b.c2);
-    float2 out[3];
+  using isp_b200::add2;
+  using isp_b200::bc2;
+  using isp_b200::mul2;
+  using isp_b200::psum2;
+  const float2 s0 = make_float2(a.c0, b.c0), s1 = make_float2(a.c1, b.c1), s2 = make_float2(a.c2, b.c2);
+  float2 out[3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const float2 t0 = mul2(bc2(p.m[3 * k]), s0);
-      const float2 t1 = mul2(bc2(p.m[3 * k + 1]), s1);
-      const float2 t2 = mul2(bc2(p.m[3 * k + 2]), s2);
-      out[k] = add2(psum2(t2, psum2(t0, t1)), bc2(p.o[k]));
-    }
-    a.c0 = out[0].x;
-    b.c0 = out[0].y;
-    a.c1 = out[1].x;
-    b.c1 = out[1].y;
-    a.c2 = out[2].x;
-    b.c2 = out[2].y;
+  for (int k = 0; k < 3; ++k) {
+    const float2 t0 = mul2(bc2(p.m[3 * k]), s0);
+    const float2 t1 = mul2(bc2(p.m[3 * k + 1]), s1);
+    const float2 t2 = mul2(bc2(p.m[3 * k + 2]), s2);
+    out[k] = add2(psum2(t2, psum2(t0, t1)), bc2(p.o[k]));
   }
+  a.c0 = out[0].x;
+  b.c0 = out[0].y;
+  a.c1 = out[1].x;
+  b.c1 = out[1].y;
+  a.c2 = out[2].x;
+  b.c2 = out[2].y;
 }
 
 // code8_bits of two values: the + 0.5 and the add of 2^23 rounded toward

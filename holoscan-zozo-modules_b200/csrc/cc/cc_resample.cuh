@@ -576,8 +576,8 @@ __global__ void __launch_bounds__(kThreadsX* kResampleThreadsY, resample_blocks(
         sample_group<kF, kMode, kAlpha, kFast>(p, ax, ay, v[r]);
       }
       if (!p.identity) {
-        affine_pair<false>(p, v[r][0], v[r][1]);
-        affine_pair<false>(p, v[r][2], v[r][3]);
+        affine_pair(p, v[r][0], v[r][1]);
+        affine_pair(p, v[r][2], v[r][3]);
       }
       if (!inside || y != y0 + r) {
 #pragma unroll

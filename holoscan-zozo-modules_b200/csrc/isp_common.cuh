@@ -369,11 +369,10 @@ struct LscTile {
 
 // Fills the column and row maps (mirrored coordinates, grid cells) and, when
 // it fits, the table. Threads 0..ncols-1 do columns, the next nrows do rows.
-// kPaired: the table holds float2 pairs {T(s), T(s + kHalf)} for s < kPW
-// (the tile pass's paired columns); otherwise one float per column.
+// The table holds float2 pairs {T(s), T(s + kHalf)} for s < kPW (the tile pass's
+// paired columns).
 // `grid`: the frame's lens shading gains (the frame's own, or a copy in
 // shared memory).
-template <bool kPaired = false>
 __device__ LscTile build_lsc(const FrameDesc& p, Span<const float> grid, int pattern, int x_first, int ncols, int y_first,
                              int nrows,
                              bool mirror_xy, int xclamp, int yclamp, Span<int> col_mx, Span<int> col_ix, Span<float> col_tx,
@@ -435,46 +434,33 @@ __device__ LscTile build_lsc(const FrameDesc& p, Span<const float> grid, int pat
     Span<const float> g = grid + ((lt.iy0 + k) * p.lsc_width + col_ix[i]) * step + ch;
     return g[0] + (g[step] - g[0]) * col_tx[i];
   };
-  if constexpr (kPaired) {
-    Span<float2> table2 = span_cast<float2>(table);
-    for (int e = t; e < lt.rows * planes * kPW; e += kThreads) {
-      const int i = e % kPW;
-      const int kp = e / kPW;
-      const int par = kp % planes;
-      const int k = kp / planes;
-      table2[(k * 2 + par) * kPW + i] = make_float2(entry(k, par, i), entry(k, par, i + kHalf));
-    }
-  } else {
-    for (int e = t; e < lt.rows * planes * ncols; e += kThreads) {
-      const int i = e % ncols;
-      const int kp = e / ncols;
-      const int par = kp % planes;
-      const int k = kp / planes;
-      table[(k * 2 + par) * kSW + i] = entry(k, par, i);
-    }
+  Span<float2> table2 = span_cast<float2>(table);
+  for (int e = t; e < lt.rows * planes * kPW; e += kThreads) {
+    const int i = e % kPW;
+    const int kp = e / kPW;
+    const int par = kp % planes;
+    const int k = kp / planes;
+    table2[(k * 2 + par) * kPW + i] = make_float2(entry(k, par, i), entry(k, par, i + kHalf));
   }
   if (t < nrows) row_k[t] -= lt.iy0;
   __syncthreads();
   return lt;
 }
 
-// build_lsc<true> for a tile none of whose rows and columns is mirrored:
+// build_lsc for a tile none of whose rows and columns is mirrored:
 // the grid rows it spans follow from its first and last rows (a row's grid
 // cell never decreases down the frame), so the row maps and the paired table
 // are written in one pass behind one block barrier, each table entry working
 // out its own column's cell (the same operations as build_lsc's column maps).
-// Tiles whose table would not fit take build_lsc<true>. Of the column maps
-// only the columns themselves are written (the path of phase A without a TMA
-// box reads them); the cells are worked out where the table needs them.
+// Tiles whose table would not fit take build_lsc. The mirrored rows and columns
+// are not written: phase A reads those of edge tiles and of grids too dense for
+// the table only.
 __device__ LscTile build_lsc_inner(const FrameDesc& p, Span<const float> grid, int pattern, int x_first, int y_first,
                                    int nrows, Span<int> col_mx, Span<int> col_ix, Span<float> col_tx, Span<int> row_my, Span<int> row_k,
                                    Span<float> row_ty, Span<float> table, int* minmax) {
   LscTile lt{0, 0};
   const int t = threadIdx.x;
   if (p.lsc == nullptr) {
-    if (t < kSW) col_mx[t] = x_first + t;
-    if (t < nrows) row_my[t] = y_first + t;
-    __syncthreads();
     return lt;
   }
   const auto row_cell = [&](int y) {
@@ -484,13 +470,11 @@ __device__ LscTile build_lsc_inner(const FrameDesc& p, Span<const float> grid, i
   lt.iy0 = row_cell(y_first);
   lt.rows = row_cell(y_first + nrows - 1) - lt.iy0 + 2;
   if (lt.rows > kLscTableRows) {
-    return build_lsc<true>(p, grid, pattern, x_first, kSW, y_first, nrows, false, 0, 0, col_mx, col_ix, col_tx, row_my,
+    return build_lsc(p, grid, pattern, x_first, kSW, y_first, nrows, false, 0, 0, col_mx, col_ix, col_tx, row_my,
                            row_k, row_ty, table, minmax);
   }
-  if (t < kSW) col_mx[t] = x_first + t;
   if (t < nrows) {
     const int y = y_first + t;
-    row_my[t] = y;
     const float fy = static_cast<float>(y) * p.lsc_sy;
     int iy = static_cast<int>(fy);
     iy = iy > p.lsc_height - 2 ? p.lsc_height - 2 : iy;

@@ -208,7 +208,7 @@ __device__ __forceinline__ unsigned int tile_samples(const FrameDesc& p, const F
   }
   t.lt = interior ? build_lsc_inner(p, f.grid, p.pattern, x0 - 4, y0 - kHalo, kSH, m.col_mx, m.col_ix, m.col_tx, m.row_my,
                                     m.row_k, m.row_ty, span_cast<float>(m.table), minmax)
-                  : build_lsc<true>(p, f.grid, p.pattern, x0 - 4, kSW, y0 - kHalo, kSH, true, p.width + 3,
+                  : build_lsc(p, f.grid, p.pattern, x0 - 4, kSW, y0 - kHalo, kSH, true, p.width + 3,
                                     p.height + kHalo - 1, m.col_mx, m.col_ix, m.col_tx, m.row_my, m.row_k, m.row_ty,
                                     span_cast<float>(m.table), minmax);
   if (use_tma) {

@@ -19,15 +19,15 @@
 //      isp_math.hpp:219-227), colour matrix, statistics sums, tone, store and
 //      histogram codes (isp_math.hpp:229-305).
 //
-// What bounds the pass is the shared-memory pipe: ncu counts 57 wavefronts per
-// 32 pixels of a sharpened 3840x2160 RAW10 frame, 75 % of the pipe while the
-// SMs work (issue slots 59 %, FMA pipe 44 %): tone table lookups 20 and
-// histogram atomics 13, most of them bank conflicts that the data decides,
-// the rest the planes and tables of the phases. So the phases are shaped to
-// touch shared memory less (A keeps its table rows in registers, B's units are
-// six rows high), and sums of products run two lanes at a time (isp_ops.cuh).
-// The frame's pass went from 101.0 to 91.9 us with these, a 1920x1080 16-bit
-// one with the same stages from 43.3 to 38.8 us.
+// What bounds the pass is the shared-memory pipe: ncu counts 48 wavefronts per
+// 32 pixels of a sharpened 3840x2160 RAW10 frame, 70 % of the pipe while the SMs
+// work (issue slots 57 %, FMA pipe 46 %); 17 of them are bank conflicts of the
+// tone table's lookups and the histogram's atomics, whose addresses the data
+// decides. So the phases are shaped to touch shared memory less (A keeps its table
+// rows in registers, B's units are six rows high; 57 wavefronts and 75 % before),
+// and sums of products run two lanes at a time (isp_ops.cuh). The frame's pass
+// went from 101.0 to 91.9 us with these, a 1920x1080 16-bit one with the same
+// stages from 43.3 to 38.8 us.
 #pragma once
 
 #include "isp_common.cuh"
