@@ -541,7 +541,6 @@ int isp_b200_batch_launch(isp_b200_batch* b, void* stream_ptr, int32_t use_graph
   b->next_slot = (b->next_slot + 1) % kStagingSlots;
   for (const Entry& en : b->entries) {
     drop_stream_tail(en.camera);
-    en.camera->last = {};  // its next frame waits for the event
     e = cudaEventRecord(en.camera->done, stream);
     if (e != cudaSuccess) return fail_cuda(e, "cudaEventRecord");
     en.camera->queued = true;

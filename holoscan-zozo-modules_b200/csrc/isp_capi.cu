@@ -327,7 +327,10 @@ cudaError_t blocks_per_sm(LaunchShapes& shapes, const void* kernel, size_t smem_
   return cudaSuccess;
 }
 
-void drop_stream_tail(isp_b200_pipeline* pl) { g_tails.drop(pl); }
+void drop_stream_tail(isp_b200_pipeline* pl) {
+  g_tails.drop(pl, pl->last);
+  pl->last = {};
+}
 
 void forget_stream_tail(cudaStream_t stream) {
   if (!g_tails.idle()) g_tails.forget(place_of(stream));
@@ -592,9 +595,10 @@ int isp_b200_process(isp_b200_pipeline* pl, const isp_raw_view_c* raw, const isp
   error = cudaEventRecord(pl->done, stream);
   if (error != cudaSuccess) return fail_cuda(error, "cudaEventRecord");
   pl->queued = true;
+  const StreamKey before = pl->last;
   pl->last = here.capturing ? place_of(stream) : here;
   const auto image = reinterpret_cast<uintptr_t>(out->data);
-  call.finish({pl, image, image + out->pitch * static_cast<size_t>(raw->height)}, pl->last);
+  call.finish({pl, image, image + out->pitch * static_cast<size_t>(raw->height)}, pl->last, before);
   clear_error();
   return ISP_OK;
 }
@@ -739,7 +743,6 @@ int isp_b200_check_bounded_wait(isp_b200_pipeline* pl, uint32_t polls, void* str
     error = cudaLaunchKernel(wait_check_kernel(), dim3(1), dim3(32), args, 0, stream);
   }
   drop_stream_tail(pl);
-  pl->last = {};  // its next frame waits for the event
   if (error == cudaSuccess) error = cudaEventRecord(pl->done, stream);
   if (error != cudaSuccess) return fail_cuda(error, "isp_b200_check_bounded_wait");
   pl->queued = true;

@@ -105,7 +105,8 @@ LaunchShapes& shapes_for_current_device(cudaError_t* error);
 cudaError_t launch_dependent(const void* kernel, dim3 grid, dim3 block, void** args, cudaStream_t stream);
 
 // For whoever records a pipeline's `done` elsewhere than behind a single frame:
-// frames of other pipelines no longer wait for it.
+// frames of other pipelines no longer wait for it, and the pipeline's next frame
+// follows nothing but its event.
 void drop_stream_tail(isp_b200_pipeline* pl);
 // For whoever queued a kernel that lets its dependents start early, and is no
 // pipeline's single frame, after its launch on a stream that does not capture:

@@ -65,22 +65,24 @@ class StreamTails {
       tails_.recount();
     }
     ~Call() {
+      if (finished_) return;
       std::lock_guard<std::mutex> lock(tails_.mutex_);
       leave();
-      if (!finished_) tails_.announce(key_);
+      tails_.announce(key_);
       tails_.recount();
     }
     Call(const Call&) = delete;
     Call& operator=(const Call&) = delete;
 
     // The frame is queued, and the next work will come at `place` (the Call's
-    // own outside captures).
-    void finish(const Tail& tail, const StreamKey& place) {
+    // own outside captures); `before`: the place after the owner's last frame.
+    // Frames in turn on one stream cost no allocation.
+    void finish(const Tail& tail, const StreamKey& place, const StreamKey& before) {
       std::lock_guard<std::mutex> lock(tails_.mutex_);
       leave();
       finished_ = true;
       tails_.announce(key_);
-      tails_.remove(tail.owner);
+      if (disturbed_ || !place.known() || !same(place, before)) tails_.remove(tail.owner, before);
       if (!disturbed_ && place.known()) tails_.put(place, tail);
       tails_.recount();
     }
@@ -113,9 +115,10 @@ class StreamTails {
     return true;
   }
 
-  void drop(Owner* owner) {
+  // `place`: the place after the owner's last frame.
+  void drop(Owner* owner, const StreamKey& place) {
     std::lock_guard<std::mutex> lock(mutex_);
-    remove(owner);
+    remove(owner, place);
     recount();
   }
 
@@ -133,25 +136,21 @@ class StreamTails {
 
  private:
   struct Entry {
-    Tail tail;
-    bool last;  // nothing was announced behind it
+    Tail tail{};
+    bool last = false;  // nothing was announced behind it
   };
 
   void put(const StreamKey& key, const Tail& tail) {
-    const auto it = tails_.find(key);
-    if (it != tails_.end()) remove(it->second.tail.owner);
-    tails_[key] = {tail, true};
-    places_[tail.owner] = key;
-    ++last_;
+    Entry& e = tails_[key];
+    if (!e.last) ++last_;
+    e = {tail, true};
   }
 
-  void remove(Owner* owner) {
-    const auto place = places_.find(owner);
-    if (place == places_.end()) return;
-    const auto it = tails_.find(place->second);
+  void remove(Owner* owner, const StreamKey& place) {
+    const auto it = tails_.find(place);
+    if (it == tails_.end() || it->second.tail.owner != owner) return;
     bury(it->second);
     tails_.erase(it);
-    places_.erase(place);
   }
 
   void bury(Entry& e) {
@@ -179,7 +178,6 @@ class StreamTails {
 
   std::mutex mutex_;
   std::map<StreamKey, Entry> tails_;
-  std::map<Owner*, StreamKey> places_;
   Call* calls_ = nullptr;
   size_t last_ = 0;               // entries that are still last
   std::atomic<size_t> count_{0};  // these, and one more while there are Calls

@@ -7,7 +7,9 @@
 
 namespace {
 
-struct Camera {};
+struct Camera {
+  isp_b200::StreamKey last;
+};
 using Tails = isp_b200::StreamTails<Camera>;
 using isp_b200::StreamKey;
 
@@ -41,7 +43,8 @@ void expect(const char* name, Camera* got, Camera* want) {
 
 void frame(Tails& t, Camera& c, const StreamKey& k) {
   Tails::Call call(t, k);
-  call.finish({&c, 0, 1}, k);
+  call.finish({&c, 0, 1}, k, c.last);
+  c.last = k;
 }
 
 }  // namespace
@@ -63,7 +66,7 @@ int main() {
     t.forget(other);
     expect("a conversion takes the entry", last(t, other), nullptr);
     frame(t, a, s);
-    t.drop(&a);
+    t.drop(&a, a.last);
     expect("a dropped camera", last(t, s), nullptr);
     frame(t, a, s);
     frame(t, b, nowhere);
@@ -78,8 +81,8 @@ int main() {
     expect("a camera in the place of an ended entry", last(u, s), &b);
     frame(u, a, other);
     expect("the camera of the ended entry", last(u, other), &a);
-    u.drop(&a);
-    u.drop(&b);
+    u.drop(&a, a.last);
+    u.drop(&b, b.last);
     if (!u.idle()) ++failures, std::printf("idle again\n");
   }
   {
@@ -89,7 +92,7 @@ int main() {
     {
       Tails::Call call(t, s);
       t.forget(s);
-      call.finish({&a, 0, 1}, s);
+      call.finish({&a, 0, 1}, s, a.last);
     }
     expect("a conversion within a frame's call", last(t, s), nullptr);
     // Launched within the call, announced after it.
@@ -100,7 +103,7 @@ int main() {
     {
       Tails::Call call(t, s);
       t.forget(other);
-      call.finish({&a, 0, 1}, s);
+      call.finish({&a, 0, 1}, s, a.last);
     }
     expect("a conversion on another stream", last(t, s), &a);
   }
@@ -109,8 +112,8 @@ int main() {
     Tails t;
     Tails::Call first(t, s);
     Tails::Call second(t, s);
-    second.finish({&b, 0, 1}, s);
-    first.finish({&a, 0, 1}, s);
+    second.finish({&b, 0, 1}, s, b.last);
+    first.finish({&a, 0, 1}, s, a.last);
     expect("two frames at once", last(t, s), nullptr);
   }
   {
@@ -126,7 +129,7 @@ int main() {
     frame(t, a, s);
     {
       Tails::Call call(t, node(1, 100));
-      call.finish({&b, 0, 1}, node(1, 101));
+      call.finish({&b, 0, 1}, node(1, 101), b.last);
     }
     expect("the captured frame", last(t, node(1, 101)), &b);
     expect("another node", last(t, node(1, 102)), nullptr);
@@ -136,7 +139,7 @@ int main() {
     begin.capturing = true;
     {
       Tails::Call call(t, begin);
-      call.finish({&b, 0, 1}, node(3, 100));
+      call.finish({&b, 0, 1}, node(3, 100), node(1, 101));
     }
     expect("the first frame of a capture", last(t, node(3, 100)), &b);
     expect("outside that capture", last(t, s), &a);
